@@ -3,6 +3,7 @@
 // the host translation units include it.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 
 #include <vector_types.h>
@@ -25,9 +26,16 @@ constexpr int kBinDirectMax = 4;              // triangles spanning <= 4 tiles b
 constexpr int kStageSlots = 3;                // pinned staging slots for back-to-back async draws
 constexpr int kRasterMaxSlices = 32;          // CTAs that may share one tile's bin
 static_assert(kRasterMaxSlices <= 32, "a raster work item packs its slice into 5 bits");
+// The raster's cost estimate, in about eighths of a staged bin entry: an entry
+// costs kEntryCost and half the pixels of its tile-clipped box.  Frames of the
+// default 32 x 32 tiles at slice costs of 4096 / 8192 / 16384: 200k-face terrain at
+// 1280x720 102 / 94 / 116 us, 82k-face icosphere presented at 1920x1080 75 / 74 /
+// 84 us, 64 icospheres (5.0 M faces) 333 / 328 / 325 us.  (With 32 an entry and whole
+// boxes, which splits tiles of small triangles four times as far: 121 / 105 /
+// 98, 86 / 80 / 75, 382 / 348 / 333 us.)
 constexpr int kDefaultSliceCost = 8192;       // raster cost per slice before a tile is split
-constexpr int kEntryCost = 32;                // raster cost of a bin entry covering <= kSmallBox pixels
-constexpr int kSmallBox = 64;                 // larger tile-clipped boxes add their area to the tile's cost
+constexpr int kEntryCost = 8;                 // raster cost of a bin entry covering <= kSmallBox pixels
+constexpr int kSmallBox = 64;                 // larger tile-clipped boxes add half their area to the tile's cost
 // k_setup: resident CTAs an SM by the frame's face count (its k_cull lane
 // count): 2 (at most 104 registers a thread, no spills, room for a k_clip CTA
 // beside them) below 1 M faces; 3 (at most 80 registers, 64 bytes spilled)
@@ -123,6 +131,20 @@ __host__ __device__ inline int box_visibility(const float* m, const float* bbox)
     if (outside > 0) return 1;
   }
   return 2;
+}
+
+// Correctly rounded a / b from y = RN(1 / b), without a branch: one
+// multiplication and two residual corrections (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990: when q
+// is within an ulp of a / b and y is 1 / b rounded to nearest, q + RN(a - bq) y
+// rounds to RN(a / b)).  The first correction brings a * y, up to two ulps
+// off, within that ulp.  Needs y, the quotient and the residuals clear of
+// overflow and underflow (narrow_fast).  Five operations where the general
+// division takes about twice as many and a branch to its special cases.
+__host__ __device__ inline float div_by(float a, float b, float y) {
+  float q = a * y;
+  q = fmaf(fmaf(-b, q, a), y, q);
+  return fmaf(fmaf(-b, q, a), y, q);
 }
 
 // Raster setup of one binned triangle (64 bytes, in registers and shared
@@ -285,7 +307,8 @@ struct FrameArgs {
   unsigned long long* pkey;         // per pixel of every view: final visibility keys, shaded by k_resolve
                                     // (null: k_raster shades each tile itself)
   uint4* tile_info;                 // per tile, from k_plan: x bin entries, y raster slices, z first key
-                                    // slot of a split tile of a one-view frame (kNoSlot: merged in gkey)
+                                    // slot of a split tile of a one-view frame (kNoSlot: merged in gkey),
+                                    // w pixels of its large entries' boxes
   unsigned long long* slot_keys;    // one-view frames: slot_cap slots of TS x TS keys, one per slice of a
                                     // split tile; k_resolve takes the max over a tile's slots
   uint32_t slot_cap;

@@ -18,9 +18,9 @@
 //              the work queue heaviest first.
 //   k_raster   persistent CTAs over the queue, one TS x TS tile slice each:
 //              visibility in shared memory as a 64-bit max of (ordered zRec,
-//              draw-order key); each row of a footprint is narrowed to its
-//              exact covered span, so only covered pixels reach the depth
-//              test; slices merge through global keys.  Many views: the
+//              draw-order key); footprints go as runs of up to 8 pixels of a
+//              row, shared out among the CTA's warps, and only covered pixels
+//              reach the depth test; slices merge through global keys.  Many views: the
 //              tile is shaded in place.  One view: the final keys are stored
 //              and
 //   k_resolve  shades every pixel once for its winner (deferred), with Clear,
@@ -1228,7 +1228,7 @@ __device__ __forceinline__ void edges_at(const TriRaster& t, const TriWide* wide
 template <int TS>
 struct RasterShape {
   static constexpr int kThreads = TS * TS / 4;  // 4 pixels per thread in the resolve
-  static constexpr int kStride = TS + 8;        // padded key row: 8x4 warp blocks hit disjoint banks
+  static constexpr int kStride = TS + 2;        // padded key row: eight rows' pixels of one column hit disjoint banks
   static constexpr int kWarps = kThreads / 32;
   static constexpr int kMinBlocks = 2048 / kThreads / 2;  // 32 warps per SM: 64 registers a thread
 };
@@ -1252,74 +1252,35 @@ __device__ __forceinline__ void depth_at(unsigned long long* p, const TriRaster&
   if (k > *(volatile unsigned long long*)p) atomicMax(p, k);
 }
 
-// True when the pixel at p already holds a depth that a candidate with
-// vertex depths w0..w2 cannot reach (the early out above).
-__device__ __forceinline__ bool depth_beaten(const unsigned long long* p, const TriRaster& t) {
-  const uint32_t o = (uint32_t)(*(const volatile unsigned long long*)p >> 32);
-  if (!(o & 0x80000000u)) return false;  // the pixel holds a depth < +0
-  const float wmin = fminf(fminf(-t.w0, -t.w1), -t.w2);
-  return wmin > 0.0f && __fmul_rn(__uint_as_float(o & 0x7FFFFFFFu), wmin) > 1.00001f;
+// True when a pixel whose key is k already holds a depth that a candidate
+// with vertex depths of at least wmin = min(-w) cannot reach (the early out
+// above; 0 where some w is not negative).  A key depth below +0 turns into a
+// negative number or a NaN here, which is not beaten.
+__device__ __forceinline__ bool depth_beaten(unsigned long long k, float wmin) {
+  return __fmul_rn(__uint_as_float((uint32_t)(k >> 32) ^ 0x80000000u), wmin) > 1.00001f;
 }
 
 template <int TS>
 __device__ __forceinline__ void depth_candidate(unsigned long long* skey, const TriRaster& t, const TriWide* wide,
                                                 uint32_t r, int x, int y, int tx0, int ty0) {
   unsigned long long* p = skey + (y - ty0) * RasterShape<TS>::kStride + (x - tx0);
-  if (depth_beaten(p, t)) return;
+  const float wmin = fmaxf(fminf(fminf(-t.w0, -t.w1), -t.w2), 0.0f);
+  if (depth_beaten(*(volatile unsigned long long*)p, wmin)) return;
   bool inside;
   float e12f, e20f;
   edges_at(t, wide, r, x, y, inside, e12f, e20f);
   depth_at(p, t, e12f, e20f);
 }
 
-// Depth test of a pixel known to be covered by narrow triangle t.
-template <int TS>
-__device__ __forceinline__ void depth_covered(unsigned long long* skey, const TriRaster& t, int x, int y, int tx0,
-                                              int ty0) {
-  unsigned long long* p = skey + (y - ty0) * RasterShape<TS>::kStride + (x - tx0);
-  if (depth_beaten(p, t)) return;
-  const int e12 = t.a12 * x + t.b12 * y + t.c12;
-  const int e20 = t.a20 * x + t.b20 * y + t.c20;
-  depth_at(p, t, __int2float_rn(e12), __int2float_rn(e20));
-}
-
-// floor(n / d) for d > 0, exact when the quotient lies in [lo - 1, hi + 1];
-// otherwise a value on the same side of that range.  The float estimate is
-// within one of the quotient (|n| < 2^31, d < 2^15: a few ulps of relative
-// error, below 1 while |n / d| < 2^20; beyond that the clamp decides), and
-// one exact integer step corrects it.
-__device__ __forceinline__ int floor_div_near(int n, int d, int lo, int hi) {
-  float q = floorf(__fdividef(__int2float_rn(n), __int2float_rn(d)));
-  q = fminf(fmaxf(q, (float)(lo - 1)), (float)(hi + 1));
-  int qi = (int)q;
-  if (qi * d > n) --qi;
-  else if ((qi + 1) * d <= n) ++qi;
-  return qi;
-}
-
-// Narrows [xl, xr] on row y to the x where a*x + (b*y + c) < 0 (one edge of
-// the inside test, rasterizer.go:147).  All products stay in int32 for
-// narrow triangles (|a|, |b| < 2^15, |c| < 2^29, 0 <= x, y < 2^14).
-__device__ __forceinline__ void span_edge(int a, int b, int c, int y, int& xl, int& xr) {
-  const int k = b * y + c;
-  const int n = a > 0 ? -k - 1 : k;  // a > 0: x <= floor((-k-1)/a); a < 0: x >= floor(k/-a) + 1
-  const int q = floor_div_near(n, a > 0 ? a : max(-a, 1), xl, xr);
-  if (a > 0) xr = min(xr, q);
-  else if (a < 0) xl = max(xl, q + 1);
-  else if (k >= 0) xr = xl - 1;      // a == 0: the whole row is outside this edge
-}
-
-// Last lane j with start[j] <= g (start non-decreasing across lanes, lane 0's
-// start <= g); zero-length lanes share the next lane's start and are skipped.
-__device__ __forceinline__ int owner_lane(int start, int g) {
-  int own = 0;
-#pragma unroll
-  for (int step = 16; step > 0; step >>= 1) {
-    const int cand = own + step;
-    const int cs = __shfl_sync(FULL_MASK, start, cand & 31);
-    if (cand < 32 && cs <= g) own = cand;
-  }
-  return own;
+// Whether triangle t takes the raster's unit walk: a narrow triangle whose
+// W's magnitudes lie in [2^-60, 2^60], where div_by is exact.  Its sum and
+// edge values are whole numbers in [1, 2^32) by magnitude, so al and be lie in
+// [2^-32, 1] and ga is 0 or at least 2^-57 (a difference of values on a
+// 2^-57 grid): quotients by W stay above 2^-117 and residuals above 2^-104.
+__device__ __forceinline__ bool narrow_fast(const TriRaster& t) {
+  const uint32_t e0 = (__float_as_uint(t.w0) >> 23) & 0xFFu, e1 = (__float_as_uint(t.w1) >> 23) & 0xFFu,
+                 e2 = (__float_as_uint(t.w2) >> 23) & 0xFFu;
+  return !(t.key & 0x80000000u) && e0 - 67u <= 120u && e1 - 67u <= 120u && e2 - 67u <= 120u;
 }
 
 __device__ __forceinline__ int warp_incl_scan(int v) {
@@ -1344,86 +1305,6 @@ __device__ __forceinline__ bool covers(const TriRaster& t, const TriWide* wide, 
   return inside;
 }
 
-// Minimum of a narrow edge function over the pixel box [X0,X1] x [Y0,Y1].
-__device__ __forceinline__ int edge_min(int a, int b, int c, int X0, int X1, int Y0, int Y1) {
-  return c + min(a * X0, a * X1) + min(b * Y0, b * Y1);
-}
-
-// Per-warp queue of covered pixels awaiting the exact depth test, so that the
-// division-heavy part runs with every lane busy.  Each entry names a slot of
-// the warp's triangle table (records staged in shared memory, so a drain
-// reads no global memory) and a pixel.  qn is warp-uniform; capacity 64: the
-// warp drains 32 whenever qn >= 32.
-template <int TS>
-struct CandQueue {
-  uint32_t* ent;        // slot | x << 8 | y << 20
-  const TriRaster* tri; // the warp's triangle table (kSlots entries)
-  const uint32_t* rec;  // record index per slot (for int64 edge coefficients)
-  int qn;
-
-  __device__ __forceinline__ void run(uint32_t e, unsigned long long* skey, const FrameArgs& a, int tx0, int ty0) {
-    const uint32_t slot = e & 0xFFu;
-    const TriRaster t = tri[slot];
-    depth_candidate<TS>(skey, t, a.wide, rec[slot], tx0 + (int)((e >> 8) & 0xFFFu), ty0 + (int)(e >> 20), tx0,
-                        ty0);
-  }
-
-  __device__ __forceinline__ void push(bool covered, uint32_t slot, int x, int y, unsigned long long* skey,
-                                       const FrameArgs& a, int tx0, int ty0) {
-    const unsigned lane = lane_id();
-    const unsigned m = __ballot_sync(FULL_MASK, covered);
-    if (covered) ent[qn + __popc(m & ((1u << lane) - 1u))] = slot | ((uint32_t)x << 8) | ((uint32_t)y << 20);
-    qn += __popc(m);
-    if (qn >= 32) {
-      __syncwarp();
-      run(ent[lane], skey, a, tx0, ty0);
-      const int rest = qn - 32;
-      uint32_t e = 0;
-      if ((int)lane < rest) e = ent[32 + lane];
-      __syncwarp();
-      if ((int)lane < rest) ent[lane] = e;
-      __syncwarp();
-      qn = rest;
-    }
-  }
-
-  __device__ __forceinline__ void flush(unsigned long long* skey, const FrameArgs& a, int tx0, int ty0) {
-    const unsigned lane = lane_id();
-    __syncwarp();
-    if ((int)lane < qn) run(ent[lane], skey, a, tx0, ty0);
-    __syncwarp();
-    qn = 0;
-  }
-};
-
-
-// Walks the 8x4 blocks j = j0, j0 + step, ... of the footprint [bx0,bx1] x
-// [by0,by1] of the triangle in table slot `slot`, one pixel per lane.  Blocks
-// that one edge excludes entirely are skipped before any per-pixel work;
-// covered pixels go to the warp's queue.
-template <int TS>
-__device__ __forceinline__ void walk_blocks(CandQueue<TS>& q, unsigned long long* skey, const FrameArgs& a,
-                                            const TriRaster& tt, uint32_t rr, uint32_t slot, int bx0, int bx1,
-                                            int by0, int by1, int j0, int step, int tx0, int ty0) {
-  const unsigned lane = lane_id();
-  const bool narrow = !(tt.key & 0x80000000u);
-  const int px = (int)(lane & 7u), py = (int)(lane >> 3);
-  const int nbx = (bx1 - bx0 + 8) >> 3;
-  const int nblk = nbx * ((by1 - by0 + 4) >> 2);
-  for (int j = j0; j < nblk; j += step) {
-    const int bj = j / nbx;
-    const int x8 = bx0 + ((j - bj * nbx) << 3), y4 = by0 + (bj << 2);
-    const int X1 = min(x8 + 7, bx1), Y1 = min(y4 + 3, by1);
-    if (narrow && (edge_min(tt.a01, tt.b01, tt.c01, x8, X1, y4, Y1) >= 0 ||
-                   edge_min(tt.a12, tt.b12, tt.c12, x8, X1, y4, Y1) >= 0 ||
-                   edge_min(tt.a20, tt.b20, tt.c20, x8, X1, y4, Y1) >= 0))
-      continue;
-    const int x = x8 + px, y = y4 + py;
-    const bool c = x <= X1 && y <= Y1 && covers(tt, a.wide, rr, x, y);
-    q.push(c, slot, x - tx0, y - ty0, skey, a, tx0, ty0);
-  }
-}
-
 // Number of raster slices of a tile holding n bin entries of estimated total
 // cost `cost` (kEntryCost per entry plus the boxes of the large ones): about
 // one slice per slice_cost, at most kRasterMaxSlices, at least 4 entries each.
@@ -1432,18 +1313,235 @@ __device__ __forceinline__ uint32_t tile_slices(const FrameArgs& a, uint32_t n, 
   return max(1u, min(min(by_cost, (uint32_t)kRasterMaxSlices), (n + 3u) / 4u));
 }
 
+constexpr int kSegShift = 3;                 // raster units are runs of up to 8 pixels of one row
+constexpr int kSeg = 1 << kSegShift;
+constexpr int kTinyBox = 3;                  // boxes of at most 3 x 3 pixels may stay on their lane
+
+// A warp's share of a batch of bin entries: its narrow triangles, five
+// 16-byte words a slot with the slots side by side (lanes that read different
+// slots hit different banks), with coordinates relative to the tile.
+struct WarpTable {
+  int4 e01[32];      // a01, b01, c01; first pixel x | y << 8 | width << 16 of the box in the tile
+  int4 e12[32];      // a12, b12, c12; order key
+  int4 e20[32];      // a20, b20, c20; min(-w), 0 where some w is not negative
+  float4 d0[32];     // sumf, 1 / sumf, w0, 1 / w0
+  float4 d1[32];     // w1, 1 / w1, w2, 1 / w2
+  int start[32];     // the slot's first unit (INT_MAX: no triangle)
+  uint2 run[32];     // runs with covered pixels of the step: x | y << 8 | slot << 16, first pixel number
+  uint32_t wide[32]; // records of the other triangles
+  int units;         // the table's units
+  int nwide;
+};
+
 template <int TS>
 struct RasterSmem {
   static constexpr int kWarps = RasterShape<TS>::kWarps;
-  static constexpr uint32_t kWideCap = 128;  // queued wide triangles per round
-  static constexpr int kSlots = 64;           // triangle table: 32 lane slots + 32 for wide ones
   __align__(16) unsigned long long skey[TS * RasterShape<TS>::kStride];
-  __align__(16) TriRaster tri[kWarps][kSlots];
-  uint32_t trec[kWarps][kSlots];
-  uint32_t ent[kWarps][64];
-  uint32_t wideq[kWideCap + RasterShape<TS>::kThreads];
-  uint32_t next, nwide, last;
+  __align__(16) WarpTable tab[kWarps];
+  uint32_t last;
 };
+
+// Depth test of a covered pixel: the exact zRec of the reference, then a max
+// of its key (depth_key, with a zRec of -0 made +0 by the subtraction; one
+// below -1 loses to the background key) into the tile's.  The first
+// compare-and-swap uses the key already read, so an uncontended pixel takes
+// one.
+__device__ __forceinline__ void depth_test(unsigned long long* p, const float4& d0, const float4& d1, float wmin,
+                                           int e12, int e20, uint32_t okey) {
+  unsigned long long c = *(volatile unsigned long long*)p;
+  if (depth_beaten(c, wmin)) return;
+  const float al = div_by(__int2float_rn(e12), d0.x, d0.y), be = div_by(__int2float_rn(e20), d0.x, d0.y);
+  const float ga = fs(fs(1.0f, al), be);
+  const float z = fs(0.0f, fa(fa(div_by(al, d0.z, d0.w), div_by(be, d1.x, d1.y)), div_by(ga, d1.z, d1.w)));
+  const uint32_t u = __float_as_uint(z);
+  const unsigned long long k = ((unsigned long long)(u ^ (uint32_t)(((int)u >> 31) | (int)0x80000000)) << 32) | okey;
+  while (k > c) {
+    const unsigned long long old = atomicCAS(p, c, k);
+    if (old == c) break;
+    c = old;
+  }
+}
+
+// Coverage of the n pixels (1 to 8) of a row that starts with edge values
+// e01, e12, e20 and steps a01, a12, a20: the first pixel at bit 31.
+__device__ __forceinline__ unsigned run_coverage(int e01, int e12, int e20, int a01, int a12, int a20, int n) {
+  unsigned cov = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    cov = __funnelshift_l((unsigned)(e01 & e12 & e20), cov, 1);
+    e01 += a01; e12 += a12; e20 += a20;
+  }
+  if (n <= 4) return cov >> (4 - n) << (32 - n);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    cov = __funnelshift_l((unsigned)(e01 & e12 & e20), cov, 1);
+    e01 += a01; e12 += a12; e20 += a20;
+  }
+  return cov >> (8 - n) << (32 - n);
+}
+
+// The calling warp's n <= 32 entries of a batch, one a lane, into its table.
+// With `tiny` (the tile's keys are ready), where at least half of them have
+// boxes of at most kTinyBox x kTinyBox pixels, those lanes depth-test their
+// pixels at once: a unit's bookkeeping costs several times as much as the
+// fraction of a pixel that such a triangle covers on average.
+template <int TS>
+__device__ __forceinline__ void raster_stage(const FrameArgs& a, const DevView& vw, const uint32_t* bin, uint32_t n,
+                                             int tx0, int ty0, int tx1, int ty1, bool tiny, unsigned long long* skey,
+                                             WarpTable& tab) {
+  const unsigned lane = threadIdx.x & 31u;
+  const bool valid = lane < n;
+  uint32_t r = 0;
+  int lx0 = 0, lx1 = -1, ly0 = 0, ly1 = -1;
+  TriRaster t;
+  if (valid) {
+    r = bin[lane];
+    t = unpack_tri(a, r, vw.W, vw.H);
+    lx0 = max((int)t.bx0, tx0); lx1 = min((int)t.bx1, tx1);
+    ly0 = max((int)t.by0, ty0); ly1 = min((int)t.by1, ty1);
+  }
+  const bool live = valid && lx1 >= lx0 && ly1 >= ly0;
+  bool fast = live && narrow_fast(t);
+  const unsigned wm = __ballot_sync(FULL_MASK, live && !fast);
+  if (live && !fast) tab.wide[__popc(wm & ((1u << lane) - 1u))] = r;
+  const int bw = lx1 - lx0 + 1, bh = ly1 - ly0 + 1;
+  if (tiny) {
+    const bool here = fast && bw <= kTinyBox && bh <= kTinyBox;
+    if (__popc(__ballot_sync(FULL_MASK, here)) >= 16) {
+      if (here) {
+        int e01 = t.a01 * lx0 + t.b01 * ly0 + t.c01, e12 = t.a12 * lx0 + t.b12 * ly0 + t.c12,
+            e20 = t.a20 * lx0 + t.b20 * ly0 + t.c20;
+        unsigned cov = 0;  // pixel (x, y) of the box at bit kTinyBox y + x
+#pragma unroll
+        for (int y = 0; y < kTinyBox; ++y)
+#pragma unroll
+          for (int x = 0; x < kTinyBox; ++x) {
+            const int in = (e01 + t.a01 * x + t.b01 * y) & (e12 + t.a12 * x + t.b12 * y) & (e20 + t.a20 * x + t.b20 * y);
+            if (in < 0 && x < bw && y < bh) cov |= 1u << (kTinyBox * y + x);
+          }
+        if (cov) {
+          const float4 d0 = make_float4(t.sumf, __frcp_rn(t.sumf), t.w0, __frcp_rn(t.w0));
+          const float4 d1 = make_float4(t.w1, __frcp_rn(t.w1), t.w2, __frcp_rn(t.w2));
+          const float wmin = fmaxf(fminf(fminf(-t.w0, -t.w1), -t.w2), 0.0f);
+          unsigned long long* const p = skey + (ly0 - ty0) * RasterShape<TS>::kStride + (lx0 - tx0);
+          while (cov) {
+            const int k = __ffs((int)cov) - 1, x = k % kTinyBox, y = k / kTinyBox;
+            cov &= cov - 1u;
+            depth_test(p + y * RasterShape<TS>::kStride + x, d0, d1, wmin, e12 + t.a12 * x + t.b12 * y,
+                       e20 + t.a20 * x + t.b20 * y, t.key);
+          }
+        }
+      }
+      fast = fast && !here;
+    }
+  }
+  const unsigned fm = __ballot_sync(FULL_MASK, fast);
+  const int units = fast ? bh * ((bw + kSeg - 1) >> kSegShift) : 0;
+  const int incl = warp_incl_scan(units);
+  const unsigned slot = __popc(fm & ((1u << lane) - 1u));
+  if (fast) {
+    tab.e01[slot] = make_int4(t.a01, t.b01, t.c01 + t.a01 * tx0 + t.b01 * ty0,
+                              (lx0 - tx0) | (ly0 - ty0) << 8 | bw << 16);
+    tab.e12[slot] = make_int4(t.a12, t.b12, t.c12 + t.a12 * tx0 + t.b12 * ty0, (int)t.key);
+    tab.e20[slot] = make_int4(t.a20, t.b20, t.c20 + t.a20 * tx0 + t.b20 * ty0,
+                              __float_as_int(fmaxf(fminf(fminf(-t.w0, -t.w1), -t.w2), 0.0f)));
+    tab.d0[slot] = make_float4(t.sumf, __frcp_rn(t.sumf), t.w0, __frcp_rn(t.w0));
+    tab.d1[slot] = make_float4(t.w1, __frcp_rn(t.w1), t.w2, __frcp_rn(t.w2));
+    tab.start[slot] = incl - units;
+  }
+  if (lane >= (unsigned)__popc(fm)) tab.start[lane] = 0x7FFFFFFF;
+  if (lane == 31u) {
+    tab.units = incl;
+    tab.nwide = __popc(wm);
+  }
+}
+
+// Units [g0, g0 + 32) of a warp table, by one warp, one a lane: the lane
+// finds its triangle from the start bits, evaluates the three edge functions
+// along its run (exact int32, one addition a pixel an edge) and so knows its
+// covered pixels, which are consecutive.  These are numbered again (a warp
+// scan) and depth-tested 32 at a time, so that the divisions run with every
+// lane busy; runs of nearly equal length are tested by their own lanes
+// instead, one pixel a turn.
+template <int TS>
+__device__ __forceinline__ void raster_units(const WarpTable& tab, uint2* runs, int total, int g0,
+                                             unsigned long long* skey) {
+  constexpr int kStride = RasterShape<TS>::kStride;
+  const unsigned lane = threadIdx.x & 31u;
+  const unsigned upto = FULL_MASK >> (31u - lane);  // lanes <= this one
+  int num = 0, x = 0, y = 0, own = 0;
+  {
+    const int d = tab.start[lane] - g0;  // the slots' first units never decrease
+    const unsigned starts = __reduce_or_sync(FULL_MASK, d >= 0 && d < 32 ? 1u << d : 0u);
+    const int before = __popc(__ballot_sync(FULL_MASK, d < 0));
+    const int g = g0 + (int)lane;
+    if (g < total) {
+      own = before + __popc(starts & upto) - 1;
+      const int4 q0 = tab.e01[own], q1 = tab.e12[own], q2 = tab.e20[own];
+      const int w = q0.w >> 16, u = g - tab.start[own];
+      const int n = (w + kSeg - 1) >> kSegShift;
+      const int row = n == 3 ? (u * 171) >> 9 : u >> (n >> 1);  // u / n for u < 128, n <= 4
+      const int sx = (u - row * n) << kSegShift;
+      x = (q0.w & 0xFF) + sx;
+      y = ((q0.w >> 8) & 0xFF) + row;
+      const unsigned cov = run_coverage(q0.x * x + q0.y * y + q0.z, q1.x * x + q1.y * y + q1.z,
+                                        q2.x * x + q2.y * y + q2.z, q0.x, q1.x, q2.x, min(w - sx, kSeg));
+      num = __popc(cov);
+      x += __clz((int)cov);
+    }
+  }
+  const int incl = warp_incl_scan(num);
+  const int pixels = __shfl_sync(FULL_MASK, incl, 31);
+  const int longest = __reduce_max_sync(FULL_MASK, num);
+  if (2 * longest <= 3 * ((pixels + 31) >> 5)) {
+    if (num) {
+      const int4 q1 = tab.e12[own], q2 = tab.e20[own];
+      const float4 d0 = tab.d0[own], d1 = tab.d1[own];
+      int e12 = q1.x * x + q1.y * y + q1.z, e20 = q2.x * x + q2.y * y + q2.z;
+      unsigned long long* p = skey + y * kStride + x;
+      for (int k = 0; k < num; ++k, ++p) {
+        depth_test(p, d0, d1, __int_as_float(q2.w), e12, e20, (uint32_t)q1.w);
+        e12 += q1.x;
+        e20 += q2.x;
+      }
+    }
+    return;
+  }
+  const unsigned some = __ballot_sync(FULL_MASK, num != 0);
+  const int excl = incl - num;
+  if (num) runs[__popc(some & (upto >> 1))] = make_uint2((uint32_t)(x | y << 8 | own << 16), (uint32_t)excl);
+  __syncwarp();
+  for (int h0 = 0; h0 < pixels; h0 += 32) {
+    const int d = excl - h0;
+    const unsigned starts = __reduce_or_sync(FULL_MASK, num != 0 && d >= 0 && d < 32 ? 1u << d : 0u);
+    const int before = __popc(__ballot_sync(FULL_MASK, num != 0 && d < 0));
+    const int h = h0 + (int)lane;
+    if (h < pixels) {
+      const uint2 q = runs[before + __popc(starts & upto) - 1];
+      const int px = (int)(q.x & 0xFFu) + h - (int)q.y, py = (int)((q.x >> 8) & 0xFFu), s = (int)(q.x >> 16);
+      const int4 q1 = tab.e12[s], q2 = tab.e20[s];
+      depth_test(skey + py * kStride + px, tab.d0[s], tab.d1[s], __int_as_float(q2.w), q1.x * px + q1.y * py + q1.z,
+                 q2.x * px + q2.y * py + q2.z, (uint32_t)q1.w);
+    }
+  }
+  __syncwarp();  // the runs are rewritten by the next step
+}
+
+// A triangle that the units do not take (int64 edges, or W's out of
+// narrow_fast's range): the CTA's warps share the 8 x 4 blocks of its box.
+template <int TS>
+__device__ __forceinline__ void raster_wide(const FrameArgs& a, const DevView& vw, uint32_t r, int tx0, int ty0,
+                                            int tx1, int ty1, unsigned long long* skey) {
+  const unsigned lane = threadIdx.x & 31u;
+  const TriRaster t = unpack_tri(a, r, vw.W, vw.H);
+  const int bx0 = max((int)t.bx0, tx0), bx1 = min((int)t.bx1, tx1);
+  const int by0 = max((int)t.by0, ty0), by1 = min((int)t.by1, ty1);
+  const int nbx = (bx1 - bx0 + 8) >> 3, nblk = nbx * ((by1 - by0 + 4) >> 2);
+  for (int j = (int)(threadIdx.x >> 5); j < nblk; j += RasterShape<TS>::kWarps) {
+    const int x = bx0 + (j % nbx) * 8 + (int)(lane & 7u), y = by0 + (j / nbx) * 4 + (int)(lane >> 3);
+    if (x <= bx1 && y <= by1 && covers(t, a.wide, r, x, y)) depth_candidate<TS>(skey, t, a.wide, r, x, y, tx0, ty0);
+  }
+}
 
 // Final colour and depth of pixel (x, y) of view vw whose visibility key is k:
 // deferred shading of the winning triangle (rasterizer.go:149-176), or Clear
@@ -1536,20 +1634,23 @@ __device__ __forceinline__ void resolve_pixel(const FrameArgs& a, const DevView&
 }
 
 // One raster work item: slice `slice` of global tile `tile` of view `view`.
+// The slice's bin entries go in batches of one a thread.  The warps stage a
+// batch in equal shares and then take its groups of 32 units in turn, so that
+// a batch of few large triangles and one of many small ones keep all of them
+// busy.  Bound by issue (45-63 % of the slots) and, in small frames, by the
+// latency of one tile.  k_raster before (each warp rasterised the entries that
+// it had taken, and waited at the end of the slice for a third to two thirds
+// of its time; spans narrowed by division; branching divisions) and now:
+// 199,712-triangle terrain at 1280x720 92 -> 54 us, 81,920-triangle icosphere
+// at 1920x1080 40 -> 31, 960-triangle sphere at 640x360 28 -> 18, a box that
+// fills 3840x2160 235 -> 87, 5.0 M-triangle icospheres 124 -> 79.
 template <int TS>
 __device__ __forceinline__ void raster_item(const FrameArgs& a, uint32_t tile, uint32_t slice, int view,
                                             RasterSmem<TS>& sm) {
   constexpr int kThreads = RasterShape<TS>::kThreads;
   constexpr int kStride = RasterShape<TS>::kStride;
   constexpr int kWarps = RasterShape<TS>::kWarps;
-  constexpr uint32_t kWideCap = RasterSmem<TS>::kWideCap;
   unsigned long long* skey = sm.skey;
-  auto& s_tri = sm.tri;
-  auto& s_trec = sm.trec;
-  auto& s_ent = sm.ent;
-  uint32_t* s_wideq = sm.wideq;
-  uint32_t& s_next = sm.next;
-  uint32_t& s_nwide = sm.nwide;
   uint32_t& s_last = sm.last;
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -1566,158 +1667,47 @@ __device__ __forceinline__ void raster_item(const FrameArgs& a, uint32_t tile, u
   const int ty0 = (int)(lt / (uint32_t)vw.tiles_x) * TS;
   const int tx1 = min(tx0 + TS - 1, vw.W - 1);
   const int ty1 = min(ty0 + TS - 1, vw.H - 1);
+  // this thread's four pixels of a row, where the tile's keys are set, stored or shaded
+  constexpr int kPerRow = TS / 4;
+  const int row = tid / kPerRow;
+  const int col = (tid % kPerRow) * 4;
+  unsigned long long* const mine = skey + row * kStride + col;
 
-  // A tile with no bin entry is all background: with the resolve in this
-  // kernel it needs no keys and goes straight to it (Clear + DotGrid,
-  // overlays, crosshair, fog).  Measured: a 256-view batch 5 % faster; for
-  // frames shaded by k_resolve the short cut did not pay (their empty tiles
-  // still store background keys the ordinary way).
-  const bool empty = n == 0 && !a.pkey;
+  // A tile with no bin entry is all background: it needs no keys and goes
+  // straight to the resolve (Clear + DotGrid, overlays, crosshair, fog).
+  const bool empty = n == 0;
   if (!empty) {
-    for (int i = tid; i < TS * kStride; i += kThreads) skey[i] = BG_KEY;
-    if (tid == 0) {
-      s_next = lo;
-      s_nwide = 0;
-    }
-    __syncthreads();
-
     const unsigned lane = lane_id();
     const uint32_t* bin = a.bins + (size_t)tile * a.bin_cap;
-    TriRaster* tri = s_tri[warp];
-    uint32_t* trec = s_trec[warp];
-    CandQueue<TS> q{s_ent[warp], tri, trec, 0};
-    // Entries per warp chunk: small bins use shorter chunks so that every warp
-    // gets some (the span walk below keeps all lanes busy either way).
-    const uint32_t chunk = min(32u, max(8u, (hi - lo + 2u * kWarps - 1u) / (2u * kWarps)));
-    for (;;) {
-      // Phase 1: warps take `chunk` bin entries at a time from a shared cursor.
-      // Narrow triangles are walked by the warp that took them (span walk
-      // below); int64 ("wide") triangles are queued for the whole CTA.
-      for (;;) {
-        if (*(volatile uint32_t*)&s_nwide >= kWideCap) break;
-        uint32_t b = 0;
-        if (lane == 0) b = atomicAdd(&s_next, chunk);
-        b = __shfl_sync(FULL_MASK, b, 0);
-        if (b >= hi) break;
-        const uint32_t i = b + lane;
-        const bool valid = lane < chunk && i < hi;
-        uint32_t r = 0;
-        int lx0 = 0, lx1 = -1, ly0 = 0, ly1 = -1;
-        TriRaster t;
-        if (valid) {
-          r = bin[i];
-          t = unpack_tri(a, r, vw.W, vw.H);
-          lx0 = max((int)t.bx0, tx0); lx1 = min((int)t.bx1, tx1);
-          ly0 = max((int)t.by0, ty0); ly1 = min((int)t.by1, ty1);
-        }
-        const bool live = valid && lx1 >= lx0 && ly1 >= ly0;
-        const int area = live ? (lx1 - lx0 + 1) * (ly1 - ly0 + 1) : 0;
-        const bool by_lane = live && !(t.key & 0x80000000u);
-        const bool wide = live && !by_lane;
-        const unsigned lm = __ballot_sync(FULL_MASK, wide);
-        if (lm) {
-          uint32_t qb = 0;
-          const int ldr = __ffs(lm) - 1;
-          if ((int)lane == ldr) qb = atomicAdd(&s_nwide, (uint32_t)__popc(lm));
-          qb = __shfl_sync(FULL_MASK, qb, ldr);
-          if (wide) s_wideq[qb + __popc(lm & ((1u << lane) - 1u))] = r;
-        }
-        if (by_lane) {
-          tri[lane] = t;
-          trec[lane] = r;
-        }
-        // Span walk.  The chunk's (triangle, footprint row) pairs are numbered
-        // consecutively (a warp scan of the row counts), 32 rows per step; each
-        // lane narrows its row to the exact covered x-range, and the covered
-        // pixels of the 32 spans are numbered again and depth-tested 32 at a
-        // time, so no lane tests a pixel that the triangle does not cover.
-        // Chunks of tiny footprints take the per-lane box walk instead.
-        const int my = by_lane ? ly1 - ly0 + 1 : 0;
-        const int incl = warp_incl_scan(my);
-        const int excl = incl - my;
-        const int total = __shfl_sync(FULL_MASK, incl, 31);
-        const int widest = __reduce_max_sync(FULL_MASK, by_lane ? area : 0);
-        __syncwarp();
-        if (widest * 5 <= ((total + 31) >> 5) * 27) {
-          // Footprints of a few pixels: a span costs about five box-pixel tests,
-          // so each lane tests its own box, queueing covered pixels.
-          int x = lx0, y = ly0;
-          for (int it = 0; it < widest; ++it) {
-            const bool c = by_lane && it < area && t.a01 * x + t.b01 * y + t.c01 < 0 &&
-                           t.a12 * x + t.b12 * y + t.c12 < 0 && t.a20 * x + t.b20 * y + t.c20 < 0;
-            q.push(c, lane, x - tx0, y - ty0, skey, a, tx0, ty0);
-            if (++x > lx1) {
-              x = lx0;
-              ++y;
-            }
-          }
-          q.flush(skey, a, tx0, ty0);
-          continue;
-        }
-        for (int g0 = 0; g0 < total; g0 += 32) {
-          const int g = g0 + (int)lane;
-          const int own = owner_lane(excl, g);
-          const int y = __shfl_sync(FULL_MASK, ly0, own) + g - __shfl_sync(FULL_MASK, excl, own);
-          int xl = __shfl_sync(FULL_MASK, lx0, own), xr = __shfl_sync(FULL_MASK, lx1, own);
-          if (g < total) {
-            const TriRaster& tt = tri[own];
-            span_edge(tt.a01, tt.b01, tt.c01, y, xl, xr);
-            span_edge(tt.a12, tt.b12, tt.c12, y, xl, xr);
-            span_edge(tt.a20, tt.b20, tt.c20, y, xl, xr);
-          } else {
-            xr = xl - 1;
-          }
-          const int len = max(xr - xl + 1, 0);
-          const int incl2 = warp_incl_scan(len);
-          const int excl2 = incl2 - len;
-          const int total2 = __shfl_sync(FULL_MASK, incl2, 31);
-          // two pixels a lane per pass: their depth tests are independent
-          // chains of divisions that overlap
-          for (int h0 = 0; h0 < total2; h0 += 64) {
-            const int ha = h0 + (int)lane, hb = ha + 32;
-            const int oa = owner_lane(excl2, ha), ob = owner_lane(excl2, hb);
-            const int xa = __shfl_sync(FULL_MASK, xl, oa) + ha - __shfl_sync(FULL_MASK, excl2, oa);
-            const int xb = __shfl_sync(FULL_MASK, xl, ob) + hb - __shfl_sync(FULL_MASK, excl2, ob);
-            const int ya = __shfl_sync(FULL_MASK, y, oa), yb = __shfl_sync(FULL_MASK, y, ob);
-            const int sa = __shfl_sync(FULL_MASK, own, oa), sb = __shfl_sync(FULL_MASK, own, ob);
-            if (ha < total2) depth_covered<TS>(skey, tri[sa], xa, ya, tx0, ty0);
-            if (hb < total2) depth_covered<TS>(skey, tri[sb], xb, yb, tx0, ty0);
-          }
-        }
-        __syncwarp();  // lane slots are rewritten by the next chunk
+    *reinterpret_cast<ulonglong2*>(mine) = make_ulonglong2(BG_KEY, BG_KEY);
+    *reinterpret_cast<ulonglong2*>(mine + 2) = make_ulonglong2(BG_KEY, BG_KEY);
+    // no box of the tile beyond kSmallBox pixels: the tile may be one of tiny triangles
+    const bool tiny = ti.w == 0u && n >= 64u;
+    if (tiny) __syncthreads();  // raster_stage tests pixels too
+    for (uint32_t base = lo; base < hi; base += kThreads) {
+      const uint32_t m = min((uint32_t)kThreads, hi - base);
+      const uint32_t share = (m + kWarps - 1) / kWarps;  // entries a warp, at most 32
+      if ((uint32_t)warp * share < m) {
+        raster_stage<TS>(a, vw, bin + base + (uint32_t)warp * share, min(share, m - (uint32_t)warp * share), tx0, ty0,
+                         tx1, ty1, tiny, skey, sm.tab[warp]);
+      } else if (lane == 0) {
+        sm.tab[warp].units = 0;
+        sm.tab[warp].nwide = 0;
       }
       __syncthreads();
-      const uint32_t nl = s_nwide;
-      const bool more = s_next < hi;
-      // Phase 2: every warp walks the queued wide triangles and takes an
-      // interleaved share of their 8x4 blocks (global block index mod warps).
-      int base = 0;
-      for (uint32_t k = 0; k < nl; ++k) {
-        const uint32_t slot = 32u + (k & 31u);
-        if ((k & 31u) == 0) {
-          // slots 32..63 are about to be reused: drain, then stage the next 32
-          // wide records with one load per lane
-          q.flush(skey, a, tx0, ty0);
-          if (k + lane < nl) {
-            const uint32_t r2 = s_wideq[k + lane];
-            tri[32 + lane] = unpack_tri(a, r2, vw.W, vw.H);
-            trec[32 + lane] = r2;
-          }
-          __syncwarp();
-        }
-        const TriRaster tt = tri[slot];
-        const uint32_t rr = trec[slot];
-        const int bx0 = max((int)tt.bx0, tx0), bx1 = min((int)tt.bx1, tx1);
-        const int by0 = max((int)tt.by0, ty0), by1 = min((int)tt.by1, ty1);
-        const int nblk = ((bx1 - bx0 + 8) >> 3) * ((by1 - by0 + 4) >> 2);
-        const int j0 = (warp - base + kWarps) % kWarps;
-        walk_blocks<TS>(q, skey, a, tt, rr, slot, bx0, bx1, by0, by1, j0, kWarps, tx0, ty0);
-        base = (base + nblk) % kWarps;
+      // the batch's groups of 32 units, table by table: lane l < kWarps holds
+      // the number of groups up to table l
+      const int groups = warp_incl_scan(lane < (unsigned)kWarps ? (sm.tab[lane].units + 31) >> 5 : 0);
+      const int all = __shfl_sync(FULL_MASK, groups, kWarps - 1);
+      for (int g = warp; g < all; g += kWarps) {
+        const int seg = __popc(__ballot_sync(FULL_MASK, lane < (unsigned)kWarps && groups <= g));
+        const int prev = __shfl_sync(FULL_MASK, groups, (seg + 31) & 31);
+        raster_units<TS>(sm.tab[seg], sm.tab[warp].run, sm.tab[seg].units, (g - (seg ? prev : 0)) << 5, skey);
       }
-      q.flush(skey, a, tx0, ty0);
-      __syncthreads();
-      if (!more) break;
-      if (tid == 0) s_nwide = 0;
+      if (__ballot_sync(FULL_MASK, lane < (unsigned)kWarps && sm.tab[lane].nwide != 0)) {
+        for (int w = 0; w < kWarps; ++w)
+          for (int k = 0; k < sm.tab[w].nwide; ++k) raster_wide<TS>(a, vw, sm.tab[w].wide[k], tx0, ty0, tx1, ty1, skey);
+      }
       __syncthreads();
     }
 
@@ -1727,55 +1717,55 @@ __device__ __forceinline__ void raster_item(const FrameArgs& a, uint32_t tile, u
       // kernel boundary orders them, so no slice waits on a fence or hands
       // over (the merge below took a fifth of this kernel's warp time on
       // single frames).
-      unsigned long long* dst = a.slot_keys + (size_t)(ti.z + slice) * (TS * TS);
-      for (int i = tid; i < TS * TS; i += kThreads) dst[i] = skey[(i / TS) * kStride + (i % TS)];
+      ulonglong2* dst = reinterpret_cast<ulonglong2*>(a.slot_keys + (size_t)(ti.z + slice) * (TS * TS) + row * TS + col);
+      dst[0] = *reinterpret_cast<const ulonglong2*>(mine);
+      dst[1] = *reinterpret_cast<const ulonglong2*>(mine + 2);
       return;
     }
     if (nslices > 1) {
       // Merge this slice's keys into the tile's global keys; the last slice to
       // arrive resolves the tile and returns the global keys to zero (zero is
       // below every key, since no key encodes a NaN depth).
-      unsigned long long* g = a.gkey + (size_t)tile * (TS * TS);
-      for (int i = tid; i < TS * TS; i += kThreads) {
-        const unsigned long long k = skey[(i / TS) * kStride + (i % TS)];
-        if (k != BG_KEY) atomicMax(g + i, k);
-      }
+      unsigned long long* g = a.gkey + (size_t)tile * (TS * TS) + row * TS + col;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (mine[j] != BG_KEY) atomicMax(g + j, mine[j]);
       __threadfence();
       __syncthreads();
       if (tid == 0) s_last = atomicAdd(&a.tile_done[tile], 1u) == nslices - 1 ? 1u : 0u;
       __syncthreads();
       if (!s_last) return;
       __threadfence();
-      for (int i = tid; i < TS * TS; i += kThreads) {
-        const unsigned long long k = *(volatile unsigned long long*)(g + i);
-        skey[(i / TS) * kStride + (i % TS)] = k > BG_KEY ? k : BG_KEY;
-        g[i] = 0ull;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const unsigned long long k = *(volatile unsigned long long*)(g + j);
+        mine[j] = k > BG_KEY ? k : BG_KEY;
+        g[j] = 0ull;
       }
       if (tid == 0) a.tile_done[tile] = 0u;
-      __syncthreads();
     }
   }
 
+  const int x = tx0 + col, y = ty0 + row;
   if (a.pkey) {
-    // the tile's final keys, shaded by k_resolve
-    for (int i = tid; i < TS * TS; i += kThreads) {
-      const int rr = i / TS, cc = i % TS;
-      const int x = tx0 + cc, y = ty0 + rr;
-      if (x <= tx1 && y <= ty1)
-        a.pkey[vw.pix_base + (size_t)y * (size_t)vw.W + (size_t)x] = empty ? BG_KEY : skey[rr * kStride + cc];
+    // the tile's final keys, shaded by k_resolve (which takes a tile without entries for background)
+    if (!empty && y <= ty1) {
+      unsigned long long* dst = a.pkey + vw.pix_base + (size_t)y * (size_t)vw.W + (size_t)x;
+      if (vw.vec_ok && x + 3 <= tx1) {  // a row's pixels start at a multiple of 4: 16-byte stores
+        reinterpret_cast<ulonglong2*>(dst)[0] = *reinterpret_cast<const ulonglong2*>(mine);
+        reinterpret_cast<ulonglong2*>(dst)[1] = *reinterpret_cast<const ulonglong2*>(mine + 2);
+      } else {
+        for (int j = 0; j < 4 && x + j <= tx1; ++j) dst[j] = mine[j];
+      }
     }
   } else {
     // Resolve + deferred shading, four pixels a thread
-    constexpr int kPerRow = TS / 4;
-    const int row = tid / kPerRow;
-    const int col = (tid % kPerRow) * 4;
-    const int y = ty0 + row;
     if (y <= ty1) {
       uint32_t out_c[4];
       float out_z[4];
       unsigned long long keys[4] = {BG_KEY, BG_KEY, BG_KEY, BG_KEY};
       if (!empty) {
-        const ulonglong2* kp = reinterpret_cast<const ulonglong2*>(skey + row * kStride + col);
+        const ulonglong2* kp = reinterpret_cast<const ulonglong2*>(mine);
         const ulonglong2 k01 = kp[0], k23 = kp[1];
         keys[0] = k01.x; keys[1] = k01.y; keys[2] = k23.x; keys[3] = k23.y;
       }
@@ -1783,9 +1773,8 @@ __device__ __forceinline__ void raster_item(const FrameArgs& a, uint32_t tile, u
       for (int j = 0; j < 4; ++j) {
         out_c[j] = 0u;
         out_z[j] = 0.0f;
-        if (tx0 + col + j <= tx1) resolve_pixel(a, vw, tx0 + col + j, y, keys[j], out_c[j], out_z[j]);
+        if (x + j <= tx1) resolve_pixel(a, vw, x + j, y, keys[j], out_c[j], out_z[j]);
       }
-      const int x = tx0 + col;
       const size_t o = (size_t)y * (size_t)vw.W + (size_t)x;
       const bool with_z = !(vw.flags & kViewFaceIds);  // face-id views output no depth
       if (vw.vec_ok && x + 3 <= tx1) {
@@ -1900,7 +1889,8 @@ __global__ void __launch_bounds__(256) k_plan(const FrameArgs a) {
   __syncthreads();
   const bool valid = tile < a.total_tiles;
   const uint32_t count = valid ? a.bin_count[tile] : 0u;
-  const uint32_t cost = valid ? count * (uint32_t)kEntryCost + a.tile_cost[tile] : 0u;
+  const uint32_t boxes = valid ? a.tile_cost[tile] : 0u;
+  const uint32_t cost = valid ? count * (uint32_t)kEntryCost + boxes / 2u : 0u;
   const uint32_t ns = valid ? tile_slices(a, min(count, a.bin_cap), cost) : 0u;
   if (valid) {  // the bins are complete: ready for the next frame's appends
     a.bin_count[tile] = 0u;
@@ -1923,10 +1913,13 @@ __global__ void __launch_bounds__(256) k_plan(const FrameArgs a) {
   // A tile without bin entries of a batch shaded in place goes to the list
   // of tiles to clear instead of the raster queue: all background, no keys.
   const bool clear = count == 0 && a.clear_empty;
+  // One of a frame shaded by k_resolve needs no work item at all.
+  const bool none = count == 0 && a.pkey;
   uint32_t mf = 0, mb = 0, me = 0;
   if (valid) {
     atomicMax(&s_max, count);
     if (clear) me = atomicAdd(&s_ne, 1u);
+    else if (none) {}
     else if (heavy) mf = atomicAdd(&s_nf, ns);
     else mb = atomicAdd(&s_nb, 1u);
   }
@@ -1947,9 +1940,10 @@ __global__ void __launch_bounds__(256) k_plan(const FrameArgs a) {
   // it the latter 1 % slower).
   const uint32_t slot =
       heavy && ns > 1 && ns <= 8u && a.slot_keys && s_bf + mf + ns <= a.slot_cap ? s_bf + mf : kNoSlot;
-  a.tile_info[tile] = make_uint4(min(count, a.bin_cap), ns, slot, 0u);
+  a.tile_info[tile] = make_uint4(min(count, a.bin_cap), ns, slot, boxes);
   if (clear) {
     if (s_be + me < a.empty_cap) a.empty_tiles[s_be + me] = make_uint2(tile, (uint32_t)view);
+  } else if (none) {
   } else if (heavy) {
     for (uint32_t k = 0; k < ns; ++k) a.plan[s_bf + mf + k] = make_uint2(tile, k | vbits);
   } else {
@@ -2095,6 +2089,7 @@ __global__ void __launch_bounds__(256) k_resolve(const FrameArgs a) {
     k = sk[0];
     for (uint32_t s = 1; s < ti.y; ++s) k = max(k, sk[(size_t)s * (size_t)(ts * ts)]);
   }
+  if (ti.x == 0) k = BG_KEY;  // a tile without entries: k_raster stored no keys
   uint32_t c;
   float z;
   resolve_pixel(a, vw, x, y, k, c, z);

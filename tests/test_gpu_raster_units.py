@@ -1,0 +1,71 @@
+"""The raster's unit walk at the sizes where it can go wrong, bit for bit
+against the oracle: bins of one entry, of a whole batch and of one more (256
+entries at 32 x 32 tiles, 64 at 16 x 16), tiles of tiny triangles (at most 3 x 3
+pixels, points and slivers among them), boxes one pixel either side of a unit
+(8 pixels) and of a tile, slices without entries, W's beyond the range of
+the exact division (the general path), and their mixtures."""
+import numpy as np
+import pytest
+
+import gorender_gb300 as gr
+from gorender_gb300 import _native as N
+from gorender_gb300 import scenes
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+FLAGS = (gr.FLAGS_DEFAULT | gr.FLAT_SHADING) & ~gr.BACKFACE_CULLING
+
+
+def _scene(size, n, seed, w=130, h=70, far=1.0):
+    """n triangles of about `size` pixels over the frame, both windings, a
+    fifth of them copies (depth ties); far scales the scene, and with it W."""
+    rng = scenes.SplitMix64(seed)
+    c = rng.uniform(3 * n, -1.0, 1.0).reshape(n, 1, 3) * np.array([1.1, 0.6, 0.3], np.float32)
+    tri = c + rng.uniform(9 * n, -0.5, 0.5).reshape(n, 3, 3) * np.float32(size * 1.16 / h)
+    copies = np.arange(0, n, 5)[1:]
+    tri[copies] = tri[copies - 1]
+    pos = np.ones((3 * n, 4), np.float32)
+    pos[:, :3] = tri.reshape(-1, 3) * np.float32(far)
+    m = scenes.MeshData(pos=pos, vidx=np.arange(3 * n, dtype=np.int32).reshape(n, 3))
+    cam = scenes.CameraData((0.0, 0.0, far), (0.0, 0.0, -1.0), (0.0, 1.0, 0.0))
+    return scenes.SceneData("units", w, h, [scenes.ObjectData(m)], cam, [], FLAGS)
+
+
+@pytest.mark.parametrize("tile", [32, 16])
+@pytest.mark.parametrize("size,n", [(1, 3000), (2, 6000), (3, 2500), (7, 900), (9, 700), (30, 257), (34, 64), (80, 65),
+                                    (400, 1), (400, 9), (400, 300)])
+def test_units(tile, size, n):
+    ctx = gr.Context(0)
+    try:
+        ctx.set_tuning(tile, 0)
+        sc = _scene(size, n, seed=3 + 10 * size + n)
+        for cost in (1 << 20, 64):  # one slice a tile, and as many as there can be
+            N.check(N.lib().gr_context_set_raster(ctx.handle, cost, 0))
+            up = gr.UploadedScene(ctx, sc)
+            rgba, z, tpf = up.render()
+            ref = oracle.draw_scene(sc, items_override=up.matrices, nthreads=4)
+            assert ref[3] == 0 and tpf == ref[2]
+            assert np.array_equal(rgba, ref[0])
+            assert np.array_equal(z.view(np.uint32), ref[1].view(np.uint32))
+            assert (z > -1).any()
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("far", [2.0 ** -58, 2.0 ** -63])
+def test_units_and_general_path_by_w(far):
+    """W's of about 2^-58 take the units, of 2^-63 the general path; clipping
+    is off (the planes stand at W's of 1) and the depths are huge."""
+    ctx = gr.Context(0)
+    try:
+        sc = _scene(20, 200, seed=7, far=far)
+        sc.flags &= ~gr.FRUSTUM_CLIPPING
+        up = gr.UploadedScene(ctx, sc)
+        rgba, z, tpf = up.render()
+        ref = oracle.draw_scene(sc, items_override=up.matrices, nthreads=4)
+        assert ref[3] == 0 and tpf == ref[2]
+        assert np.array_equal(rgba, ref[0]) and np.array_equal(z.view(np.uint32), ref[1].view(np.uint32))
+        assert (z > -1).any()
+    finally:
+        ctx.close()
