@@ -125,6 +125,7 @@ struct gr_context {
   uint32_t tiles_cap = 0;
   uint2* big = nullptr;             // multi-tile queue: (record, view)
   uint32_t big_cap = 0;
+  uint2* huge = nullptr;            // huge triangles' list, kHugeCap entries
   unsigned long long* gkey = nullptr;  // merged keys of tiles split over several CTAs
   uint32_t* tile_done = nullptr;
   uint32_t gkey_tiles = 0;
@@ -656,6 +657,7 @@ int32_t prepare(gr_context* c, const ViewIn* views, int nviews, const gr_draw_it
   a.bin_count = c->bin_count;
   a.tile_cost = c->tile_cost;
   a.big = c->big;
+  a.huge = c->huge;
   a.gkey = c->gkey;
   a.tile_done = c->tile_done;
   a.slice_cost = c->slice_cost;
@@ -918,6 +920,7 @@ int32_t gr_context_create(int32_t device, gr_context** out) {
   cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->work, sizeof(DevWork));
   if (e == cudaSuccess) e = cudaMemset(c->work, 0, sizeof(DevWork));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&c->huge, sizeof(uint2) * kHugeCap);
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_result, sizeof(DevResult));
   if (e == cudaSuccess) e = cudaMemset(c->d_result, 0, sizeof(DevResult));
   if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_result, 2 * sizeof(DevResult));  // + the done word
@@ -954,7 +957,7 @@ int32_t gr_context_destroy(gr_context* c) {
   if (c->h_tables) cudaFreeHost(c->h_tables);
   dev_free(c->rast); dev_free(c->shade); dev_free(c->suv); dev_free(c->wide); dev_free(c->tcol);
   dev_free(c->rec_of_face); dev_free(c->bins); dev_free(c->bin_count); dev_free(c->tile_cost); dev_free(c->tile_info);
-  dev_free(c->big);
+  dev_free(c->big); dev_free(c->huge);
   dev_free(c->gkey); dev_free(c->tile_done); dev_free(c->clip); dev_free(c->kept); dev_free(c->vlight);
   dev_free(c->vclip); dev_free(c->vscr);
   dev_free(c->view_tpf); dev_free(c->view_tpf_out); dev_free(c->plan); dev_free(c->empty_tiles);

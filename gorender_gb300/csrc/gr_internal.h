@@ -23,6 +23,13 @@ __host__ __device__ constexpr int project_faces_per_lane(unsigned long long face
   return faces >= 2000000ull ? 4 : faces >= 1000000ull ? 2 : 1;
 }
 constexpr int kBinDirectMax = 4;              // triangles spanning <= 4 tiles bin directly
+// Triangles over more tiles than this are binned by k_plan, each tile's thread
+// looking at all of them: a warp alone takes about 1 us for every 32 tiles, so
+// 8 us at the line; a thread of k_plan about 0.04 us a triangle, so 40 us for a
+// full list (further ones are binned by a warp).
+constexpr int kHugeTiles = 256;
+constexpr int kHugeCap = 1024;
+constexpr int kHugeBatch = 128;               // huge triangles k_plan stages at once
 constexpr int kStageSlots = 3;                // pinned staging slots for back-to-back async draws
 constexpr int kRasterMaxSlices = 32;          // CTAs that may share one tile's bin
 static_assert(kRasterMaxSlices <= 32, "a raster work item packs its slice into 5 bits");
@@ -234,6 +241,7 @@ struct DevWork {
   unsigned int novl, ovl_need;      // overlay records written / needed
   unsigned int nempty, clear_next;  // tiles without bin entries (k_plan); the next one k_raster clears
   unsigned int nkept;               // faces k_cull kept whole, for k_setup
+  unsigned int nhuge;               // triangles offered to the list of huge ones (up to kHugeCap are in it)
 };
 
 struct alignas(8) DevResult {
@@ -272,6 +280,7 @@ struct FrameArgs {
   uint32_t* bin_count;              // per tile: entries
   uint32_t* tile_cost;              // per tile: tile-clipped box pixels of entries larger than kSmallBox
   uint2* big;                       // multi-tile queue: (record, view)
+  uint2* huge;                      // huge triangles, binned by k_plan: (record, view), kHugeCap entries
   uint2* clip;                      // (item, face) pairs for the general clipper
   uint32_t clip_cap;
   uint2* kept;                      // (item, face) of the faces k_cull kept whole; k_setup writes

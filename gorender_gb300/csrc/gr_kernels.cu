@@ -14,7 +14,7 @@
 //              (__match_any_sync) or, past four tiles, queued for k_bin_big.
 //   k_bin_big  one warp per multi-tile triangle: appends it to every tile its
 //              edge functions can reach.
-//   k_plan     splits heavy tiles into slices by estimated cost and orders
+//   k_plan     bins the few huge triangles, a tile a thread; splits heavy tiles into slices by estimated cost and orders
 //              the work queue heaviest first.
 //   k_raster   persistent CTAs over the queue, one TS x TS tile slice each:
 //              visibility in shared memory as a 64-bit max of (ordered zRec,
@@ -570,32 +570,50 @@ __device__ __forceinline__ bool bin_record_direct(const FrameArgs& a, uint32_t r
   return false;
 }
 
+// Tiles of a triangle's box.
+__device__ __forceinline__ uint32_t box_tiles(const TriRaster& t, int sh) {
+  return (((uint32_t)t.bx1 >> sh) - ((uint32_t)t.bx0 >> sh) + 1u) * (((uint32_t)t.by1 >> sh) - ((uint32_t)t.by0 >> sh) + 1u);
+}
+
+// Whether narrow triangle t may cover a pixel of tile (tx, ty): none of its
+// edges excludes the tile-clipped box entirely (the exact int32 edge minimum
+// over it is < 0).
+__device__ __forceinline__ bool reaches_tile(const TriRaster& t, uint32_t tx, uint32_t ty, int sh) {
+  const int ts = 1 << sh;
+  const int X0 = max((int)(tx << sh), (int)t.bx0);
+  const int X1 = min((int)(tx << sh) + ts - 1, (int)t.bx1);
+  const int Y0 = max((int)(ty << sh), (int)t.by0);
+  const int Y1 = min((int)(ty << sh) + ts - 1, (int)t.by1);
+  return t.c01 + min(t.a01 * X0, t.a01 * X1) + min(t.b01 * Y0, t.b01 * Y1) < 0 &&
+         t.c12 + min(t.a12 * X0, t.a12 * X1) + min(t.b12 * Y0, t.b12 * Y1) < 0 &&
+         t.c20 + min(t.a20 * X0, t.a20 * X1) + min(t.b20 * Y0, t.b20 * Y1) < 0;
+}
+
+// Puts the record of a triangle over more than kHugeTiles tiles into the list
+// that k_plan bins; false where the list is full (it is binned like others
+// then).
+__device__ __forceinline__ bool queue_huge(const FrameArgs& a, uint32_t ntiles, uint32_t r, int view) {
+  if (ntiles <= (uint32_t)kHugeTiles) return false;
+  const uint32_t q = atomicAdd(&a.work->nhuge, 1u);
+  if (q >= (uint32_t)kHugeCap) return false;
+  a.huge[q] = make_uint2(r, (uint32_t)view);
+  return true;
+}
+
 // One warp appends record r (view `view`) to every tile its box overlaps,
-// lanes over the tiles; a narrow triangle skips tiles that one of its edges
-// excludes entirely (the exact int32 edge minimum over the tile-clipped box
-// is >= 0).  All lanes of the warp must call it with the same r.
+// lanes over the tiles; a narrow triangle skips tiles that it does not reach.
+// All lanes of the warp must call it with the same r.
 __device__ __forceinline__ void bin_tiles_warp(const FrameArgs& a, uint32_t r, int view) {
   const int sh = a.tile_shift;
-  const int ts = 1 << sh;
   const uint32_t lane = threadIdx.x & 31u;
   const DevView& vw = a.views[view];
   const TriRaster t = unpack_tri(a, r, vw.W, vw.H);
-  const uint32_t tx0 = (uint32_t)t.bx0 >> sh, tx1 = (uint32_t)t.bx1 >> sh;
-  const uint32_t ty0 = (uint32_t)t.by0 >> sh, ty1 = (uint32_t)t.by1 >> sh;
-  const uint32_t nx = tx1 - tx0 + 1, n = nx * (ty1 - ty0 + 1);
+  const uint32_t tx0 = (uint32_t)t.bx0 >> sh, ty0 = (uint32_t)t.by0 >> sh;
+  const uint32_t nx = ((uint32_t)t.bx1 >> sh) - tx0 + 1, n = box_tiles(t, sh);
   const bool wide = (t.key & 0x80000000u) != 0;
   for (uint32_t j = lane; j < n; j += 32u) {
     const uint32_t tx = tx0 + j % nx, ty = ty0 + j / nx;
-    if (!wide) {
-      const int X0 = max((int)(tx << sh), (int)t.bx0);
-      const int X1 = min((int)(tx << sh) + ts - 1, (int)t.bx1);
-      const int Y0 = max((int)(ty << sh), (int)t.by0);
-      const int Y1 = min((int)(ty << sh) + ts - 1, (int)t.by1);
-      const int e01 = t.c01 + min(t.a01 * X0, t.a01 * X1) + min(t.b01 * Y0, t.b01 * Y1);
-      const int e12 = t.c12 + min(t.a12 * X0, t.a12 * X1) + min(t.b12 * Y0, t.b12 * Y1);
-      const int e20 = t.c20 + min(t.a20 * X0, t.a20 * X1) + min(t.b20 * Y0, t.b20 * Y1);
-      if (e01 >= 0 || e12 >= 0 || e20 >= 0) continue;
-    }
+    if (!wide && !reaches_tile(t, tx, ty, sh)) continue;
     const uint32_t tile = vw.tile_base + ty * (uint32_t)vw.tiles_x + tx;
     bin_store(a, tile, bin_append(a, tile, tile_box(t.bx0, t.bx1, t.by0, t.by1, tx, ty, sh)), r);
   }
@@ -920,8 +938,8 @@ __global__ void __maxnreg__(CTAS == 3 ? 80 : 104) k_setup(const FrameArgs a) {
         bin_store(a, tile[k], p, r);
       }
     }
-    // more: the multi-tile queue, one atomic per warp
-    const bool many = ntiles > (uint32_t)kBinDirectMax;
+    // more: the multi-tile queue, one atomic per warp (or the list of huge triangles)
+    const bool many = ntiles > (uint32_t)kBinDirectMax && !queue_huge(a, ntiles, r, view);
     const unsigned mm = __ballot_sync(FULL_MASK, many);
     if (mm) {
       uint32_t qb = 0;
@@ -1000,7 +1018,8 @@ __global__ void __maxnreg__(96) k_clip(const FrameArgs a) {
       face_attributes(a, it, f, i0, i1, i2, it.world, p0, p1, p2, tex);
       const int ik = lane == 0 ? i0 : (lane == 1 ? i1 : i2);
       v = lane == 0 ? p0 : (lane == 1 ? p1 : p2);
-      v.p = mat_vec(it.mvp, ld4(it.pos + 4 * (size_t)ik));
+        const float4 c = __ldg(a.vclip + it.vert_base + ik);  // k_vertex's: the same arithmetic, once per vertex
+      v.p = V4{c.x, c.y, c.z, c.w};
     }
     int count = 3;
     bool overflow = false;
@@ -1090,7 +1109,7 @@ __global__ void __maxnreg__(96) k_clip(const FrameArgs a) {
       const uint32_t r = first + (uint32_t)lane;
       if (emit && r < a.rec_cap) {
         write_record(a, r, s, s0, s1, s2, tex, (it.face_base + (uint32_t)f) * (uint32_t)kKeysPerFace + (uint32_t)lane + 1u);
-        many = bin_record_direct(a, r, s.r, it.view);
+        many = bin_record_direct(a, r, s.r, it.view) && !queue_huge(a, box_tiles(s.r, a.tile_shift), r, it.view);
         rr = r;
       } else if (emit) {
         atomicMax(&a.work->rec_need, r + 1);
@@ -1879,6 +1898,8 @@ __global__ void __launch_bounds__(256) k_overlay(const FrameArgs a) {
 __global__ void __launch_bounds__(256) k_plan(const FrameArgs a) {
   griddep_wait();
   __shared__ uint32_t s_nf, s_nb, s_ne, s_bf, s_bb, s_be, s_max;
+  __shared__ TriRaster s_tri[kHugeBatch];
+  __shared__ uint2 s_huge[kHugeBatch];
   const uint32_t tile = blockIdx.x * 256u + threadIdx.x;
   if (threadIdx.x == 0) {
     s_nf = 0;
@@ -1888,14 +1909,8 @@ __global__ void __launch_bounds__(256) k_plan(const FrameArgs a) {
   }
   __syncthreads();
   const bool valid = tile < a.total_tiles;
-  const uint32_t count = valid ? a.bin_count[tile] : 0u;
-  const uint32_t boxes = valid ? a.tile_cost[tile] : 0u;
-  const uint32_t cost = valid ? count * (uint32_t)kEntryCost + boxes / 2u : 0u;
-  const uint32_t ns = valid ? tile_slices(a, min(count, a.bin_cap), cost) : 0u;
-  if (valid) {  // the bins are complete: ready for the next frame's appends
-    a.bin_count[tile] = 0u;
-    a.tile_cost[tile] = 0u;
-  }
+  uint32_t count = valid ? a.bin_count[tile] : 0u;
+  uint32_t boxes = valid ? a.tile_cost[tile] : 0u;
   // the tile's view (last view whose first tile <= tile), packed into the
   // work item beside the slice so the raster CTAs do not search for it
   int view = 0;
@@ -1905,6 +1920,39 @@ __global__ void __launch_bounds__(256) k_plan(const FrameArgs a) {
       const int mid = (view + hi + 1) >> 1;
       if (a.views[mid].tile_base <= tile) view = mid; else hi = mid - 1;
     }
+  }
+  // The huge triangles: every tile's thread appends those that reach it, to a
+  // bin that is its own by now (a warp that walks such a triangle's tiles
+  // waits an atomic's round trip for every 32: a box that fills 3840 x 2160
+  // took k_clip 228 us and now 10; the whole frame 426 -> 234 us).
+  const uint32_t nhuge = min(*(volatile uint32_t*)&a.work->nhuge, (uint32_t)kHugeCap);
+  for (uint32_t h0 = 0; h0 < nhuge; h0 += kHugeBatch) {
+    const uint32_t m = min(nhuge - h0, (uint32_t)kHugeBatch);
+    for (uint32_t k = threadIdx.x; k < m; k += 256u) {
+      const uint2 e = a.huge[h0 + k];
+      s_huge[k] = e;
+      s_tri[k] = unpack_tri(a, e.x, a.views[e.y].W, a.views[e.y].H);
+    }
+    __syncthreads();
+    if (valid) {
+      const DevView& vw = a.views[view];
+      const uint32_t lt = tile - vw.tile_base, ty = lt / (uint32_t)vw.tiles_x, tx = lt - ty * (uint32_t)vw.tiles_x;
+      for (uint32_t k = 0; k < m; ++k) {
+        if (s_huge[k].y != (uint32_t)view) continue;
+        const TriRaster& t = s_tri[k];
+        const uint32_t box = tile_box(t.bx0, t.bx1, t.by0, t.by1, tx, ty, a.tile_shift);
+        if (!box || (!(t.key & 0x80000000u) && !reaches_tile(t, tx, ty, a.tile_shift))) continue;
+        if (box > (uint32_t)kSmallBox) boxes += box;
+        bin_store(a, tile, count++, s_huge[k].x);
+      }
+    }
+    __syncthreads();
+  }
+  const uint32_t cost = valid ? count * (uint32_t)kEntryCost + boxes / 2u : 0u;
+  const uint32_t ns = valid ? tile_slices(a, min(count, a.bin_cap), cost) : 0u;
+  if (valid) {  // the bins are complete: ready for the next frame's appends
+    a.bin_count[tile] = 0u;
+    a.tile_cost[tile] = 0u;
   }
   const uint32_t vbits = (uint32_t)view << 5;  // slices < kRasterMaxSlices = 32
   // heavy items (split tiles, or whole tiles worth half a slice) go to the
@@ -2034,7 +2082,7 @@ __global__ void __launch_bounds__(RasterShape<TS>::kThreads, RasterShape<TS>::kM
     r->ovl_need = w->ovl_need;
     w->novl = 0; w->ovl_need = 0;
     w->tpf = 0; w->nrec = 0; w->nbig = 0; w->bin_need = 0; w->rec_need = 0; w->big_need = 0; w->error = 0;
-    w->nclip = 0; w->clip_need = 0; w->max_bin = 0; w->nkept = 0;
+    w->nclip = 0; w->clip_need = 0; w->max_bin = 0; w->nkept = 0; w->nhuge = 0;
     w->plan_front = 0; w->plan_back = 0; w->raster_next = 0; w->raster_exit = 0;
     w->nempty = 0; w->clear_next = 0;
   }

@@ -63,7 +63,7 @@ constexpr size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // Byte offsets of the sub-buffers inside g_scratch.
 struct Layout {
-  size_t items, texs, views, view_tpf, view_tpf_out, plan, empty, rast, shade, suv, wide, tcol, keys, bins, bin_count, tile_cost, big, clip, kept,
+  size_t items, texs, views, view_tpf, view_tpf_out, plan, empty, rast, shade, suv, wide, tcol, keys, bins, bin_count, tile_cost, big, huge, clip, kept,
       vlight, vclip, vscr, gkey, tile_done, tile_info, work, result, check, end;
 };
 
@@ -87,6 +87,7 @@ constexpr Layout make_layout() {
   l.bin_count = o; o += up256(sizeof(uint32_t) * kTiles);
   l.tile_cost = o; o += up256(sizeof(uint32_t) * kTiles);
   l.big = o; o += up256(sizeof(uint2) * kQueueCap);
+  l.huge = o; o += up256(sizeof(uint2) * kHugeCap);
   l.clip = o; o += up256(sizeof(uint2) * kQueueCap);
   l.kept = o; o += up256(sizeof(uint2) * kMaxFaces);
   l.vlight = o; o += up256(sizeof(float) * kMaxNormals);
@@ -305,6 +306,7 @@ extern "C" int32_t gr_draw_noalloc(int32_t device, const gr_noalloc_object* obje
   a.bin_count = (uint32_t*)(base + kLayout.bin_count);
   a.tile_cost = (uint32_t*)(base + kLayout.tile_cost);
   a.big = (uint2*)(base + kLayout.big);
+  a.huge = (uint2*)(base + kLayout.huge);
   a.clip = (uint2*)(base + kLayout.clip);
   a.kept = (uint2*)(base + kLayout.kept);
   a.kept_cap = kMaxFaces;

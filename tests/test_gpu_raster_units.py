@@ -69,3 +69,41 @@ def test_units_and_general_path_by_w(far):
         assert (z > -1).any()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("tile", [32, 16])
+def test_huge_triangles(tile):
+    """Triangles over more than 256 tiles, which k_plan bins: whole and clipped
+    (the camera among them), more of them than its list holds (1024), alone and
+    in a batch with a view of few tiles."""
+    torch = pytest.importorskip("torch")
+    from gorender_gb300 import renderer as R
+
+    ctx = gr.Context(0)
+    try:
+        ctx.set_tuning(tile, 0)
+        scs = [_scene(1500, 30, seed=5, w=1101, h=603), _scene(3000, 6, seed=6, w=64, h=40),
+               _scene(1500, 2600, seed=8, w=640, h=420)]
+        for sc in scs[:2]:  # corners behind the camera too
+            sc.objects[0].mesh.pos[::4, 2] += np.float32(1.5)
+        views, entries, outs = [], [], []
+        for v, sc in enumerate(scs):
+            up = gr.UploadedScene(ctx, sc)
+            ref = oracle.draw_scene(sc, items_override=up.matrices, nthreads=4)
+            rgba, z, tpf = up.render()
+            assert ref[3] == 0 and tpf == ref[2] and (ref[1] > -1).any()
+            assert np.array_equal(rgba, ref[0]) and np.array_equal(z.view(np.uint32), ref[1].view(np.uint32))
+            c = torch.zeros((sc.height, sc.width, 4), dtype=torch.uint8, device="cuda")
+            d = torch.zeros((sc.height, sc.width), dtype=torch.float32, device="cuda")
+            outs.append((up, ref, c, d))
+            views.append((up.params, c.data_ptr(), d.data_ptr()))
+            entries += [(h, m[0], m[1], v) for h, m in zip(up.mesh_handles, up.matrices)]
+        torch.cuda.synchronize()
+        b = R.Batch(ctx, views, entries, autotune=False)
+        b.run()
+        b.sync()
+        for _, ref, c, d in outs:
+            assert np.array_equal(c.cpu().numpy(), ref[0])
+            assert np.array_equal(d.cpu().numpy().view(np.uint32), ref[1].view(np.uint32))
+    finally:
+        ctx.close()
