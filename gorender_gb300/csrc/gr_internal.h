@@ -41,6 +41,7 @@ static_assert(kRasterMaxSlices <= 32, "a raster work item packs its slice into 5
 // boxes, which splits tiles of small triangles four times as far: 121 / 105 /
 // 98, 86 / 80 / 75, 382 / 348 / 333 us.)
 constexpr int kDefaultSliceCost = 8192;       // raster cost per slice before a tile is split
+constexpr int kMinSliceCost = 2048;           // ... the least in frames of few tiles
 constexpr int kEntryCost = 8;                 // raster cost of a bin entry covering <= kSmallBox pixels
 constexpr int kSmallBox = 64;                 // larger tile-clipped boxes add half their area to the tile's cost
 // k_setup: resident CTAs an SM by the frame's face count (its k_cull lane
