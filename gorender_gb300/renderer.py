@@ -417,6 +417,11 @@ class Renderer:
         N.check(N.lib().gr_renderer_fog(self._h, fog_start, fog_end, C.cast(col, C.c_void_p)))
 
     def close(self):
+        # its presenters first: they draw through this renderer, and at the end
+        # of a program either may be finalised before the other
+        for b in list(self._ctx._batches):
+            if isinstance(b, Presenter) and b.renderer is self:
+                b.close()
         if self._h:
             N.lib().gr_renderer_destroy(self._h)
             object.__setattr__(self, "_h", C.c_void_p())

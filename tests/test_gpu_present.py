@@ -65,3 +65,18 @@ def test_presenter_frames_equal_synchronous_draws(tiny_bins):
     finally:
         pctx.close()
         ctx.close()
+
+
+def test_renderer_closed_before_its_presenter():
+    """A renderer closes its presenters first, whichever the program (or its
+    end) drops first; the presenter's own close then does nothing."""
+    ctx = gr.Context(0)
+    try:
+        r, objs, cam = _renderer(ctx)
+        p = gr.Presenter(r)
+        p.frame(objs, cam)
+        r.close()
+        assert not p._h and p not in ctx._batches and r not in ctx._batches
+        p.close()
+    finally:
+        ctx.close()
