@@ -1767,26 +1767,30 @@ struct gr_diff {
   std::vector<gr_draw_item> items;      // one item per view
   std::vector<DiffView> hviews;
   uint64_t pixels = 0;
-  int max_pixels = 0;
+  int max_w = 0, max_h = 0;
   DiffView* d_views = nullptr;
   DevView* d_frame_views = nullptr;     // the visibility pass's own tables
   DevItem* d_items = nullptr;
   uint32_t* ids = nullptr;              // per pixel: visible face
   float* z = nullptr;                   // per pixel: zRec of the visible face
   DiffRecord* rec = nullptr;
-  float* vh = nullptr;                  // views x vertices x 6 (three float-float pairs)
+  int4* faces = nullptr;                // per face: indices and corner UVs side by side
+  int apart = 0;                        // some normal index differs from its vertex index
+  float4* col4 = nullptr;               // per vertex: its colour in one word
+  float* lit = nullptr;                 // per normal: its intensity
+  float4* vh = nullptr;                 // views x vertices x 2 (three float-float pairs)
   float4* col_tab = nullptr;
   float4* row_tab = nullptr;
   uint32_t cols = 0, rows = 0;
-  int max_side = 0;
   float* nhat = nullptr;
   float* d_world = nullptr;
   float* bbox_partial = nullptr;        // kBBoxBlocks x 6
   unsigned* bbox_done = nullptr;
+  unsigned* sums_done = nullptr;        // k_diff_shade's and k_diff_scatter's finished CTAs, zero when idle
   double* d_partials = nullptr;         // per-warp sums (kDiffSlots x 4), zero when idle
   float* d_gface = nullptr;             // per-face corner gradient sums (nf x 3 x 8), zero when idle
   double* h_acc = nullptr;              // pinned: loss, light gradient x 3
-  double* h_acc_dev = nullptr;          // its device address (k_diff_sum writes the sums there)
+  double* h_acc_dev = nullptr;          // its device address (the kernels write the sums there)
   gr_diff_params last{};                // parameters of the last forward
   const float* last_target = nullptr;
   bool have_forward = false;
@@ -1800,17 +1804,25 @@ DiffArgs diff_args(const gr_diff* d, const gr_diff_params& p, const float* targe
   const MeshRec& mr = d->ctx->meshes[d->mesh];
   a.views = d->d_views;
   a.num_views = (int)d->hviews.size();
-  a.max_pixels = d->max_pixels;
+  a.max_w = d->max_w;
+  a.max_h = d->max_h;
+  // four blocks of 8 rows a CTA where that leaves each SM several CTAs: one
+  // reduction of the loss and one look at the counter for 1024 pixels
+  a.rows8 = d->pixels >= (1ull << 21) ? 8 : 1;
+  a.vert_blocks = (d->nv + 255) / 256;
+  a.norm_blocks = (d->nn + 255) / 256;
   a.nv = d->nv; a.nf = d->nf; a.nn = d->nn;
   a.pos = p.positions;
   a.vcol = p.vertex_colors;
   a.tex = p.texture;
   a.tw = d->tw; a.th = d->th;
   for (int k = 0; k < 3; ++k) a.L[k] = p.light[k];
-  a.vidx = mr.vidx;
-  a.nidx = mr.nidx;
+  a.faces = d->faces;
+  a.apart = d->apart;
   a.uv = mr.uv;
   a.nhat = d->nhat;
+  a.col4 = d->col4;
+  a.lit = d->lit;
   a.vh = d->vh;
   a.col_tab = d->col_tab;
   a.row_tab = d->row_tab;
@@ -1821,6 +1833,7 @@ DiffArgs diff_args(const gr_diff* d, const gr_diff_params& p, const float* targe
   a.g_light = d->h_acc_dev + 1;
   a.partials = d->d_partials;
   a.g_face = d->d_gface;
+  a.done = d->sums_done;
   return a;
 }
 
@@ -1828,7 +1841,8 @@ void diff_free(gr_diff* d) {
   dev_free(d->d_views); dev_free(d->d_frame_views); dev_free(d->d_items);
   dev_free(d->ids); dev_free(d->z); dev_free(d->rec); dev_free(d->nhat); dev_free(d->d_world);
   dev_free(d->vh); dev_free(d->col_tab); dev_free(d->row_tab);
-  dev_free(d->bbox_partial); dev_free(d->bbox_done);
+  dev_free(d->faces); dev_free(d->col4); dev_free(d->lit);
+  dev_free(d->bbox_partial); dev_free(d->bbox_done); dev_free(d->sums_done);
   dev_free(d->d_partials);
   dev_free(d->d_gface);
   if (d->h_acc) cudaFreeHost(d->h_acc);
@@ -1924,7 +1938,6 @@ int32_t gr_diff_create(gr_context* c, int32_t mesh, const float* world, int32_t 
     hv.row_base = d->rows;
     d->cols += (uint32_t)dv.width;
     d->rows += (uint32_t)dv.height;
-    d->max_side = std::max(d->max_side, std::max(dv.width, dv.height));
     // Q = rows 0 and 1 of S * MVP (homogeneous screen x and y) and row 3 of
     // MVP (clip W), in double: products of two floats are exact there
     for (int j = 0; j < 4; ++j) {
@@ -1943,7 +1956,8 @@ int32_t gr_diff_create(gr_context* c, int32_t mesh, const float* world, int32_t 
       hv.Qf[2 * j + 1] = (float)(hv.Q[j] - (double)hi);
     }
     pix += (uint64_t)dv.width * (uint64_t)dv.height;
-    d->max_pixels = std::max(d->max_pixels, dv.width * dv.height);
+    d->max_w = std::max(d->max_w, dv.width);
+    d->max_h = std::max(d->max_h, dv.height);
     if (pix >= (1ull << 32)) st = fail(GR_ERR_UNSUPPORTED, "more than 2^32 pixels over all views");
   }
   d->pixels = pix;
@@ -1954,13 +1968,18 @@ int32_t gr_diff_create(gr_context* c, int32_t mesh, const float* world, int32_t 
   if (!st) st = dev_alloc(&d->z, (size_t)pix);
   if (!st) st = dev_alloc(&d->rec, (size_t)pix);
   if (!st) st = dev_alloc(&d->nhat, (size_t)mr.nn * 4);
-  if (!st) st = dev_alloc(&d->vh, (size_t)num_views * (size_t)mr.nv * 6);
+  if (!st) st = dev_alloc(&d->vh, (size_t)num_views * (size_t)mr.nv * 2);
+  if (!st) st = dev_alloc(&d->faces, (size_t)mr.nf * 4);
+  if (!st) st = dev_alloc(&d->col4, (size_t)mr.nv);
+  if (!st) st = dev_alloc(&d->lit, (size_t)mr.nn);
   if (!st) st = dev_alloc(&d->col_tab, (size_t)d->cols);
   if (!st) st = dev_alloc(&d->row_tab, (size_t)d->rows);
   if (!st) st = dev_alloc(&d->d_world, (size_t)16);
   if (!st) st = dev_alloc(&d->bbox_partial, (size_t)kBBoxBlocks * 6);
   if (!st) st = dev_alloc(&d->bbox_done, (size_t)1);
-  if (!st && cudaMemsetAsync(d->bbox_done, 0, sizeof(unsigned), c->stream) != cudaSuccess)
+  if (!st) st = dev_alloc(&d->sums_done, (size_t)1);
+  if (!st && (cudaMemsetAsync(d->bbox_done, 0, sizeof(unsigned), c->stream) != cudaSuccess ||
+              cudaMemsetAsync(d->sums_done, 0, sizeof(unsigned), c->stream) != cudaSuccess))
     st = fail(GR_ERR_CUDA, "diff counters");
   if (!st) st = dev_alloc(&d->d_partials, (size_t)kDiffSlots * 4);
   if (!st && cudaMemsetAsync(d->d_partials, 0, sizeof(double) * kDiffSlots * 4, c->stream) != cudaSuccess)
@@ -1986,8 +2005,12 @@ int32_t gr_diff_create(gr_context* c, int32_t mesh, const float* world, int32_t 
   }
   if (!st) {
     int e = launch_diff_normals(d->d_world, mr.vnrm, mr.nn, d->nhat, c->stream);
+    int* apart = reinterpret_cast<int*>(d->h_acc_dev);  // page-locked memory, written by the kernel
+    *reinterpret_cast<volatile int*>(d->h_acc) = 0;
+    if (!e) e = launch_diff_faces(mr.vidx, mr.nidx, mr.uv, mr.nf, d->faces, apart, c->stream);
     if (!e) e = (int)cudaStreamSynchronize(c->stream);
     if (e) st = fail(GR_ERR_CUDA, "diff normals: %s", cudaGetErrorString((cudaError_t)e));
+    else d->apart = *reinterpret_cast<volatile int*>(d->h_acc);
   }
   // the visibility pass's raster tuning (the context's default slice cost
   // left a 64-view forward 12 % slower than the best)
@@ -2037,7 +2060,7 @@ int32_t gr_diff_forward(gr_diff* d, const gr_diff_params* p, const float* target
     // memory from the kernels themselves: no copy between or after them
     pr.a.result_host = c->h_result_dev;
     if ((st = launch(c, pr.a))) return st;
-    e = launch_diff_forward(a, d->max_side, c->stream);
+    e = launch_diff_forward(a, c->stream);
     if (e) return fail(GR_ERR_CUDA, "diff forward: %s", cudaGetErrorString((cudaError_t)e));
     CK(cudaStreamSynchronize(c->stream));
     int32_t err;

@@ -54,6 +54,7 @@ namespace gr {
 namespace {
 
 constexpr int kThreads = 256;
+static_assert(kDiffSlots == kThreads, "sum_slots takes a slot a thread");
 
 __device__ __forceinline__ float go_min(float a, float b) {
   // Go's min: NaN wins, -0 below +0
@@ -178,29 +179,6 @@ __global__ void __launch_bounds__(kThreads) k_diff_normals(const float* __restri
   reinterpret_cast<float4*>(nhat)[n] = make_float4(v.x / len, v.y / len, v.z / len, 0.0f);
 }
 
-// Per view: Q_0 - x Q_3 for every column x and Q_1 - y Q_3 for every row y
-// (d u / d p and d v / d p), evaluated in double and rounded to float.
-__global__ void __launch_bounds__(kThreads) k_diff_tables(const DiffArgs a) {
-  const DiffView& vw = a.views[blockIdx.y];
-  const int i = blockIdx.x * kThreads + threadIdx.x;
-  if (i < vw.W) {
-    float4 r;
-    r.x = (float)__fma_rn(-(double)i, vw.Q[8], vw.Q[0]);
-    r.y = (float)__fma_rn(-(double)i, vw.Q[9], vw.Q[1]);
-    r.z = (float)__fma_rn(-(double)i, vw.Q[10], vw.Q[2]);
-    r.w = 0.0f;
-    a.col_tab[vw.col_base + i] = r;
-  }
-  if (i < vw.H) {
-    float4 r;
-    r.x = (float)__fma_rn(-(double)i, vw.Q[8], vw.Q[4]);
-    r.y = (float)__fma_rn(-(double)i, vw.Q[9], vw.Q[5]);
-    r.z = (float)__fma_rn(-(double)i, vw.Q[10], vw.Q[6]);
-    r.w = 0.0f;
-    a.row_tab[vw.row_base + i] = r;
-  }
-}
-
 // Float-float arithmetic: a value is hi + lo with |lo| <= ulp(hi) / 2.
 struct FF {
   float hi, lo;
@@ -238,25 +216,99 @@ __device__ __forceinline__ FF ff_mul_f(FF a, float b) {
   return fast_two_sum(p, e);
 }
 
-// Per (view, vertex): homogeneous screen x and y and clip W as float pairs,
+// Per face, once for the mesh: its vertex and normal indices and corner UVs
+// side by side (64 bytes, the indices and the first UV in 32), so that a pixel
+// reads two words instead of twelve.  *apart: some normal index differs from
+// its vertex index.
+__global__ void __launch_bounds__(kThreads) k_diff_faces(const int* __restrict__ vidx, const int* __restrict__ nidx,
+                                                         const float* __restrict__ uv, int nf, int4* out, int* apart) {
+  const int f = blockIdx.x * kThreads + threadIdx.x;
+  if (f >= nf) return;
+  const int* v = vidx + 3 * (size_t)f;
+  const int* n = nidx + 3 * (size_t)f;
+  int t[6] = {0, 0, 0, 0, 0, 0};
+  if (uv)
+    for (int k = 0; k < 6; ++k) t[k] = __float_as_int(uv[6 * (size_t)f + k]);
+  int4* o = out + 4 * (size_t)f;
+  o[0] = make_int4(v[0], v[1], v[2], n[0]);
+  o[1] = make_int4(n[1], n[2], t[0], t[1]);
+  o[2] = make_int4(t[2], t[3], t[4], t[5]);
+  o[3] = make_int4(0, 0, 0, 0);
+  if (v[0] != n[0] || v[1] != n[1] || v[2] != n[2]) *apart = 1;
+}
+
+// 32 bytes (one sector), p 32-byte aligned.
+struct Word8 {
+  uint32_t x[8];
+};
+__device__ __forceinline__ Word8 ldg8(const void* p) {
+  const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+  return Word8{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+}
+
+// Gouraud intensity of normal i.
+__device__ __forceinline__ float lit_of(const DiffArgs& a, int i) {
+  const float4 n = ldg4(a.nhat + 4 * (size_t)i);
+  return 0.5f + 0.5f * (n.x * a.L[0] + n.y * a.L[1] + n.z * a.L[2]);
+}
+
+// What the pixels of a pass gather, in one launch.  Blocks [0, a.vert_blocks)
+// of a view: per vertex homogeneous screen x and y and clip W as float pairs,
 // Q.p formed in float-float from Q's float pairs (the products of Q's hi and
 // the float coordinates are exact with an FMA; ~48-bit significands, more
-// than the geometry needs, with no FP64 instruction).
-__global__ void __launch_bounds__(kThreads) k_diff_vertices(const DiffArgs a) {
-  const int i = blockIdx.x * kThreads + threadIdx.x;
-  if (i >= a.nv) return;
+// than the geometry needs, with no FP64 instruction), in one 32-byte sector;
+// for the first view also the vertex's colour as one word, with its intensity
+// where the mesh's normals have the vertices' indices.  Blocks up to
+// a.vert_blocks + a.norm_blocks of the first view: the Gouraud intensity of
+// every normal.  The others: Q_0 - x Q_3 for every column x and Q_1 - y Q_3 for every
+// row y (d u / d p and d v / d p), evaluated in double and rounded to float.
+__global__ void __launch_bounds__(kThreads) k_diff_prepare(const DiffArgs a) {
   const DiffView& vw = a.views[blockIdx.y];
-  const float4 p = ldg4(a.pos + 4 * (size_t)i);
-  const float c[3] = {p.x, p.y, p.z};
-  float* o = a.vh + 6 * ((size_t)blockIdx.y * (size_t)a.nv + (size_t)i);
+  if ((int)blockIdx.x < a.vert_blocks) {
+    const int i = blockIdx.x * kThreads + threadIdx.x;
+    if (i >= a.nv) return;
+    const float4 p = ldg4(a.pos + 4 * (size_t)i);
+    const float c[3] = {p.x, p.y, p.z};
+    float h[6];
 #pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    const float* q = vw.Qf + 8 * r;
-    FF d{q[6], q[7]};
+    for (int r = 0; r < 3; ++r) {
+      const float* q = vw.Qf + 8 * r;
+      FF d{q[6], q[7]};
 #pragma unroll
-    for (int j = 0; j < 3; ++j) d = ff_add(d, ff_mul_f(FF{q[2 * j], q[2 * j + 1]}, c[j]));
-    o[2 * r] = d.hi;
-    o[2 * r + 1] = d.lo;
+      for (int j = 0; j < 3; ++j) d = ff_add(d, ff_mul_f(FF{q[2 * j], q[2 * j + 1]}, c[j]));
+      h[2 * r] = d.hi;
+      h[2 * r + 1] = d.lo;
+    }
+    float4* o = a.vh + 2 * ((size_t)blockIdx.y * (size_t)a.nv + (size_t)i);
+    o[0] = make_float4(h[0], h[1], h[2], h[3]);
+    o[1] = make_float4(h[4], h[5], 0.0f, 0.0f);
+    if (blockIdx.y == 0) {
+      const float* cp = a.vcol + 3 * (size_t)i;
+      a.col4[i] = make_float4(__ldg(cp), __ldg(cp + 1), __ldg(cp + 2), !a.apart && i < a.nn ? lit_of(a, i) : 0.0f);
+    }
+    return;
+  }
+  int i = ((int)blockIdx.x - a.vert_blocks) * kThreads + threadIdx.x;
+  if ((int)blockIdx.x < a.vert_blocks + a.norm_blocks) {
+    if (blockIdx.y == 0 && i < a.nn) a.lit[i] = lit_of(a, i);
+    return;
+  }
+  i -= a.norm_blocks * kThreads;
+  if (i < vw.W) {
+    float4 r;
+    r.x = (float)__fma_rn(-(double)i, vw.Q[8], vw.Q[0]);
+    r.y = (float)__fma_rn(-(double)i, vw.Q[9], vw.Q[1]);
+    r.z = (float)__fma_rn(-(double)i, vw.Q[10], vw.Q[2]);
+    r.w = 0.0f;
+    a.col_tab[vw.col_base + i] = r;
+  }
+  if (i < vw.H) {
+    float4 r;
+    r.x = (float)__fma_rn(-(double)i, vw.Q[8], vw.Q[4]);
+    r.y = (float)__fma_rn(-(double)i, vw.Q[9], vw.Q[5]);
+    r.z = (float)__fma_rn(-(double)i, vw.Q[10], vw.Q[6]);
+    r.w = 0.0f;
+    a.row_tab[vw.row_base + i] = r;
   }
 }
 
@@ -271,16 +323,18 @@ struct FaceGeom {
   bool ok;
 };
 
-__device__ __forceinline__ void face_geom(const DiffArgs& a, int view, int f, int px, int py, FaceGeom& g) {
-  const int* vi = a.vidx + 3 * (size_t)f;
+__device__ __forceinline__ void face_geom(const DiffArgs& a, int view, const Word8& face, int px, int py,
+                                          FaceGeom& g) {
   const float X = (float)px, Y = (float)py;  // exact (< 2^24)
   FF u[3], v[3];
   g.ok = true;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    g.vi[k] = __ldg(vi + k);
-    const float2* h = reinterpret_cast<const float2*>(a.vh + 6 * ((size_t)view * (size_t)a.nv + (size_t)g.vi[k]));
-    const float2 hx = __ldg(h), hy = __ldg(h + 1), w = __ldg(h + 2);
+    g.vi[k] = (int)face.x[k];
+    const Word8 h = ldg8(a.vh + 2 * ((size_t)view * (size_t)a.nv + (size_t)g.vi[k]));
+    const float2 hx = make_float2(__uint_as_float(h.x[0]), __uint_as_float(h.x[1]));
+    const float2 hy = make_float2(__uint_as_float(h.x[2]), __uint_as_float(h.x[3]));
+    const float2 w = make_float2(__uint_as_float(h.x[4]), __uint_as_float(h.x[5]));
     const FF W{w.x, w.y};
     g.ok = g.ok && W.hi < 0.0f;  // in front of the camera (W is negative there)
     u[k] = ff_sub(FF{hx.x, hx.y}, ff_mul_f(W, X));
@@ -322,15 +376,12 @@ __device__ __forceinline__ void shade(const DiffArgs& a, const FaceGeom& g, floa
   for (int ch = 0; ch < 3; ++ch) s.col[ch] = 0.0f;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const float* cp = a.vcol + 3 * (size_t)g.vi[k];
-    const float4 n = ldg4(a.nhat + 4 * (size_t)__ldg(ni + k));
-    s.Ii[k] = 0.5f + 0.5f * (n.x * a.L[0] + n.y * a.L[1] + n.z * a.L[2]);
+    const float4 c = __ldg(a.col4 + g.vi[k]);
+    s.Ii[k] = a.apart ? __ldg(a.lit + ni[k]) : c.w;
     s.I += s.l[k] * s.Ii[k];
+    s.c[k][0] = c.x; s.c[k][1] = c.y; s.c[k][2] = c.z;
 #pragma unroll
-    for (int ch = 0; ch < 3; ++ch) {
-      s.c[k][ch] = __ldg(cp + ch);
-      s.col[ch] += s.l[k] * s.c[k][ch];
-    }
+    for (int ch = 0; ch < 3; ++ch) s.col[ch] += s.l[k] * s.c[k][ch];
   }
   s.t = texel != kNoFace ? ldg4(a.tex + 4 * (size_t)texel) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
   s.out = make_float4(s.I * s.col[0] * s.t.x, s.I * s.col[1] * s.t.y, s.I * s.col[2] * s.t.z, s.t.w);
@@ -339,30 +390,93 @@ __device__ __forceinline__ void shade(const DiffArgs& a, const FaceGeom& g, floa
 __device__ __forceinline__ int wrap_index(float u, int n) {
   const float f = floorf(u * (float)n);
   if (!(f > -2.0e9f && f < 2.0e9f)) return 0;
-  int i = (int)f % n;
+  int i = (int)f;
+  if ((unsigned)i < (unsigned)n) return i;
+  i %= n;
   return i < 0 ? i + n : i;
+}
+
+// The pixels of a CTA: 32 wide, a.rows8 x 8 rows high, each warp an 8 x 4 block
+// of every 8 rows (blocks share more faces, and so more gathered lines, than
+// rows of 32 do).
+__device__ __forceinline__ int block_x() {
+  return (int)blockIdx.x * 32 + (int)((threadIdx.x >> 5) & 3u) * 8 + (int)(threadIdx.x & 7u);
+}
+__device__ __forceinline__ int block_y(const DiffArgs& a, int k) {
+  return ((int)blockIdx.y * a.rows8 + k) * 8 + (int)(threadIdx.x >> 7) * 4 + (int)((threadIdx.x >> 3) & 3u);
 }
 
 // The calling warp's slot of DiffArgs::partials (warps spread over the slots
 // so that their atomics rarely meet).
-__device__ __forceinline__ int diff_slot() {
-  return (int)(((blockIdx.y * gridDim.x + blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5)) & (kDiffSlots - 1));
+__device__ __forceinline__ int diff_slot(unsigned block) {
+  return (int)((block * (kThreads / 32) + (threadIdx.x >> 5)) & (kDiffSlots - 1));
 }
 
-// Forward: per pixel record, shaded pixel and the loss.  Grid (pixels/256, views).
+// The last of a grid's `blocks` CTAs to get here (an atomic counter, no
+// waiting) writes the sums of components [c0, c0 + N) of the slots to dst
+// (page-locked host memory, through its device address: no copy follows) and
+// returns the slots and the counter to zero.  Called by every thread.
+template <int N>
+__device__ __forceinline__ void sum_slots(const DiffArgs& a, unsigned blocks, int c0, double* dst) {
+  __shared__ double s_w[N][kThreads / 32];
+  __shared__ bool s_last;
+  if ((threadIdx.x & 31) == 0) __threadfence();  // the warp's slot sums before the count
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(a.done, 1u) == blocks - 1u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  double* p = a.partials + 4 * threadIdx.x + c0;  // kDiffSlots = kThreads
+  double t[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) t[j] = __ldcg(p + j);
+#pragma unroll
+  for (int j = 0; j < N; ++j) p[j] = 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) t[j] += __shfl_xor_sync(0xffffffffu, t[j], o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) s_w[j][threadIdx.x >> 5] = t[j];
+  }
+  __syncthreads();
+  if (threadIdx.x < N) {
+    double sum = 0.0;
+    for (int w = 0; w < kThreads / 32; ++w) sum += s_w[threadIdx.x][w];
+    dst[threadIdx.x] = sum;
+  }
+  if (threadIdx.x == 0) *a.done = 0u;
+}
+
+// Forward: per pixel record, shaded pixel and the loss.  Grid (columns / 32,
+// rows / (8 a.rows8), views).  Bound by the latency of its gathers (face, then
+// corners, then texel: 40 % of the issue slots, 38 % of the memory rate).  64 views
+// of 512 x 512 pixels of an 81,920-face mesh: 394 -> 238 us with the gathered data
+// packed (36 loads a covered pixel before, 13 now), blocks instead of rows of
+// pixels a warp, and the loss out of the FP64 pipe.
 __global__ void __launch_bounds__(kThreads) k_diff_shade(const DiffArgs a) {
-  const DiffView& vw = a.views[blockIdx.y];
-  const int p = blockIdx.x * kThreads + threadIdx.x;
-  float lp = 0.0f;
-  if (p < vw.W * vw.H) {
-    const size_t gp = (size_t)vw.pix_base + (size_t)p;
+  const DiffView& vw = a.views[blockIdx.z];
+  const int px = block_x();
+  // the pixels' losses, summed as hi + lo (error-free sums; the warp's sum goes
+  // to FP64), since FP64 additions, one a pixel or five for each warp's tree,
+  // held this kernel at the FP64 pipe's rate.  Losses near float32's end, and
+  // infinities and NaN, are summed apart, scaled by 2^-80.
+  float hi = 0.0f, lo = 0.0f, bhi = 0.0f, blo = 0.0f;
+  for (int k = 0; k < a.rows8; ++k) {
+    const int py = block_y(a, k);
+    if (px >= vw.W || py >= vw.H) break;
+    const size_t gp = (size_t)vw.pix_base + (size_t)py * (size_t)vw.W + (size_t)px;
     const uint32_t gf = a.ids[gp];
+    const float4 tg = reinterpret_cast<const float4*>(a.target)[gp];
     DiffRecord rec{kNoFace, kNoFace, 0.0f, 0.0f};
     float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (gf != kNoFace) {
-      const int f = (int)(gf - vw.face_base);
+      const int4* fr = a.faces + 4 * (size_t)(gf - vw.face_base);
+      const Word8 face = ldg8(fr);
       FaceGeom g;
-      face_geom(a, blockIdx.y, f, p % vw.W, p / vw.W, g);
+      face_geom(a, blockIdx.z, face, px, py, g);
       if (g.ok) {
         // the visibility pass snaps corners to whole pixels, so a pixel may lie
         // just outside the unsnapped face: its barycentrics are clipped to it
@@ -370,46 +484,86 @@ __global__ void __launch_bounds__(kThreads) k_diff_shade(const DiffArgs a) {
         uint32_t texel = kNoFace;
         if (a.tex && a.uv) {
           const float l2 = 1.0f - l0 - l1;
-          const float* uv = a.uv + 6 * (size_t)f;
-          const float u = l0 * __ldg(uv) + l1 * __ldg(uv + 2) + l2 * __ldg(uv + 4);
-          const float v = l0 * __ldg(uv + 1) + l1 * __ldg(uv + 3) + l2 * __ldg(uv + 5);
+          const int4 r2 = __ldg(fr + 2);
+          const float u = l0 * __uint_as_float(face.x[6]) + l1 * __int_as_float(r2.x) + l2 * __int_as_float(r2.z);
+          const float v = l0 * __uint_as_float(face.x[7]) + l1 * __int_as_float(r2.y) + l2 * __int_as_float(r2.w);
           texel = (uint32_t)(wrap_index(v, a.th) * a.tw + wrap_index(u, a.tw));
         }
         Shade s;
-        shade(a, g, l0, l1, texel, a.nidx + 3 * (size_t)f, s);
+        const int ni[3] = {(int)face.x[3], (int)face.x[4], (int)face.x[5]};
+        shade(a, g, l0, l1, texel, ni, s);
         out = s.out;
         rec = DiffRecord{gf, texel, l0, l1};
       }
     }
-    a.rec[gp] = rec;
+    reinterpret_cast<uint4*>(a.rec)[gp] =
+        make_uint4(rec.face, rec.texel, __float_as_uint(rec.l0), __float_as_uint(rec.l1));
     if (a.image) reinterpret_cast<float4*>(a.image)[gp] = out;
-    const float4 tg = reinterpret_cast<const float4*>(a.target)[gp];
     const float dx = out.x - tg.x, dy = out.y - tg.y, dz = out.z - tg.z, dw = out.w - tg.w;
-    lp = dx * dx + dy * dy + dz * dz + dw * dw;
+    const float lp = dx * dx + dy * dy + dz * dz + dw * dw;
+    if (lp < 1e36f) {
+      const FF t = two_sum(hi, lp);
+      hi = t.hi;
+      lo = __fadd_rn(lo, t.lo);
+    } else {
+      const FF t = two_sum(bhi, lp * 0x1p-80f);
+      bhi = t.hi;
+      blo = __fadd_rn(blo, t.lo);
+    }
   }
-  // the loss in FP64: within the warp, then one atomic into the warp's slot
-  // (k_diff_sum adds the slots up), so warps never wait for each other
-  double t = (double)lp;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if ((threadIdx.x & 31) == 0 && t != 0.0) atomicAdd(a.partials + 4 * diff_slot(), t);
+  for (int o = 16; o > 0; o >>= 1) {
+    const FF t = two_sum(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    lo = __fadd_rn(__fadd_rn(lo, __shfl_xor_sync(0xffffffffu, lo, o)), t.lo);
+    hi = t.hi;
+  }
+  double sum = (double)hi + (double)lo;
+  if (__any_sync(0xffffffffu, bhi != 0.0f)) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const FF t = two_sum(bhi, __shfl_xor_sync(0xffffffffu, bhi, o));
+      blo = __fadd_rn(__fadd_rn(blo, __shfl_xor_sync(0xffffffffu, blo, o)), t.lo);
+      bhi = t.hi;
+    }
+    sum += (isfinite(bhi) ? (double)bhi + (double)blo : (double)bhi) * 0x1p80;
+  }
+  // one atomic into the warp's slot, so that warps never wait for each other
+  const unsigned block = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  if ((threadIdx.x & 31) == 0 && sum != 0.0) atomicAdd(a.partials + 4 * diff_slot(block), sum);
+  sum_slots<1>(a, gridDim.x * gridDim.y * gridDim.z, 0, a.loss);
 }
 
-// Backward: gradients of the loss of the last forward pass.
+// Backward: gradients of the loss of the last forward pass.  Bound by the
+// reductions' way through L1 (78 % of its data pipe on the busiest SMs before
+// pixels were paired).  64 views of 512 x 512 pixels of an 81,920-face mesh: 400 ->
+// 254 us with the gathered data packed, the normals and the light's sums left
+// to k_diff_scatter (303 us), neighbouring pixels of a face paired (263; side
+// by side alone 272) and the face ids read a step ahead (254).
 __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
-  const DiffView& vw = a.views[blockIdx.y];
-  const int p = blockIdx.x * kThreads + threadIdx.x;
-  float gl[3] = {0.0f, 0.0f, 0.0f};
-  if (p < vw.W * vw.H) {
-    const size_t gp = (size_t)vw.pix_base + (size_t)p;
-    const DiffRecord rec = a.rec[gp];
+  const DiffView& vw = a.views[blockIdx.z];
+  const int px = block_x();
+  size_t gp = (size_t)vw.pix_base + (size_t)block_y(a, 0) * (size_t)vw.W + (size_t)px;
+  // the face ids first, a step ahead: most pixels of a view are background, and
+  // their records (four times the bytes) are not read
+  uint32_t next = px < vw.W && block_y(a, 0) < vw.H ? a.ids[gp] : kNoFace;
+  for (int k8 = 0; k8 < a.rows8; ++k8, gp += 8 * (size_t)vw.W) {
+    const int py = block_y(a, k8);
+    bool on = next != kNoFace;
+    next = k8 + 1 < a.rows8 && px < vw.W && py + 8 < vw.H ? a.ids[gp + 8 * (size_t)vw.W] : kNoFace;
+    if (!__any_sync(0xffffffffu, on)) continue;
+    DiffRecord rec{kNoFace, kNoFace, 0.0f, 0.0f};
+    if (on) {
+      const uint4 rw = reinterpret_cast<const uint4*>(a.rec)[gp];
+      rec = DiffRecord{rw.x, rw.y, __uint_as_float(rw.z), __uint_as_float(rw.w)};
+    }
+    const int f = (int)(rec.face - vw.face_base);
+    float gc[3][7];  // the corners' sums: colour, position, light weight
     if (rec.face != kNoFace) {
-      const int f = (int)(rec.face - vw.face_base);
-      const int px = p % vw.W, py = p / vw.W;
+      const Word8 face = ldg8(a.faces + 4 * (size_t)f);
       FaceGeom g;
-      face_geom(a, blockIdx.y, f, px, py, g);
-      const int* ni = a.nidx + 3 * (size_t)f;
+      face_geom(a, blockIdx.z, face, px, py, g);
       Shade s;
+      const int ni[3] = {(int)face.x[3], (int)face.x[4], (int)face.x[5]};
       shade(a, g, rec.l0, rec.l1, rec.texel, ni, s);
       const float4 tg = reinterpret_cast<const float4*>(a.target)[gp];
       const float go[4] = {2.0f * (s.out.x - tg.x), 2.0f * (s.out.y - tg.y), 2.0f * (s.out.z - tg.z),
@@ -423,24 +577,6 @@ __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
       float dI = 0.0f;
 #pragma unroll
       for (int ch = 0; ch < 3; ++ch) dI += go[ch] * s.col[ch] * t3[ch];
-      // colour and position gradients go to the face's corners first
-      // (k_diff_scatter adds them to the vertices): a vertex is shared by
-      // about six faces, so per-face sums meet far fewer atomics at one
-      // address (measured: the backward pass 20 % faster).  Each corner's six
-      // sums are two float4 (padded to eight floats), and the texel's four
-      // one float4: seven vector reductions a pixel instead of 22 scalar ones
-      // (the 64-view workload's backward 0.79 -> 0.47 ms; spreading a warp's
-      // lanes over different faces instead made it slower, 0.90 ms)
-      float4* gf = reinterpret_cast<float4*>(a.g_face + 24 * (size_t)f);
-      // light: dI/dL = sum_k l_k 0.5 nhat_k
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float4 n = ldg4(a.nhat + 4 * (size_t)__ldg(ni + k));
-        const float w = dI * 0.5f * s.l[k];
-        gl[0] += w * n.x;
-        gl[1] += w * n.y;
-        gl[2] += w * n.z;
-      }
       // positions through the barycentrics: G_k = d loss / d l_k
       float G[3];
 #pragma unroll
@@ -461,72 +597,106 @@ __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
       const float gv[3] = {dD[1] * g.u[2] - dD[2] * g.u[1], dD[2] * g.u[0] - dD[0] * g.u[2],
                            dD[0] * g.u[1] - dD[1] * g.u[0]};
       // u_k = (Q_0 - x Q_3) . p_k, v_k = (Q_1 - y Q_3) . p_k
-      const float4 A = a.col_tab[vw.col_base + px];
-      const float4 B = a.row_tab[vw.row_base + py];
+      const float4 A = __ldg(a.col_tab + vw.col_base + px);
+      const float4 B = __ldg(a.row_tab + vw.row_base + py);
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        atomicAdd(gf + 2 * k, make_float4(go[0] * s.I * t3[0] * s.l[k], go[1] * s.I * t3[1] * s.l[k],
-                                          go[2] * s.I * t3[2] * s.l[k], gu[k] * A.x + gv[k] * B.x));
-        atomicAdd(gf + 2 * k + 1, make_float4(gu[k] * A.y + gv[k] * B.y, gu[k] * A.z + gv[k] * B.z, 0.0f, 0.0f));
+        gc[k][0] = go[0] * s.I * t3[0] * s.l[k];
+        gc[k][1] = go[1] * s.I * t3[1] * s.l[k];
+        gc[k][2] = go[2] * s.I * t3[2] * s.l[k];
+        gc[k][3] = gu[k] * A.x + gv[k] * B.x;
+        gc[k][4] = gu[k] * A.y + gv[k] * B.y;
+        gc[k][5] = gu[k] * A.z + gv[k] * B.z;
+        gc[k][6] = dI * 0.5f * s.l[k];
       }
     }
-  }
-  // light gradient: float sums within the warp, then FP64 atomics into the
-  // warp's slot (k_diff_sum adds the slots up)
+    // Colour and position gradients go to the face's corners first
+    // (k_diff_scatter adds them to the vertices): a vertex is shared by about
+    // six faces, so per-face sums meet far fewer atomics at one address
+    // (measured: the backward pass 20 % faster).  Each corner's seven sums are
+    // two float4 (padded to eight floats), and the texel's four one float4:
+    // seven vector reductions a pixel.  The seventh is the corner's weight in
+    // the light's gradient, dI/dL = sum_k l_k 0.5 nhat_k, which k_diff_scatter
+    // multiplies with its normal: no normal is read here.  The reductions'
+    // way out of the SM bounds this kernel, so pixels of one face side by side
+    // or one above the other are added up first.
+    on = rec.face != kNoFace;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    gl[0] += __shfl_xor_sync(0xffffffffu, gl[0], o);
-    gl[1] += __shfl_xor_sync(0xffffffffu, gl[1], o);
-    gl[2] += __shfl_xor_sync(0xffffffffu, gl[2], o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    double* p = a.partials + 4 * diff_slot();
+    for (int o = 1; o <= 8; o <<= 3) {
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, on ? rec.face : kNoFace, o);
+      const bool same = on && other == rec.face;
+      if (!__any_sync(0xffffffffu, same)) continue;
+      const bool take = same && !(threadIdx.x & o);
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
-      if (gl[j] != 0.0f) atomicAdd(p + 1 + j, (double)gl[j]);
+      for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int j = 0; j < 7; ++j) {
+          const float x = __shfl_xor_sync(0xffffffffu, gc[k][j], o);
+          if (take) gc[k][j] += x;
+        }
+      }
+      if (same && (threadIdx.x & o)) on = false;
+    }
+    if (on) {
+      float4* gf = reinterpret_cast<float4*>(a.g_face + 24 * (size_t)f);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        atomicAdd(gf + 2 * k, make_float4(gc[k][0], gc[k][1], gc[k][2], gc[k][3]));
+        atomicAdd(gf + 2 * k + 1, make_float4(gc[k][4], gc[k][5], gc[k][6], 0.0f));
+      }
+    }
   }
 }
 
 // Adds every face's corner sums (k_diff_grad) to its vertices' colour and
-// position gradients and returns the sums to zero.  One thread per face.
+// position gradients and, weighted with its normals, to the light's, and
+// returns the sums to zero.  One thread per face; position gradients as one
+// vector reduction where the caller's buffer is aligned for it.
 __global__ void __launch_bounds__(kThreads) k_diff_scatter(const DiffArgs a) {
   const int f = blockIdx.x * kThreads + threadIdx.x;
-  if (f >= a.nf) return;
-  float* gf = a.g_face + 24 * (size_t)f;
+  double gl[3] = {0.0, 0.0, 0.0};
+  if (f < a.nf) {
+    float4* gf = reinterpret_cast<float4*>(a.g_face + 24 * (size_t)f);
+    const Word8 face = ldg8(a.faces + 4 * (size_t)f);
+    const bool vec = !((uintptr_t)a.g_pos & 15u);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const int v = __ldg(a.vidx + 3 * (size_t)f + k);
+    for (int k = 0; k < 3; ++k) {
+      const float4 p = gf[2 * k], q = gf[2 * k + 1];
+      const float x[6] = {p.x, p.y, p.z, p.w, q.x, q.y};
+      const int v = (int)face.x[k];
 #pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      const float x = gf[8 * k + j];
-      if (x == 0.0f) continue;
-      gf[8 * k + j] = 0.0f;
-      if (j < 3) atomicAdd(a.g_vcol + 3 * (size_t)v + j, x);
-      else atomicAdd(a.g_pos + 4 * (size_t)v + (j - 3), x);
+      for (int j = 0; j < 3; ++j)
+        if (x[j] != 0.0f) atomicAdd(a.g_vcol + 3 * (size_t)v + j, x[j]);
+      if (x[3] != 0.0f || x[4] != 0.0f || x[5] != 0.0f) {
+        if (vec) {
+          atomicAdd(reinterpret_cast<float4*>(a.g_pos) + v, make_float4(x[3], x[4], x[5], 0.0f));
+        } else {
+#pragma unroll
+          for (int j = 3; j < 6; ++j) atomicAdd(a.g_pos + 4 * (size_t)v + (j - 3), x[j]);
+        }
+      }
+      if (q.z != 0.0f) {
+        const float4 n = ldg4(a.nhat + 4 * (size_t)face.x[3 + k]);
+        gl[0] += (double)q.z * (double)n.x;
+        gl[1] += (double)q.z * (double)n.y;
+        gl[2] += (double)q.z * (double)n.z;
+      }
+      if (p.x != 0.0f || p.y != 0.0f || p.z != 0.0f || p.w != 0.0f) gf[2 * k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (q.x != 0.0f || q.y != 0.0f || q.z != 0.0f) gf[2 * k + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
   }
-}
-
-// Writes the sums of components [c0, c0 + n) of the per-warp slots to
-// dst[0 .. n) (page-locked host memory, through its device address: no copy
-// follows) and returns the slots to zero.  One block of kDiffSlots threads.
-__global__ void __launch_bounds__(kDiffSlots) k_diff_sum(const DiffArgs a, int c0, int n, double* dst) {
-  __shared__ double s_w[kDiffSlots / 32];
-  for (int j = 0; j < n; ++j) {
-    double* p = a.partials + 4 * threadIdx.x + c0 + j;
-    double t = *p;
-    *p = 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = t;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double sum = 0.0;
-      for (int w = 0; w < kDiffSlots / 32; ++w) sum += s_w[w];
-      dst[j] = sum;
-    }
-    __syncthreads();
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) gl[j] += __shfl_xor_sync(0xffffffffu, gl[j], o);
   }
+  if ((threadIdx.x & 31) == 0) {
+    double* p = a.partials + 4 * diff_slot(blockIdx.x);
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (gl[j] != 0.0) atomicAdd(p + 1 + j, gl[j]);
+  }
+  sum_slots<3>(a, gridDim.x, 1, a.g_light);
 }
 
 }  // namespace
@@ -545,21 +715,30 @@ int launch_diff_normals(const float* world, const float* vnrm, int nn, float* nh
   return (int)cudaGetLastError();
 }
 
-int launch_diff_forward(const DiffArgs& a, int max_side, void* stream) {
+int launch_diff_faces(const int* vidx, const int* nidx, const float* uv, int nf, int4* faces, int* apart,
+                      void* stream) {
+  if (nf <= 0) return 0;
+  k_diff_faces<<<(nf + kThreads - 1) / kThreads, kThreads, 0, (cudaStream_t)stream>>>(vidx, nidx, uv, nf, faces, apart);
+  return (int)cudaGetLastError();
+}
+
+// Grid of k_diff_shade and k_diff_grad.
+static dim3 pixel_grid(const DiffArgs& a) {
+  return dim3((unsigned)(a.max_w + 31) / 32u, (unsigned)(a.max_h + 8 * a.rows8 - 1) / (unsigned)(8 * a.rows8),
+              (unsigned)a.num_views);
+}
+
+int launch_diff_forward(const DiffArgs& a, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
-  k_diff_vertices<<<dim3((unsigned)((a.nv + kThreads - 1) / kThreads), (unsigned)a.num_views), kThreads, 0, s>>>(a);
-  k_diff_tables<<<dim3((unsigned)((max_side + kThreads - 1) / kThreads), (unsigned)a.num_views), kThreads, 0, s>>>(a);
-  const dim3 grid((unsigned)((a.max_pixels + kThreads - 1) / kThreads), (unsigned)a.num_views);
-  k_diff_shade<<<grid, kThreads, 0, s>>>(a);
-  k_diff_sum<<<1, kDiffSlots, 0, s>>>(a, 0, 1, a.loss);
+  const int sides = (std::max(a.max_w, a.max_h) + kThreads - 1) / kThreads;
+  k_diff_prepare<<<dim3((unsigned)(a.vert_blocks + a.norm_blocks + sides), (unsigned)a.num_views), kThreads, 0, s>>>(a);
+  k_diff_shade<<<pixel_grid(a), kThreads, 0, s>>>(a);
   return (int)cudaGetLastError();
 }
 
 int launch_diff_backward(const DiffArgs& a, void* stream) {
-  const dim3 grid((unsigned)((a.max_pixels + kThreads - 1) / kThreads), (unsigned)a.num_views);
-  k_diff_grad<<<grid, kThreads, 0, (cudaStream_t)stream>>>(a);
+  k_diff_grad<<<pixel_grid(a), kThreads, 0, (cudaStream_t)stream>>>(a);
   k_diff_scatter<<<(unsigned)((a.nf + kThreads - 1) / kThreads), kThreads, 0, (cudaStream_t)stream>>>(a);
-  k_diff_sum<<<1, kDiffSlots, 0, (cudaStream_t)stream>>>(a, 1, 3, a.g_light);
   return (int)cudaGetLastError();
 }
 

@@ -355,19 +355,23 @@ struct DiffRecord {
 struct DiffArgs {
   const DiffView* views;
   int num_views;
-  int max_pixels;                   // largest view (grid x extent)
+  int max_w, max_h;                 // the views' largest width and height
+  int rows8;                        // blocks of 8 rows a CTA of k_diff_shade / k_diff_grad takes (diff_rows8)
+  int vert_blocks, norm_blocks;     // k_diff_prepare's blocks for vertices and normals
   int nv, nf, nn;
   const float* pos;                 // nv x 4 (parameter)
   const float* vcol;                // nv x 3 (parameter)
   const float* tex;                 // th x tw x 4 RGBA (parameter; may be null)
   int tw, th;
   float L[4];                       // light direction (parameter)
-  const int* vidx;                  // nf x 3
-  const int* nidx;                  // nf x 3
-  const float* uv;                  // nf x 6 (may be null)
+  const int4* faces;                // nf x 4 words: vertex indices, normal indices, corner UVs (k_diff_faces)
+  int apart;                        // some normal index differs from its vertex index: lit is gathered apart
+  const float* uv;                  // the mesh's corner UVs (null: none)
   const float* nhat;                // nn x 4: normalised world-space vertex normals
-  float* vh;                        // views x nv x 6: homogeneous screen x, y and clip W, each a
-                                    // float-float pair (hi, lo) rounded from double
+  float4* col4;                     // nv: the vertex colours, a word each, and the intensity (unless apart)
+  float* lit;                       // nn: 0.5 + 0.5 nhat . L
+  float4* vh;                       // views x nv x 2 words: homogeneous screen x, y and clip W, each a
+                                    // float-float pair (hi, lo)
   float4* col_tab;                  // per view and column x: Q_0 - x Q_3 (xyz)
   float4* row_tab;                  // per view and row y: Q_1 - y Q_3 (xyz)
   const uint32_t* ids;              // per pixel: global face index or kNoFace (raster output)
@@ -380,11 +384,12 @@ struct DiffArgs {
   float* g_tex;                     // th x tw x 4
   double* g_light;                  // 3 (page-locked host memory, its device address)
   double* partials;                 // kDiffSlots x {loss, light x, y, z}: per-warp sums, zero when idle
-  float* g_face;                    // nf x 3 corners x {colour r, g, b, position x, y, z, 0, 0}: the
-                                    // backward's per-face sums before k_diff_scatter (zero when idle),
+  float* g_face;                    // nf x 3 corners x {colour r, g, b, position x, y, z, light weight, 0}:
+                                    // the backward's per-face sums before k_diff_scatter (zero when idle),
                                     // two float4 a corner
+  unsigned* done;                   // CTAs that have added to the partials (zero when idle)
 };
-constexpr int kDiffSlots = 1024;     // slots of DiffArgs::partials
+constexpr int kDiffSlots = 256;      // slots of DiffArgs::partials
 
 // FrameBuffer.Fog on one framebuffer (gr_kernels.cu).
 int launch_fog(uint32_t* rgba, const float* z, long long pixels, float fog_start, float fog_end, uint32_t color,
@@ -418,9 +423,11 @@ int launch_diff_bbox(const float* pos, int nv, DevItem* items, int num_items, fl
                      void* stream);
 // nhat[n] = xyz of Vec4.Normalize(world * vnrm[n]) (renderer.go:328-331), w = 0.
 int launch_diff_normals(const float* world, const float* vnrm, int nn, float* nhat, void* stream);
-// Per (view, vertex) and per (view, column / row) tables, then per pixel
-// shading; max_side = the largest view width or height.
-int launch_diff_forward(const DiffArgs& a, int max_side, void* stream);
+// The mesh's indices and corner UVs in the layout of DiffArgs::faces.
+int launch_diff_faces(const int* vidx, const int* nidx, const float* uv, int nf, int4* faces, int* apart,
+                      void* stream);
+// Per vertex, normal, column and row tables, then per pixel shading.
+int launch_diff_forward(const DiffArgs& a, void* stream);
 int launch_diff_backward(const DiffArgs& a, void* stream);
 
 // Records a message for gr_last_error() on this thread and returns code (gr_api.cpp).
