@@ -31,8 +31,12 @@ constexpr int kHugeTiles = 256;
 constexpr int kHugeCap = 1024;
 constexpr int kHugeBatch = 128;               // huge triangles k_plan stages at once
 constexpr int kStageSlots = 3;                // pinned staging slots for back-to-back async draws
-constexpr int kRasterMaxSlices = 32;          // CTAs that may share one tile's bin
-static_assert(kRasterMaxSlices <= 32, "a raster work item packs its slice into 5 bits");
+// CTAs that may share one tile's bin (more than there are SMs for the few
+// tiles along a horizon: 1.05 M faces at 282 x 167 pixels, 35,000 entries in each of
+// nine tiles, the whole frame: 138 us with 32, 133 with 64)
+constexpr int kRasterMaxSlices = 64;
+constexpr int kSliceBits = 6;                 // a raster work item packs its slice beside its view
+static_assert(kRasterMaxSlices == 1 << kSliceBits, "slice bits");
 // The raster's cost estimate, in about eighths of a staged bin entry: an entry
 // costs kEntryCost and half the pixels of its tile-clipped box.  Frames of the
 // default 32 x 32 tiles at slice costs of 4096 / 8192 / 16384: 200k-face terrain at
@@ -304,7 +308,7 @@ struct FrameArgs {
                                     // host (every CTA fences at system scope before it retires)
   unsigned long long* view_tpf;     // per view: binned triangles (zeroed by k_plan)
   unsigned long long* view_tpf_out; // per view: published by k_plan
-  uint2* plan;                      // raster work items (tile, slice | view << 5), plan_cap entries
+  uint2* plan;                      // raster work items (tile, slice | view << kSliceBits), plan_cap entries
   uint2* empty_tiles;               // (tile, view) of tiles without bin entries, cleared by k_raster
   uint32_t empty_cap;
   int clear_empty;                  // nonzero: tiles without bin entries go to that list (batches

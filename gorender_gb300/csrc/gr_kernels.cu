@@ -1967,7 +1967,7 @@ __global__ void __launch_bounds__(256) k_plan(const FrameArgs a) {
     a.bin_count[tile] = 0u;
     a.tile_cost[tile] = 0u;
   }
-  const uint32_t vbits = (uint32_t)view << 5;  // slices < kRasterMaxSlices = 32
+  const uint32_t vbits = (uint32_t)view << kSliceBits;
   // heavy items (split tiles, or whole tiles worth half a slice) go to the
   // front of the queue so that they start first; the rest to the back
   const bool heavy = ns > 1 || cost >= slice_cost / 2u;
@@ -2037,8 +2037,8 @@ __global__ void __launch_bounds__(RasterShape<TS>::kThreads, RasterShape<TS>::kM
       if (i < total) {
         const uint2 w = i < front ? a.plan[i] : a.plan[a.plan_cap - 1u - (i - front)];
         s_tile = w.x;
-        s_slice = w.y & 31u;       // slice (kRasterMaxSlices = 32)
-        s_view = (int)(w.y >> 5);  // view, found by k_plan
+        s_slice = w.y & (uint32_t)(kRasterMaxSlices - 1);
+        s_view = (int)(w.y >> kSliceBits);  // found by k_plan
       }
     }
     __syncthreads();
