@@ -701,6 +701,8 @@ int32_t prepare(gr_context* c, const ViewIn* views, int nviews, const gr_draw_it
   a.empty_tiles = c->empty_tiles;
   a.empty_cap = c->empty_cap;
   a.total_pixels = total_pixels;
+  a.view_w = views[0].p->width;
+  a.view_h = views[0].p->height;
   out.faces = faces;
   out.nitems = live;
   return GR_OK;

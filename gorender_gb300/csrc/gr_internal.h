@@ -61,7 +61,7 @@ constexpr int kClipBlocks = 2 * 152;          // k_clip grid (grid-stride over t
 constexpr int kBigBlocks = 3 * 152;           // k_bin_big / k_overlay grid (grid-stride over the queue)
 
 // Texture table entry (texture.go:19-26).
-struct DevTex {
+struct alignas(16) DevTex {  // read as 16-byte words (tex_sample)
   int kind;             // 0 solid, 1 image (modulo), 2 image fast (mask)
   int width, height;
   float widthF, heightF, scale;
@@ -327,6 +327,7 @@ struct FrameArgs {
                                     // split tile; k_resolve takes the max over a tile's slots
   uint32_t slot_cap;
   unsigned long long total_pixels;  // sum of the views' pixels
+  int view_w, view_h;               // the first view's size (k_resolve's grid: one-view frames)
 };
 
 // View flag (internal, never set by callers): the raster resolve writes the

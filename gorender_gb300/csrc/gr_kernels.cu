@@ -268,6 +268,7 @@ __device__ __forceinline__ long long max3ll(long long a, long long b, long long 
 // Top-left adjustment (rasterizer.go:120-129): keep f when dy > 0 or
 // (dy == 0 and dx > 0), else f - 1.
 __device__ __forceinline__ bool keeps_edge(long long dx, long long dy) { return dy > 0 || (dy == 0 && dx > 0); }
+__device__ __forceinline__ bool keeps_edge(int dx, int dy) { return dy > 0 || (dy == 0 && dx > 0); }
 
 // Setup of one fan triangle.  Returns false when no pixel can pass the
 // inside test (empty clamped bounding box, or, for narrow triangles, a
@@ -302,12 +303,12 @@ __device__ __forceinline__ bool setup_tri(const SV& p0, const SV& p1, const SV& 
     if (!keeps_edge(a01, b01)) c01 -= 1;
     if (!keeps_edge(a12, b12)) c12 -= 1;
     if (!keeps_edge(a20, b20)) c20 -= 1;
-    long long sum = (long long)c01 + (long long)c12 + (long long)c20;
+    const int sum = c01 + c12 + c20;  // each within +-(2^29 + 1)
     if (sum >= 0) return false;
     s.r.a01 = a01; s.r.b01 = b01; s.r.c01 = c01;
     s.r.a12 = a12; s.r.b12 = b12; s.r.c12 = c12;
     s.r.a20 = a20; s.r.b20 = b20; s.r.c20 = c20;
-    s.r.sumf = __ll2float_rn(sum);
+    s.r.sumf = __int2float_rn(sum);
     s.wide = false;
   } else {
     typedef unsigned long long u64;
@@ -357,7 +358,7 @@ __device__ __forceinline__ TriRaster unpack_tri(const FrameArgs& a, uint32_t r, 
   if (!keeps_edge(t.a01, t.b01)) t.c01 -= 1;
   if (!keeps_edge(t.a12, t.b12)) t.c12 -= 1;
   if (!keeps_edge(t.a20, t.b20)) t.c20 -= 1;
-  t.sumf = __ll2float_rn((long long)t.c01 + (long long)t.c12 + (long long)t.c20);
+  t.sumf = __int2float_rn(t.c01 + t.c12 + t.c20);  // each within +-(2^29 + 1)
   t.bx0 = (int16_t)max(min(min(x0, x1), x2), 0);
   t.bx1 = (int16_t)min(max(max(x0, x1), x2), W - 1);
   t.by0 = (int16_t)max(min(min(y0, y1), y2), 0);
@@ -1149,20 +1150,34 @@ __global__ void __launch_bounds__(256) k_bin_big(const FrameArgs a) {
 // ---------------------------------------------------------------------------
 // k_raster / k_resolve: shading helpers, the per-tile raster, the resolve
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t tex_sample(const DevTex& t, float u, float v) {
+// int(float32) for a texture coordinate: the 32-bit conversion where it gives
+// the same number (all but absurd coordinates), several instructions less.
+__device__ __forceinline__ long long tex_int(float f) {
+  return fabsf(f) < 2147483648.0f ? (long long)__float2int_rz(f) : go_int(f);
+}
+
+__device__ __forceinline__ long long tex_mod(float f, int n) {
+  return fabsf(f) < 2147483648.0f ? (long long)(__float2int_rz(f) % n) : go_int(f) % (long long)n;
+}
+
+__device__ __forceinline__ uint32_t tex_sample(const DevTex* tex, float u, float v) {
   // Texture.Sample (texture.go:69-89)
-  if (t.kind == 0) return t.color;
-  if (t.kind == 2) {
-    long long x = go_int(fm(fm(fs(1.0f, u), t.scale), t.widthF)) & (long long)(t.width - 1);
-    long long y = go_int(fm(fm(v, t.scale), t.heightF)) & (long long)(t.height - 1);
-    return __ldg(t.px + y * t.width + x);
+  const int4 t0 = __ldg(reinterpret_cast<const int4*>(tex));  // kind, width, height, widthF
+  const int4 t1 = __ldg(reinterpret_cast<const int4*>(tex) + 1);  // heightF, scale, colour
+  const int kind = t0.x, width = t0.y, height = t0.z;
+  const float widthF = __int_as_float(t0.w), heightF = __int_as_float(t1.x), scale = __int_as_float(t1.y);
+  if (kind == 0) return (uint32_t)t1.z;
+  if (kind == 2) {
+    const int x = (int)tex_int(fm(fm(fs(1.0f, u), scale), widthF)) & (width - 1);  // the mask keeps low bits only
+    const int y = (int)tex_int(fm(fm(v, scale), heightF)) & (height - 1);
+    return __ldg(tex->px + ((long long)y * width + x));
   }
-  if (t.kind == 1) {
-    long long x = go_int(fm(fm(fs(1.0f, u), t.scale), t.widthF)) % (long long)t.width;
-    long long y = go_int(fm(fm(v, t.scale), t.heightF)) % (long long)t.height;
-    long long idx = y * t.width + x;
+  if (kind == 1) {
+    const long long x = tex_mod(fm(fm(fs(1.0f, u), scale), widthF), width);
+    const long long y = tex_mod(fm(fm(v, scale), heightF), height);
+    long long idx = y * width + x;
     if (idx < 0) idx = 0;
-    return __ldg(t.px + idx);
+    return __ldg(tex->px + idx);
   }
   return 0xFFFF00FFu;  // magenta (255, 0, 255, 255)
 }
@@ -1574,9 +1589,17 @@ __device__ __forceinline__ void raster_wide(const FrameArgs& a, const DevView& v
   }
 }
 
+__device__ __forceinline__ TriShade load_shade(const FrameArgs& a, uint32_t r) {
+  const float4 s = __ldg(reinterpret_cast<const float4*>(a.shade) + r);
+  return TriShade{s.x, s.y, s.z, __float_as_int(s.w)};
+}
+
 // Final colour and depth of pixel (x, y) of view vw whose visibility key is k:
 // deferred shading of the winning triangle (rasterizer.go:149-176), or Clear
 // and DotGrid when no triangle won; then overlay marks, the crosshair and fog.
+// EARLY: everything that the shading gathers is asked for at once, beside the
+// record (k_resolve; k_raster's registers have no room for it).
+template <bool EARLY>
 __device__ __forceinline__ void resolve_pixel(const FrameArgs& a, const DevView& vw, int x, int y,
                                               unsigned long long k, uint32_t& out_c, float& out_z) {
   const bool face_ids = vw.flags & kViewFaceIds;
@@ -1601,7 +1624,17 @@ __device__ __forceinline__ void resolve_pixel(const FrameArgs& a, const DevView&
       return;
     }
     const uint32_t r = record_of_key(a, okey);
+    TriShade s{};
+    float4 q0;
+    float2 q1;
+    auto load_uv = [&]() {
+      if (s.tex < 0) return;
+      q0 = __ldg(reinterpret_cast<const float4*>(a.suv + r));
+      q1 = __ldg(reinterpret_cast<const float2*>(a.suv + r) + 2);
+    };
+    if constexpr (EARLY) s = load_shade(a, r);
     const TriRaster t = unpack_tri(a, r, vw.W, vw.H);
+    if constexpr (EARLY) load_uv();
     bool inside;
     float e12f, e20f, al, be, ga;
     edges_at(t, a.wide, r, x, y, inside, e12f, e20f);
@@ -1611,22 +1644,28 @@ __device__ __forceinline__ void resolve_pixel(const FrameArgs& a, const DevView&
     // full zRec.
     float z;
     if ((uint32_t)(k >> 32) != 0x80000000u) {
-      al = fd(e12f, t.sumf);
-      be = fd(e20f, t.sumf);
+      if (t.key & 0x80000000u) {
+        al = fd(e12f, t.sumf);
+        be = fd(e20f, t.sumf);
+      } else {  // whole numbers in [1, 2^32) by magnitude
+        const float ys = __frcp_rn(t.sumf);
+        al = div_by(e12f, t.sumf, ys);
+        be = div_by(e20f, t.sumf, ys);
+      }
       ga = fs(fs(1.0f, al), be);
       z = key_depth(k);
     } else {
       z = zrec_of(e12f, e20f, t.sumf, t.w0, t.w1, t.w2, al, be, ga);
     }
     out_z = z;
-    const TriShade s = a.shade[r];
+    if constexpr (!EARLY) s = load_shade(a, r);
     const float I = fa(fa(fm(al, s.i0), fm(be, s.i1)), fm(ga, s.i2));
     uint32_t c;
     if (s.tex >= 0) {
-      const TriUV q = a.suv[r];
-      const float u = fd(fa(fa(fm(al, q.u0w), fm(be, q.u1w)), fm(ga, q.u2w)), z);
-      const float v = fd(fa(fa(fm(al, q.v0w), fm(be, q.v1w)), fm(ga, q.v2w)), z);
-      c = color_intensity(tex_sample(a.texs[s.tex], u, v), I);
+      if constexpr (!EARLY) load_uv();
+      const float u = fd(fa(fa(fm(al, q0.x), fm(be, q0.z)), fm(ga, q1.x)), z);
+      const float v = fd(fa(fa(fm(al, q0.y), fm(be, q0.w)), fm(ga, q1.y)), z);
+      c = color_intensity(tex_sample(a.texs + s.tex, u, v), I);
     } else if (s.tex == -2 || s.tex == -3) {
       float cc[9];
       if (s.tex == -2) {
@@ -1804,7 +1843,7 @@ __device__ __forceinline__ void raster_item(const FrameArgs& a, uint32_t tile, u
       for (int j = 0; j < 4; ++j) {
         out_c[j] = 0u;
         out_z[j] = 0.0f;
-        if (x + j <= tx1) resolve_pixel(a, vw, x + j, y, keys[j], out_c[j], out_z[j]);
+        if (x + j <= tx1) resolve_pixel<false>(a, vw, x + j, y, keys[j], out_c[j], out_z[j]);
       }
       const size_t o = (size_t)y * (size_t)vw.W + (size_t)x;
       const bool with_z = !(vw.flags & kViewFaceIds);  // face-id views output no depth
@@ -2121,30 +2160,26 @@ __global__ void __launch_bounds__(RasterShape<TS>::kThreads, RasterShape<TS>::kM
 }
 
 // ---------------------------------------------------------------------------
-// k_resolve: one thread per pixel of every view; shades the winners whose
-// keys k_raster stored (the shading of resolve_pixel, at full occupancy so
-// that its chain of dependent loads overlaps across many warps).
+// k_resolve: one thread per pixel of a one-view frame, a warp 32 pixels of a
+// row; shades the winners whose keys k_raster stored (the shading of
+// resolve_pixel, at full occupancy so that its chain of dependent loads
+// overlaps across many warps).  Bound by issue (65-77 %, about 310 instructions a
+// textured pixel).  40 registers for six CTAs an SM: a box that fills 3840 x
+// 2160 96 -> 86 us (94 with the 44 registers and five CTAs that it takes by
+// itself), 1920 x 1080 20.9 -> 18.9, 1280 x 720 16.7 -> 15.7, against rows found by
+// a division, 64-bit texture coordinates and sums, and gathers one after the other.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_resolve(const FrameArgs a) {
+__global__ void __launch_bounds__(256, 6) k_resolve(const FrameArgs a) {
   griddep_wait();
-  const unsigned long long p = (unsigned long long)blockIdx.x * 256u + threadIdx.x;
-  if (p >= a.total_pixels) return;
-  int v = 0;
-  if (a.num_views > 1) {  // last view whose first pixel <= p
-    int hi = a.num_views - 1;
-    while (v < hi) {
-      const int mid = (v + hi + 1) >> 1;
-      if (a.views[mid].pix_base <= p) v = mid; else hi = mid - 1;
-    }
-  }
-  const DevView& vw = a.views[v];
-  const uint32_t o = (uint32_t)(p - vw.pix_base);
-  const int y = (int)(o / (uint32_t)vw.W), x = (int)(o - (uint32_t)y * (uint32_t)vw.W);
+  const DevView& vw = a.views[0];
+  const int x = (int)blockIdx.x * 32 + (int)(threadIdx.x & 31u), y = (int)blockIdx.y * 8 + (int)(threadIdx.x >> 5);
+  if (x >= vw.W || y >= vw.H) return;
+  const size_t o = (size_t)y * (size_t)vw.W + (size_t)x;
   // The pixel's key is loaded beside its tile's info rather than after it (a
   // split tile, keyed in slots, ignores it): one dependent load less a pixel.
-  unsigned long long k = a.pkey[p];
+  unsigned long long k = a.pkey[o];
   const int sh = a.tile_shift, ts = 1 << sh;
-  const uint4 ti = a.tile_info[vw.tile_base + (uint32_t)(y >> sh) * (uint32_t)vw.tiles_x + (uint32_t)(x >> sh)];
+  const uint4 ti = a.tile_info[(uint32_t)(y >> sh) * (uint32_t)vw.tiles_x + (uint32_t)(x >> sh)];
   if (ti.y > 1 && ti.z != kNoSlot) {  // a split tile: the max over its slices' slots
     const unsigned long long* sk = a.slot_keys + (size_t)ti.z * (size_t)(ts * ts) + (size_t)((y & (ts - 1)) * ts + (x & (ts - 1)));
     k = sk[0];
@@ -2153,7 +2188,7 @@ __global__ void __launch_bounds__(256) k_resolve(const FrameArgs a) {
   if (ti.x == 0) k = BG_KEY;  // a tile without entries: k_raster stored no keys
   uint32_t c;
   float z;
-  resolve_pixel(a, vw, x, y, k, c, z);
+  resolve_pixel<true>(a, vw, x, y, k, c, z);
   vw.out_rgba[o] = c;
   if (!(vw.flags & kViewFaceIds)) vw.out_z[o] = z;  // face-id views output no depth
 }
@@ -2191,7 +2226,7 @@ __device__ __forceinline__ void clear_quad(const FrameArgs& a, uint2 e, uint32_t
       for (int j = 0; j < 4; ++j) {
         c[j] = 0u;
         z[j] = 0.0f;
-        if (x + j < vw.W) resolve_pixel(a, vw, x + j, y, BG_KEY, c[j], z[j]);
+        if (x + j < vw.W) resolve_pixel<false>(a, vw, x + j, y, BG_KEY, c[j], z[j]);
       }
     }
     const size_t o = (size_t)y * (size_t)vw.W + (size_t)x;
@@ -2249,9 +2284,9 @@ int raster_grid(int tile_shift, int waves) {
 // Launches kern<<<grid, block, 0, s>>>(a), after a kernel on the same stream
 // with programmatic stream serialization (the kernel waits in griddep_wait).
 template <typename K>
-static void launch_after(K kern, unsigned grid, unsigned block, cudaStream_t s, const FrameArgs& a) {
+static void launch_after(K kern, dim3 grid, unsigned block, cudaStream_t s, const FrameArgs& a) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = s;
@@ -2332,7 +2367,7 @@ int launch_frame(const FrameArgs& a, int big_blocks, void* stream, int* launches
     launch_after(a.clear_empty ? k_raster<32, true> : k_raster<32, false>, a.raster_ctas, RasterShape<32>::kThreads, s, a);
   ++n;
   if (a.pkey && a.total_pixels) {
-    launch_after(k_resolve, (unsigned)((a.total_pixels + 255) / 256), 256, s, a);
+    launch_after(k_resolve, dim3((unsigned)(a.view_w + 31) / 32u, (unsigned)(a.view_h + 7) / 8u), 256, s, a);
     ++n;
   }
   if (events) cudaEventRecord((cudaEvent_t)events[3], s);
