@@ -268,8 +268,10 @@ int32_t ensure_tables(gr_context* c, int nviews, int nitems) {
   return GR_OK;
 }
 
-// Sizes the per-frame buffers for `faces` submitted faces and `tiles` tiles.
-int32_t ensure_frame_buffers(gr_context* c, uint64_t faces, uint32_t tiles) {
+// Sizes the per-frame buffers for `faces` submitted faces and `tiles` tiles;
+// `unclipped`: some view does not clip, so that any face may lie beyond the
+// narrow bound and go to k_clip.
+int32_t ensure_frame_buffers(gr_context* c, uint64_t faces, uint32_t tiles, bool unclipped) {
   bool synced = false;
   auto sync = [&]() -> int32_t {
     if (!synced) {
@@ -323,7 +325,7 @@ int32_t ensure_frame_buffers(gr_context* c, uint64_t faces, uint32_t tiles) {
     c->tiles_cap = nt;
     c->bin_cap = nc;
   }
-  uint64_t want_clip = std::max<uint64_t>(c->want_clip_cap, faces / 16 + 1024);
+  uint64_t want_clip = std::max<uint64_t>(c->want_clip_cap, (unclipped ? faces : faces / 16) + 1024);
   if (want_clip > c->clip_cap) {
     if ((st = sync())) return st;
     dev_free(c->clip);
@@ -440,7 +442,7 @@ int32_t prepare(gr_context* c, const ViewIn* views, int nviews, const gr_draw_it
   if (nviews <= 0 || !views) return fail(GR_ERR_INVALID_ARGUMENT, "no views");
   if (n < 0 || (n > 0 && !items)) return fail(GR_ERR_INVALID_ARGUMENT, "bad item list");
   const int ts = 1 << c->tile_shift;
-  uint32_t total_tiles = 0, flags_any = 0;
+  uint32_t total_tiles = 0, flags_any = 0, flags_all = ~0u;
   for (int v = 0; v < nviews; ++v) {
     const gr_frame_params* p = views[v].p;
     if (!p) return fail(GR_ERR_INVALID_ARGUMENT, "view %d: params is NULL", v);
@@ -455,6 +457,7 @@ int32_t prepare(gr_context* c, const ViewIn* views, int nviews, const gr_draw_it
     if (total_tiles + t >= (1ull << 31)) return fail(GR_ERR_UNSUPPORTED, "too many raster tiles");
     total_tiles += (uint32_t)t;
     flags_any |= p->flags;
+    flags_all &= p->flags;
   }
   int32_t st = ensure_tables(c, nviews, std::max(n, 1));
   if (st) return st;
@@ -575,7 +578,7 @@ int32_t prepare(gr_context* c, const ViewIn* views, int nviews, const gr_draw_it
     }
   }
   if (faces >= (1ull << 28)) return fail(GR_ERR_UNSUPPORTED, "more than 2^28 faces in one frame");
-  if ((st = ensure_frame_buffers(c, faces, total_tiles))) return st;
+  if ((st = ensure_frame_buffers(c, faces, total_tiles, !(flags_all & GR_FRUSTUM_CLIPPING)))) return st;
   if (flags_any & (GR_SHOW_EDGES | GR_SHOW_VERTICES)) {
     const uint64_t want_ovl = std::max<uint64_t>(c->want_ovl_cap, std::min<uint64_t>(faces + 1024, 1u << 30));
     if (want_ovl > c->ovl_cap) {

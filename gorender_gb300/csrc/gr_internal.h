@@ -15,6 +15,7 @@ constexpr int kMaxDim = 16384;                // narrow edge-function bound
 constexpr int kNarrowLimit = 16384;           // |screen coordinate| < 2^14 => int32 edge math
 constexpr int kMaxFan = 7;                    // a triangle clipped by 6 planes fans into <= 7
 constexpr int kKeysPerFace = 8;               // order key = face * 8 + fan + 1
+constexpr uint32_t kWholeFace = 0x80000000u;  // clip queue: a face beyond the narrow bound, set up without clipping
 constexpr uint32_t kClipFace = 0x80000000u;   // rec_of_face: a clipped face, the low bits its first fan record
 constexpr int kProjectThreads = 256;
 // k_cull (and k_vertex / k_light): faces (vertices, normals) a thread, 1, 2
@@ -49,12 +50,12 @@ constexpr int kMinSliceCost = 2048;           // ... the least in frames of few 
 constexpr int kEntryCost = 8;                 // raster cost of a bin entry covering <= kSmallBox pixels
 constexpr int kSmallBox = 64;                 // larger tile-clipped boxes add half their area to the tile's cost
 // k_setup: resident CTAs an SM by the frame's face count (its k_cull lane
-// count): 2 (at most 104 registers a thread, no spills, room for a k_clip CTA
-// beside them) below 1 M faces; 3 (at most 80 registers, 64 bytes spilled)
-// from 1 M faces on, where more warps hide more of the gathers (same-box A/B:
-// the 256-view batch 40 us faster, the 5 M-face frame 3 us; the 200k-face
-// frame 1.5 us slower with 3)
-__host__ __device__ constexpr int setup_ctas_per_sm(int project_g) { return project_g >= 2 ? 3 : 2; }
+// count): 2 (at most 104 registers a thread, room for a k_clip CTA beside
+// them) below 1 M faces; 4 (at most 64 registers) from 1 M faces on, where more
+// warps hide more of the gathers (256-view batch 1101 us with 3 of 80 registers,
+// 1075 with 4; 5.0 M-face frame 275 and 270; a 200k-face frame 93.7 with 2, 97.1
+// with 3)
+__host__ __device__ constexpr int setup_ctas_per_sm(int project_g) { return project_g >= 2 ? 4 : 2; }
 // k_setup grid (grid-stride over the kept faces)
 __host__ __device__ constexpr int setup_blocks_max(int project_g) { return setup_ctas_per_sm(project_g) * 152; }
 constexpr int kClipBlocks = 2 * 152;          // k_clip grid (grid-stride over the queue)
@@ -217,11 +218,9 @@ struct TriColor {
   float c[9];
 };
 
-// One binned triangle's overlay marks (ShowEdges / ShowVertices,
-// renderer.go:191-216): its int() corners, its float corners (the centroid
-// mark uses them) and its draw-order key.
+// One binned fan triangle's overlay marks (ShowEdges / ShowVertices,
+// renderer.go:191-216): its screen corners and its draw-order key.
 struct Overlay {
-  long long X[3], Y[3];
   float sx[3], sy[3];
   uint32_t key;                     // face * 8 + fan + 1
   uint32_t view;
@@ -291,6 +290,7 @@ struct FrameArgs {
   uint2* kept;                      // (item, face) of the faces k_cull kept whole; k_setup writes
                                     // the record of entry k as record k
   uint32_t kept_cap;                // >= the frame's faces: never overflows
+  int keep_uncovered;               // nonzero: faces that cover no pixel are kept and binned too (gr_draw_noalloc)
   int setup_blocks;                 // k_setup grid
   float* vlight;                    // per-normal Gouraud intensities (k_light)
   int light_blocks;                 // k_light grid (0: no Gouraud item)

@@ -5,17 +5,18 @@
 //   k_light    Gouraud intensity once per vertex normal.
 //   k_vertex   clip-space position and unsnapped screen x, y once per vertex.
 //   k_cull     faces in groups of 32 x G per warp: backface and frustum
-//              tests on every face; faces kept whole are compacted into one
-//              list, straddling faces go to k_clip (the general clipper, one
-//              warp per face, beside k_setup).
-//   k_setup    full warps of kept faces: attributes, screen vertices, bin
-//              test (TPF) and edge-function setup; records are appended with
-//              one atomic per warp and binned with warp-aggregated atomics
+//              tests on every face, the bin test (TPF) and the coverage of
+//              small faces; faces kept whole are compacted into one list,
+//              straddling faces and those beyond the narrow bound go to
+//              k_clip (the general clipper, one warp per face, beside k_setup).
+//   k_setup    full warps of kept faces: attributes, screen vertices and
+//              their records, binned with warp-aggregated atomics
 //              (__match_any_sync) or, past four tiles, queued for k_bin_big.
 //   k_bin_big  one warp per multi-tile triangle: appends it to every tile its
 //              edge functions can reach.
-//   k_plan     bins the few huge triangles, a tile a thread; splits heavy tiles into slices by estimated cost and orders
-//              the work queue heaviest first.
+//   k_plan     bins the few huge triangles, a tile a thread; splits heavy
+//              tiles into slices by estimated cost and orders the work queue
+//              heaviest first.
 //   k_raster   persistent CTAs over the queue, one TS x TS tile slice each:
 //              visibility in shared memory as a 64-bit max of (ordered zRec,
 //              draw-order key); footprints go as runs of up to 8 pixels of a
@@ -240,31 +241,30 @@ __device__ __forceinline__ bool bin_test(const SV& a, const SV& b, const SV& c, 
   return maxX >= 0.0f && minX <= Wf && maxY >= 0.0f && minY <= Hf;
 }
 
-// Overlay record of a binned triangle (ShowEdges / ShowVertices).  Called by
-// every lane of a converged warp; one atomic per warp.
-__device__ __forceinline__ void emit_overlay(const FrameArgs& a, bool on, const SV& s0, const SV& s1, const SV& s2,
-                                             uint32_t key, int view) {
+// Overlay record of a binned fan triangle (ShowEdges / ShowVertices) from its
+// screen corners (k_overlay reads kept faces' corners itself).  Called by every
+// lane of a converged warp; one atomic per warp.
+__device__ __noinline__ void emit_overlay(Overlay* ovl, uint32_t ovl_cap, DevWork* work, bool on, float x0, float y0,
+                                          float x1, float y1, float x2, float y2, uint32_t key, int view) {
   const unsigned m = __ballot_sync(FULL_MASK, on);
   if (!m) return;
   const unsigned lane = threadIdx.x & 31u;
   const int ldr = __ffs(m) - 1;
   uint32_t b = 0;
-  if ((int)lane == ldr) b = atomicAdd(&a.work->novl, (uint32_t)__popc(m));
+  if ((int)lane == ldr) b = atomicAdd(&work->novl, (uint32_t)__popc(m));
   b = __shfl_sync(FULL_MASK, b, ldr);
   if (!on) return;
   const uint32_t q = b + __popc(m & ((1u << lane) - 1u));
-  if (q >= a.ovl_cap) {
-    atomicMax(&a.work->ovl_need, q + 1);
+  if (q >= ovl_cap) {
+    atomicMax(&work->ovl_need, q + 1);
     return;
   }
   Overlay o;
-  o.X[0] = s0.X; o.X[1] = s1.X; o.X[2] = s2.X;
-  o.Y[0] = s0.Y; o.Y[1] = s1.Y; o.Y[2] = s2.Y;
-  o.sx[0] = s0.sx; o.sx[1] = s1.sx; o.sx[2] = s2.sx;
-  o.sy[0] = s0.sy; o.sy[1] = s1.sy; o.sy[2] = s2.sy;
+  o.sx[0] = x0; o.sx[1] = x1; o.sx[2] = x2;
+  o.sy[0] = y0; o.sy[1] = y1; o.sy[2] = y2;
   o.key = key;
   o.view = (uint32_t)view;
-  a.ovl[q] = o;
+  ovl[q] = o;
 }
 
 __device__ __forceinline__ long long min3ll(long long a, long long b, long long c) { return min(min(a, b), c); }
@@ -274,6 +274,24 @@ __device__ __forceinline__ long long max3ll(long long a, long long b, long long 
 // (dy == 0 and dx > 0), else f - 1.
 __device__ __forceinline__ bool keeps_edge(long long dx, long long dy) { return dy > 0 || (dy == 0 && dx > 0); }
 __device__ __forceinline__ bool keeps_edge(int dx, int dy) { return dy > 0 || (dy == 0 && dx > 0); }
+
+// Coverage of the n pixels (1 to 8) of a row that starts with edge values
+// e01, e12, e20 and steps a01, a12, a20: the first pixel at bit 31.
+__device__ __forceinline__ unsigned run_coverage(int e01, int e12, int e20, int a01, int a12, int a20, int n) {
+  unsigned cov = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    cov = __funnelshift_l((unsigned)(e01 & e12 & e20), cov, 1);
+    e01 += a01; e12 += a12; e20 += a20;
+  }
+  if (n <= 4) return cov >> (4 - n) << (32 - n);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    cov = __funnelshift_l((unsigned)(e01 & e12 & e20), cov, 1);
+    e01 += a01; e12 += a12; e20 += a20;
+  }
+  return cov >> (8 - n) << (32 - n);
+}
 
 // Setup of one fan triangle.  Returns false when no pixel can pass the
 // inside test (empty clamped bounding box, or, for narrow triangles, a
@@ -480,7 +498,8 @@ __device__ __forceinline__ bool facing_camera(V4 v0, V4 v1, V4 v2) {
 
 // Per-vertex attributes of face f (intensity, UV, RGB) and its texture slot.
 __device__ __forceinline__ void face_attributes(const FrameArgs& a, const DevItem& it, int f, int i0, int i1, int i2,
-                                                const float* world, PV& p0, PV& p1, PV& p2, int& tex) {
+                                                const float* world, PV& p0, PV& p1, PV& p2, int& tex,
+                                                bool kept = false) {
   const DevView& vw = a.views[it.view];
   const uint32_t fl = vw.flags;
   float in0, in1, in2;
@@ -509,7 +528,7 @@ __device__ __forceinline__ void face_attributes(const FrameArgs& a, const DevIte
   } else {
     p0.u = p0.v = p1.u = p1.v = p2.u = p2.v = 0.0f;
   }
-  if (tex == -2) {
+  if (tex == -2 && !kept) {  // (a kept face's are read again by the resolve)
     const float* c0 = it.vcol + 3 * (size_t)i0;
     const float* c1 = it.vcol + 3 * (size_t)i1;
     const float* c2 = it.vcol + 3 * (size_t)i2;
@@ -521,10 +540,86 @@ __device__ __forceinline__ void face_attributes(const FrameArgs& a, const DevIte
   }
 }
 
-// Writes record r of a set-up triangle (raster part, int64 edges, shading).
-// The caller records where the resolve finds it (rec_of_face).
-__device__ __forceinline__ void write_record(const FrameArgs& a, uint32_t r, Setup& s, const SV& q0, const SV& q1,
-                                             const SV& q2, int tex, uint32_t okey, bool from_kept = false) {
+// The shading inputs of record r: intensities, texture slot and, for textured
+// triangles, u/W and v/W per vertex.
+__device__ __forceinline__ void write_shade(const FrameArgs& a, uint32_t r, float in0, float in1, float in2, int tex,
+                                            float u0, float v0, float w0, float u1, float v1, float w1, float u2,
+                                            float v2, float w2) {
+  reinterpret_cast<float4*>(a.shade)[r] = make_float4(in0, in1, in2, __int_as_float(tex));
+  if (tex >= 0) {  // read by the shading only through a texture (rasterizer.go:132-137)
+    float4* uv = reinterpret_cast<float4*>(a.suv + r);
+    uv[0] = make_float4(fd(u0, w0), fd(v0, w0), fd(u1, w1), fd(v1, w1));
+    uv[1] = make_float4(fd(u2, w2), fd(v2, w2), 0.0f, 0.0f);
+  }
+}
+
+// A triangle whose corners lie within the narrow bound, in 32-bit integers: its
+// corners and pixel box.
+struct Box {
+  int x0, x1, y0, y1;
+};
+struct Corners {
+  int x0, y0, x1, y1, x2, y2;
+};
+__device__ __forceinline__ Corners narrow_corners(float2 q0, float2 q1, float2 q2) {
+  return Corners{__float2int_rz(q0.x), __float2int_rz(q0.y), __float2int_rz(q1.x),
+                 __float2int_rz(q1.y), __float2int_rz(q2.x), __float2int_rz(q2.y)};
+}
+__device__ __forceinline__ Box narrow_box(const Corners& c, int W, int H) {
+  return Box{max(min(min(c.x0, c.x1), c.x2), 0), min(max(max(c.x0, c.x1), c.x2), W - 1),
+             max(min(min(c.y0, c.y1), c.y2), 0), min(max(max(c.y0, c.y1), c.y2), H - 1)};
+}
+
+// Whether a narrow triangle may cover a pixel: setup_tri's tests and, for
+// boxes of at most kSmallSide pixels a side, the coverage itself.
+constexpr int kSmallSide = 4;
+__device__ __forceinline__ bool narrow_covers(const Corners& c, const Box& box) {
+  if (box.x0 > box.x1 || box.y0 > box.y1) return false;
+  const int a01 = c.y0 - c.y1, b01 = c.x1 - c.x0, a12 = c.y1 - c.y2, b12 = c.x2 - c.x1, a20 = c.y2 - c.y0,
+            b20 = c.x0 - c.x2;
+  const int c01 = c.x0 * c.y1 - c.x1 * c.y0 - (keeps_edge(a01, b01) ? 0 : 1);
+  const int c12 = c.x1 * c.y2 - c.x2 * c.y1 - (keeps_edge(a12, b12) ? 0 : 1);
+  const int c20 = c.x2 * c.y0 - c.x0 * c.y2 - (keeps_edge(a20, b20) ? 0 : 1);
+  if (c01 + c12 + c20 > -3) return false;  // three covered edge values are at most -1 each
+  const int w = box.x1 - box.x0 + 1;
+  if (w > kSmallSide || box.y1 - box.y0 >= kSmallSide) return true;
+  int e01 = a01 * box.x0 + b01 * box.y0 + c01, e12 = a12 * box.x0 + b12 * box.y0 + c12,
+      e20 = a20 * box.x0 + b20 * box.y0 + c20;
+  int cov = 0;  // sign: some pixel has three negative edge values
+#pragma unroll 1
+  for (int y = box.y0; y <= box.y1; ++y) {
+    cov |= e01 & e12 & e20;
+    if (w > 1) cov |= (e01 + a01) & (e12 + a12) & (e20 + a20);
+    if (w > 2) cov |= (e01 + 2 * a01) & (e12 + 2 * a12) & (e20 + 2 * a20);
+    if (w > 3) cov |= (e01 + 3 * a01) & (e12 + 3 * a12) & (e20 + 3 * a20);
+    e01 += b01; e12 += b12; e20 += b20;
+  }
+  return cov < 0;
+}
+
+// Whether the adjusted edge functions of a narrow triangle add up to less than
+// zero: not those of the opposite winding.
+__device__ __forceinline__ bool narrow_faces(const Corners& c) {
+  const int a01 = c.y0 - c.y1, b01 = c.x1 - c.x0, a12 = c.y1 - c.y2, b12 = c.x2 - c.x1, a20 = c.y2 - c.y0,
+            b20 = c.x0 - c.x2;
+  return c.x0 * c.y1 - c.x1 * c.y0 + c.x1 * c.y2 - c.x2 * c.y1 + c.x2 * c.y0 - c.x0 * c.y2 -
+             ((keeps_edge(a01, b01) ? 0 : 1) + (keeps_edge(a12, b12) ? 0 : 1) + (keeps_edge(a20, b20) ? 0 : 1)) < 0;
+}
+
+// identifyTriangleTiles with the single screen tile on screen corners
+// (bin_test), and whether all corners lie within the narrow bound.
+__device__ __forceinline__ bool bin_test_screen(float2 q0, float2 q1, float2 q2, float Wf, float Hf, bool& narrow) {
+  const float minX = fminf(fminf(q0.x, q1.x), q2.x), maxX = fmaxf(fmaxf(q0.x, q1.x), q2.x);
+  const float minY = fminf(fminf(q0.y, q1.y), q2.y), maxY = fmaxf(fmaxf(q0.y, q1.y), q2.y);
+  const float lim = (float)kNarrowLimit;  // |int(x)| < 2^14 where |x| < 2^14
+  narrow = minX > -lim && maxX < lim && minY > -lim && maxY < lim;
+  if (isnan(q0.x) || isnan(q1.x) || isnan(q2.x) || isnan(q0.y) || isnan(q1.y) || isnan(q2.y)) return false;
+  return maxX >= 0.0f && minX <= Wf && maxY >= 0.0f && minY <= Hf;
+}
+
+// Writes the raster part of record r of a set-up triangle (int64 edges too).
+__device__ __forceinline__ void write_raster(const FrameArgs& a, uint32_t r, Setup& s, const SV& q0, const SV& q1,
+                                             const SV& q2, uint32_t okey) {
   s.r.key = okey | (s.wide ? 0x80000000u : 0u);
   int4* dst = reinterpret_cast<int4*>(a.rast + r);
   if (s.wide) {
@@ -541,13 +636,15 @@ __device__ __forceinline__ void write_record(const FrameArgs& a, uint32_t r, Set
                        (int)s.r.key);
   }
   reinterpret_cast<float4*>(dst)[1] = make_float4(s.r.w0, s.r.w1, s.r.w2, s.r.sumf);
-  reinterpret_cast<float4*>(a.shade)[r] = make_float4(q0.in, q1.in, q2.in, __int_as_float(tex == -2 && from_kept ? -3 : tex));
-  if (tex >= 0) {  // read by the shading only through a texture (rasterizer.go:132-137)
-    float4* uv = reinterpret_cast<float4*>(a.suv + r);
-    uv[0] = make_float4(fd(q0.u, q0.W), fd(q0.v, q0.W), fd(q1.u, q1.W), fd(q1.v, q1.W));
-    uv[1] = make_float4(fd(q2.u, q2.W), fd(q2.v, q2.W), 0.0f, 0.0f);
-  }
-  if (tex == -2 && !from_kept) {
+}
+
+// Writes record r of a set-up fan triangle.  The caller records where the
+// resolve finds it (rec_of_face).
+__device__ __forceinline__ void write_record(const FrameArgs& a, uint32_t r, Setup& s, const SV& q0, const SV& q1,
+                                             const SV& q2, int tex, uint32_t okey) {
+  write_raster(a, r, s, q0, q1, q2, okey);
+  write_shade(a, r, q0.in, q1.in, q2.in, tex, q0.u, q0.v, q0.W, q1.u, q1.v, q1.W, q2.u, q2.v, q2.W);
+  if (tex == -2) {
     TriColor* c = a.tcol + r;
     c->c[0] = q0.r; c->c[1] = q0.g; c->c[2] = q0.b;
     c->c[3] = q1.r; c->c[4] = q1.g; c->c[5] = q1.b;
@@ -716,19 +813,24 @@ __global__ void __launch_bounds__(256) k_light(const FrameArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// k_cull: G faces a thread, the backface and frustum tests of every face.
-// Faces for the general clipper are queued for k_clip; faces kept whole are
+// k_cull: G faces a thread, the backface and frustum tests of every face, the
+// bin test (TPF) of those kept whole, and the coverage of the small ones among
+// them.  Faces for the general clipper are queued for k_clip; faces kept are
 // compacted over the CTA and appended to the kept list with one atomic per
 // CTA, for k_setup.  Most faces of a closed mesh face away or miss the
-// screen, so the setup runs on full warps of kept faces instead of on the
-// few survivors of each warp, and k_clip can start as soon as this pass ends.
+// screen, and most small ones cover no pixel (3 of 4 facing ones of the 5.0 M-
+// face icosphere frame), so the setup runs on full warps of faces that draw
+// something instead of on the few survivors of each warp, and k_clip can start
+// as soon as this pass ends.  With the coverage here the 5.0 M-face frame
+// takes 267 us instead of 329 (k_raster 72 -> 44, the rest k_setup), the
+// 256-view batch 1075 instead of 1139.
 // ---------------------------------------------------------------------------
 template <int G>
-__global__ void __launch_bounds__(kProjectThreads) k_cull(const FrameArgs a) {
+__global__ void __launch_bounds__(kProjectThreads, 6) k_cull(const FrameArgs a) {
   griddep_wait();
   __shared__ int s_item;
   constexpr int kWarps = kProjectThreads / 32;
-  __shared__ uint32_t s_wn[kWarps];
+  __shared__ uint32_t s_wn[kWarps], s_wt[kWarps];
   __shared__ uint32_t s_base;
   __shared__ uint2 s_keep[kWarps][32 * G];  // (item, face) of the warp's kept faces
 
@@ -747,12 +849,13 @@ __global__ void __launch_bounds__(kProjectThreads) k_cull(const FrameArgs a) {
   const DevView& vw = a.views[it.view];
 
   const uint32_t fl = vw.flags;
+  const float Wf = (float)vw.W, Hf = (float)vw.H;
   const unsigned lane = lane_id();
   const int warp = tid >> 5;
   // The clip-space corners come from k_vertex: the same arithmetic, done
   // once per vertex.
   uint2* keep_list = s_keep[warp];
-  int nkeep = 0;
+  int nkeep = 0, ntpf = 0;
   const int fgroup = ((int)blockIdx.x - it.block_base) * (kProjectThreads * G) + warp * (32 * G);
   const int nf = it.nf;
   const int* vidx = it.vidx;
@@ -765,7 +868,7 @@ __global__ void __launch_bounds__(kProjectThreads) k_cull(const FrameArgs a) {
     n1 = __ldg(vidx + 3 * f + 1);
     n2 = __ldg(vidx + 3 * f + 2);
   }
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < G; ++k) {
     const int f = fgroup + k * 32 + (int)lane;
     const int i0 = n0, i1 = n1, i2 = n2;
@@ -797,7 +900,31 @@ __global__ void __launch_bounds__(kProjectThreads) k_cull(const FrameArgs a) {
         }
       }
     }
-    // Faces for the general clipper: one atomic per warp.
+    // The faces kept whole: the bin test (TPF), and out go those that cover no
+    // pixel.  Views with overlays keep them for their marks, and frames of fixed
+    // buffers because their bins' limit is stated in them.  Corners beyond
+    // the narrow bound (hardly ever with clipping on) leave the face to k_clip,
+    // which counts and sets it up without clipping it.
+    bool keep = draw && !general, far = false;
+    if (keep) {
+      const float4* scr = a.vscr + it.vert_base;
+      const float2 q0 = __ldg(reinterpret_cast<const float2*>(scr + i0)), q1 = __ldg(reinterpret_cast<const float2*>(scr + i1)),
+                   q2 = __ldg(reinterpret_cast<const float2*>(scr + i2));
+      bool narrow;
+      const bool binned = bin_test_screen(q0, q1, q2, Wf, Hf, narrow);
+      far = binned && !narrow;
+      general = far;
+      keep = binned && narrow;
+      ntpf += keep;
+      if (keep && !(fl & 0xC0u) && !a.keep_uncovered) {
+        keep = (fl & 0x02u) != 0;  // ShowFaces off: counted, not rasterised (renderer.go:180)
+        if (keep) {
+          const Corners c = narrow_corners(q0, q1, q2);
+          keep = narrow_covers(c, narrow_box(c, vw.W, vw.H));
+        }
+      }
+    }
+    // Faces for k_clip: one atomic per warp.
     const unsigned gm = __ballot_sync(FULL_MASK, general);
     if (gm) {
       uint32_t qb = 0;
@@ -806,26 +933,32 @@ __global__ void __launch_bounds__(kProjectThreads) k_cull(const FrameArgs a) {
       qb = __shfl_sync(FULL_MASK, qb, ldr);
       if (general) {
         const uint32_t q = qb + __popc(gm & ((1u << lane) - 1u));
-        if (q < a.clip_cap) a.clip[q] = make_uint2((uint32_t)item, (uint32_t)f);
+        if (q < a.clip_cap) a.clip[q] = make_uint2((uint32_t)item, (uint32_t)f | (far ? kWholeFace : 0u));
         else atomicMax(&a.work->clip_need, q + 1);
       }
     }
-    const bool keep = draw && !general;
     const unsigned km = __ballot_sync(FULL_MASK, keep);
     if (keep) keep_list[nkeep + __popc(km & ((1u << lane) - 1u))] = make_uint2((uint32_t)item, (uint32_t)f);
     nkeep += __popc(km);
   }
-  // The CTA's kept faces: one atomic, each warp's run at its offset.
-  if (lane == 0) s_wn[warp] = (uint32_t)nkeep;
+  // The CTA's kept faces: one atomic, each warp's run at its offset; and one
+  // for its binned ones.
+  ntpf = __reduce_add_sync(FULL_MASK, ntpf);
+  if (lane == 0) {
+    s_wn[warp] = (uint32_t)nkeep;
+    s_wt[warp] = (uint32_t)ntpf;
+  }
   __syncthreads();
   if (tid == 0) {
-    uint32_t t = 0;
+    uint32_t t = 0, tpf = 0;
     for (int w = 0; w < kWarps; ++w) {
       const uint32_t n = s_wn[w];
       s_wn[w] = t;
       t += n;
+      tpf += s_wt[w];
     }
     s_base = t ? atomicAdd(&a.work->nkept, t) : 0u;
+    if (tpf) atomicAdd(&a.view_tpf[it.view], (unsigned long long)tpf);
   }
   __syncthreads();
   const uint32_t base = s_base + s_wn[warp];
@@ -837,15 +970,17 @@ __global__ void __launch_bounds__(kProjectThreads) k_cull(const FrameArgs a) {
 
 // ---------------------------------------------------------------------------
 // k_setup: the faces k_cull kept, 32 a warp over the whole list: attributes,
-// screen vertices, the bin test (TPF), setup, the record and its bins.  A
-// warp's faces may belong to different items and views.
+// corners, the record and its bins.  A warp's faces may belong to different
+// items and views.
 // ---------------------------------------------------------------------------
-// CTAS resident CTAs an SM (setup_ctas_per_sm): 2 measured 3 us less than 4
-// CTAs with spills on a 200k-face frame.  Registers are capped at 104 with 2
-// CTAs (2 x 256 x 104 = 53,248: a 96-register k_clip CTA still fits beside
-// them, as k_clip runs beside k_setup) and at 80 with 3 (3 x 256 x 80).
+// Bound by the latency of its gathers and atomics, so by resident warps.  CTAS
+// of them an SM (setup_ctas_per_sm): 2 with up to 104 registers (2 x 256 x 104 =
+// 53,248: a 96-register k_clip CTA still fits beside them, as k_clip runs beside
+// k_setup), 4 with up to 64.  All corners lie within the narrow bound here and
+// TPF is counted before, which leaves 32-bit arithmetic and 63 registers where
+// the general set-up took 80 and spilled.
 template <int CTAS>
-__global__ void __maxnreg__(CTAS == 3 ? 80 : 104) k_setup(const FrameArgs a) {
+__global__ void __maxnreg__(CTAS == 4 ? 64 : 104) k_setup(const FrameArgs a) {
   griddep_wait();
   const uint32_t nkept = min(*(volatile uint32_t*)&a.work->nkept, a.kept_cap);
   const unsigned lane = lane_id();
@@ -865,52 +1000,41 @@ __global__ void __maxnreg__(CTAS == 3 ? 80 : 104) k_setup(const FrameArgs a) {
     const uint32_t fl = vw.flags;
     const int W = vw.W, H = vw.H;
     const uint32_t tile_base = vw.tile_base, tiles_x = (uint32_t)vw.tiles_x;
-    bool emit = false;   // this face yields one record
-    int ntpf = 0;
-    int tex = -1;
-    SV s0, s1, s2;
-    Setup s;
+    bool emit = false;       // this face yields one record
+    Box box{0, -1, 0, -1};   // its pixel box
     if (valid) {
-      PV p0, p1, p2;
       const int i0 = __ldg(it.vidx + 3 * f), i1 = __ldg(it.vidx + 3 * f + 1), i2 = __ldg(it.vidx + 3 * f + 2);
-      const uint32_t v0 = vbase + i0, v1 = vbase + i1, v2 = vbase + i2;
-      face_attributes(a, it, f, i0, i1, i2, it.world, p0, p1, p2, tex);
-      const float4 q0 = __ldg(a.vscr + v0), q1 = __ldg(a.vscr + v1), q2 = __ldg(a.vscr + v2);
-      s0 = sv_of(make_float2(q0.x, q0.y), q0.z, p0);
-      s1 = sv_of(make_float2(q1.x, q1.y), q1.z, p1);
-      s2 = sv_of(make_float2(q2.x, q2.y), q2.z, p2);
-      if (bin_test(s0, s1, s2, (float)W, (float)H)) {
-        ntpf = 1;
-        // ShowFaces off: triangles still count in TPF but are not rasterised (renderer.go:180)
-        emit = (fl & 0x02u) && setup_tri(s0, s1, s2, W, H, s);
+      const float4 q0 = __ldg(a.vscr + (vbase + i0)), q1 = __ldg(a.vscr + (vbase + i1)), q2 = __ldg(a.vscr + (vbase + i2));
+      PV p0, p1, p2;
+      int tex = -1;
+      if (!(fl & kViewFaceIds)) face_attributes(a, it, f, i0, i1, i2, it.world, p0, p1, p2, tex, true);
+      if (fl & 0x02u) {  // ShowFaces
+        const Corners c = narrow_corners(make_float2(q0.x, q0.y), make_float2(q1.x, q1.y), make_float2(q2.x, q2.y));
+        box = narrow_box(c, W, H);
+        emit = box.x0 <= box.x1 && box.y0 <= box.y1;
+        if ((fl & 0xC0u) || a.keep_uncovered) emit = emit && narrow_faces(c);  // else k_cull has looked
+        if (emit && r >= a.rec_cap) {
+          atomicMax(&a.work->rec_need, r + 1u);
+          emit = false;
+        }
+        if (emit) {
+          int4* dst = reinterpret_cast<int4*>(a.rast + r);
+          dst[0] = make_int4((int)((uint32_t)(uint16_t)c.x0 | (uint32_t)c.y0 << 16),
+                             (int)((uint32_t)(uint16_t)c.x1 | (uint32_t)c.y1 << 16),
+                             (int)((uint32_t)(uint16_t)c.x2 | (uint32_t)c.y2 << 16), (int)okey);
+          reinterpret_cast<float4*>(dst)[1] = make_float4(q0.z, q1.z, q2.z, 0.0f);
+          if (!(fl & kViewFaceIds)) {  // face ids are drawn from the keys alone
+            write_shade(a, r, p0.in, p1.in, p2.in, tex == -2 ? -3 : tex, p0.u, p0.v, q0.z, p1.u, p1.v, q1.z, p2.u, p2.v, q2.z);
+            if (okey / (uint32_t)kKeysPerFace < a.face_cap) a.rec_of_face[okey / (uint32_t)kKeysPerFace] = r;
+          }
+        }
       }
     }
 
-    // TPF: one atomic per view present in the warp (nearly always one).
-    unsigned pend = __ballot_sync(FULL_MASK, ntpf != 0);
-    while (pend) {
-      const int ldr = __ffs(pend) - 1;
-      const int v = __shfl_sync(FULL_MASK, view, ldr);
-      const unsigned mine = __ballot_sync(FULL_MASK, ntpf != 0 && view == v);
-      if ((int)lane == ldr) atomicAdd(&a.view_tpf[v], (unsigned long long)__popc(mine));
-      pend &= ~mine;
-    }
-    if (__any_sync(FULL_MASK, fl & 0xC0u))  // ShowEdges / ShowVertices: every binned triangle leaves marks
-      emit_overlay(a, ntpf != 0 && (fl & 0xC0u), s0, s1, s2, okey, view);
-
-    const bool ok = emit && r < a.rec_cap;
-    if (emit && !ok) atomicMax(&a.work->rec_need, r + 1u);
-    uint32_t tx0 = 0, tx1 = 0, ty0 = 0, ty1 = 0;
-    int pbx0 = 0, pbx1 = -1, pby0 = 0, pby1 = -1;  // the record's pixel box
-    if (ok) {
-      write_record(a, r, s, s0, s1, s2, tex, okey, true);
-      if (okey / (uint32_t)kKeysPerFace < a.face_cap) a.rec_of_face[okey / (uint32_t)kKeysPerFace] = r;
-      pbx0 = s.r.bx0; pbx1 = s.r.bx1; pby0 = s.r.by0; pby1 = s.r.by1;
-      tx0 = (uint32_t)s.r.bx0 >> a.tile_shift;
-      tx1 = (uint32_t)s.r.bx1 >> a.tile_shift;
-      ty0 = (uint32_t)s.r.by0 >> a.tile_shift;
-      ty1 = (uint32_t)s.r.by1 >> a.tile_shift;
-    }
+    const bool ok = emit;
+    const int pbx0 = box.x0, pbx1 = box.x1, pby0 = box.y0, pby1 = box.y1;
+    const uint32_t tx0 = (uint32_t)pbx0 >> a.tile_shift, tx1 = (uint32_t)pbx1 >> a.tile_shift;
+    const uint32_t ty0 = (uint32_t)pby0 >> a.tile_shift, ty1 = (uint32_t)pby1 >> a.tile_shift;
     const uint32_t ntiles = ok ? (tx1 - tx0 + 1) * (ty1 - ty0 + 1) : 0u;
     // One to four tiles: the k-th tile of every lane's box in round k, one
     // bin-count atomic per distinct tile of the round (neighbouring faces
@@ -1014,7 +1138,7 @@ __global__ void __maxnreg__(96) k_clip(const FrameArgs a) {
   for (uint32_t q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < nclip; q += warps) {
     const uint2 e = a.clip[q];
     const DevItem& it = a.items[e.x];
-    const int f = (int)e.y;
+    const int f = (int)(e.y & ~kWholeFace);
     // lanes 0..2: the face's vertices with their attributes
     PV v;
     int tex = -1;
@@ -1024,7 +1148,7 @@ __global__ void __maxnreg__(96) k_clip(const FrameArgs a) {
       face_attributes(a, it, f, i0, i1, i2, it.world, p0, p1, p2, tex);
       const int ik = lane == 0 ? i0 : (lane == 1 ? i1 : i2);
       v = lane == 0 ? p0 : (lane == 1 ? p1 : p2);
-        const float4 c = __ldg(a.vclip + it.vert_base + ik);  // k_vertex's: the same arithmetic, once per vertex
+      const float4 c = __ldg(a.vclip + it.vert_base + ik);  // k_vertex's: the same arithmetic, once per vertex
       v.p = V4{c.x, c.y, c.z, c.w};
     }
     int count = 3;
@@ -1034,7 +1158,7 @@ __global__ void __maxnreg__(96) k_clip(const FrameArgs a) {
     // advance `rot` (logical vertex i sits on lane (i + rot) % count); the
     // rotation is applied before the next pass that cuts, and at the end.
     int rot = 0;
-    for (int pi = 0; pi < 6 && count > 0; ++pi) {
+    for (int pi = e.y & kWholeFace ? 6 : 0; pi < 6 && count > 0; ++pi) {
       const bool act = lane < count;
       if (__all_sync(FULL_MASK, !act || plane_inside(pi, v.p))) {
         rot = rot + 1 == count ? 0 : rot + 1;
@@ -1133,7 +1257,7 @@ __global__ void __maxnreg__(96) k_clip(const FrameArgs a) {
     const int wt = __reduce_add_sync(FULL_MASK, ntpf);
     if (lane == 0 && wt) atomicAdd(&a.view_tpf[it.view], (unsigned long long)wt);
     if (vw.flags & 0xC0u)
-      emit_overlay(a, ntpf != 0, s0, s1, s2,
+      emit_overlay(a.ovl, a.ovl_cap, a.work, ntpf != 0, s0.sx, s0.sy, s1.sx, s1.sy, s2.sx, s2.sy,
                    (it.face_base + (uint32_t)f) * (uint32_t)kKeysPerFace + (uint32_t)lane + 1u, it.view);
   }
 }
@@ -1405,24 +1529,6 @@ __device__ __forceinline__ void depth_test(unsigned long long* p, const float4& 
     if (old == c) break;
     c = old;
   }
-}
-
-// Coverage of the n pixels (1 to 8) of a row that starts with edge values
-// e01, e12, e20 and steps a01, a12, a20: the first pixel at bit 31.
-__device__ __forceinline__ unsigned run_coverage(int e01, int e12, int e20, int a01, int a12, int a20, int n) {
-  unsigned cov = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    cov = __funnelshift_l((unsigned)(e01 & e12 & e20), cov, 1);
-    e01 += a01; e12 += a12; e20 += a20;
-  }
-  if (n <= 4) return cov >> (4 - n) << (32 - n);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    cov = __funnelshift_l((unsigned)(e01 & e12 & e20), cov, 1);
-    e01 += a01; e12 += a12; e20 += a20;
-  }
-  return cov >> (8 - n) << (32 - n);
 }
 
 // The calling warp's n <= 32 entries of a batch, one a lane, into its table.
@@ -1917,26 +2023,47 @@ __device__ __forceinline__ void ovl_rect3(const FrameArgs& a, const DevView& vw,
 
 __global__ void __launch_bounds__(256) k_overlay(const FrameArgs a) {
   griddep_wait();
-  const uint32_t n = min(*(volatile uint32_t*)&a.work->novl, a.ovl_cap);
+  const uint32_t nkept = min(*(volatile uint32_t*)&a.work->nkept, a.kept_cap);
+  const uint32_t n = nkept + min(*(volatile uint32_t*)&a.work->novl, a.ovl_cap);
   const int part = (int)(threadIdx.x >> 5);  // a warp's lanes do the same part of 32 triangles
   for (uint32_t q = blockIdx.x * 32u + (threadIdx.x & 31u); q < n; q += gridDim.x * 32u) {
-    const Overlay& o = a.ovl[q];
-    const DevView& vw = a.views[o.view];
+    // the kept faces of views with overlays (all their binned ones), then k_clip's fans
+    float2 p[3];
+    uint32_t key;
+    int view;
+    if (q < nkept) {
+      const uint2 e = a.kept[q];
+      const DevItem& it = a.items[e.x];
+      view = it.view;
+      if (!(a.views[view].flags & 0xC0u)) continue;
+      key = (it.face_base + e.y) * (uint32_t)kKeysPerFace + 1u;
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        p[k] = __ldg(reinterpret_cast<const float2*>(a.vscr + it.vert_base + __ldg(it.vidx + 3 * (size_t)e.y + k)));
+    } else {
+      const Overlay& o = a.ovl[q - nkept];
+      view = (int)o.view;
+      key = o.key;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) p[k] = make_float2(o.sx[k], o.sy[k]);
+    }
+    const DevView& vw = a.views[view];
     const uint32_t fl = vw.flags;
-    const uint32_t edge = o.key * 2u, vert = o.key * 2u + 1u;  // vertex marks come after the edges
+    const uint32_t edge = key * 2u, vert = key * 2u + 1u;  // vertex marks come after the edges
+    const int from = part < 3 ? part : part - 4, to = part == 2 ? 0 : part + 1;
+    const float2 a0 = from <= 0 ? p[0] : from == 1 ? p[1] : p[2], a1 = to == 0 ? p[0] : to == 1 ? p[1] : p[2];
     if (part < 3) {
-      const int next = part == 2 ? 0 : part + 1;
-      if (fl & 0x40u) ovl_line(a, vw, o.X[part], o.Y[part], o.X[next], o.Y[next], edge);
+      if (fl & 0x40u) ovl_line(a, vw, go_int_near(a0.x), go_int_near(a0.y), go_int_near(a1.x), go_int_near(a1.y), edge);
     } else if (part == 3) {
       if ((fl & 0x42u) == 0x42u) {
-        const float cx = fd(fa(fa(o.sx[0], o.sx[1]), o.sx[2]), 3.0f);
-        const float cy = fd(fa(fa(o.sy[0], o.sy[1]), o.sy[2]), 3.0f);
-        ovl_rect3(a, vw, (long long)((unsigned long long)go_int(cx) - 1ull),
-                  (long long)((unsigned long long)go_int(cy) - 1ull), edge);
+        const float cx = fd(fa(fa(p[0].x, p[1].x), p[2].x), 3.0f);
+        const float cy = fd(fa(fa(p[0].y, p[1].y), p[2].y), 3.0f);
+        ovl_rect3(a, vw, (long long)((unsigned long long)go_int_near(cx) - 1ull),
+                  (long long)((unsigned long long)go_int_near(cy) - 1ull), edge);
       }
     } else if (part < 7 && (fl & 0x80u)) {
-      ovl_rect3(a, vw, (long long)((unsigned long long)o.X[part - 4] - 1ull),
-                (long long)((unsigned long long)o.Y[part - 4] - 1ull), vert);
+      ovl_rect3(a, vw, (long long)((unsigned long long)go_int_near(a0.x) - 1ull),
+                (long long)((unsigned long long)go_int_near(a0.y) - 1ull), vert);
     }
   }
 }
@@ -2338,20 +2465,17 @@ int launch_frame(const FrameArgs& a, int big_blocks, void* stream, int* launches
     else if (a.project_g == 2) launch_after(k_cull<2>, a.total_blocks, kProjectThreads, s, a);
     else launch_after(k_cull<1>, a.total_blocks, kProjectThreads, s, a);
     ++n;
-    const bool clip = a.flags_any & 0x01u;
-    if (clip) {  // needs only k_cull's queue: runs beside k_setup and k_bin_big
-      fork(1);
-      k_clip<<<kClipBlocks, 128, 0, s2>>>(a);
-      ++n;
-    }
-    if (setup_ctas_per_sm(a.project_g) == 3) launch_after(k_setup<3>, a.setup_blocks, kProjectThreads, s, a);
+    fork(1);  // k_clip needs only k_cull's queue: runs beside k_setup and k_bin_big
+    k_clip<<<kClipBlocks, 128, 0, s2>>>(a);
+    ++n;
+    if (setup_ctas_per_sm(a.project_g) == 4) launch_after(k_setup<4>, a.setup_blocks, kProjectThreads, s, a);
     else launch_after(k_setup<2>, a.setup_blocks, kProjectThreads, s, a);
     ++n;
     if (events) cudaEventRecord((cudaEvent_t)events[1], s);
     if (events) k_bin_big<<<big_blocks, 256, 0, s>>>(a);  // timed stages: plain launches
     else launch_after(k_bin_big, big_blocks, 256, s, a);
     ++n;
-    if (clip) join(1);
+    join(1);
     if (a.flags_any & 0xC0u) {
       k_overlay<<<big_blocks, 256, 0, s>>>(a);
       ++n;

@@ -310,6 +310,7 @@ extern "C" int32_t gr_draw_noalloc(int32_t device, const gr_noalloc_object* obje
   a.clip = (uint2*)(base + kLayout.clip);
   a.kept = (uint2*)(base + kLayout.kept);
   a.kept_cap = kMaxFaces;
+  a.keep_uncovered = 1;  // the bins hold every binned triangle, as the limits say
   a.setup_blocks = (int)std::min<long>(setup_blocks_max(a.project_g), (faces + kProjectThreads - 1) / kProjectThreads);
   a.vlight = (float*)(base + kLayout.vlight);
   a.vclip = (float4*)(base + kLayout.vclip);

@@ -107,3 +107,44 @@ def test_huge_triangles(tile):
             assert np.array_equal(d.cpu().numpy().view(np.uint32), ref[1].view(np.uint32))
     finally:
         ctx.close()
+
+
+def test_far_faces_of_unclipped_views():
+    """Without clipping most faces may have corners beyond the narrow bound:
+    k_clip sets them up whole, and an asynchronous frame of them fits the
+    buffers that its size gets at once."""
+    torch = pytest.importorskip("torch")
+    sc = _scene(60000, 1500, seed=11, w=70, h=50)
+    sc.flags &= ~gr.FRUSTUM_CLIPPING
+    ref = oracle.draw_scene(sc, nthreads=4)
+    assert ref[3] == 0 and (ref[1] > -1).any()
+    ctx = gr.Context(0)
+    try:
+        up = gr.UploadedScene(ctx, sc)
+        c = torch.zeros((sc.height, sc.width, 4), dtype=torch.uint8, device="cuda")
+        d = torch.zeros((sc.height, sc.width), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        gr.draw_async(ctx, up.items, 1, up.params, c.data_ptr(), d.data_ptr())
+        ctx.sync()
+        assert np.array_equal(c.cpu().numpy(), ref[0])
+        assert np.array_equal(d.cpu().numpy().view(np.uint32), ref[1].view(np.uint32))
+        assert up.draw() == ref[2]
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("flags", [0, gr.SHOW_EDGES, gr.SHOW_VERTICES])
+@pytest.mark.parametrize("faces", [True, False])
+def test_small_triangles_with_marks_and_without_faces(flags, faces):
+    """Triangles that cover no pixel count in TPF and leave their marks."""
+    sc = _scene(2, 3000, seed=23)
+    sc.flags = (sc.flags | flags) & ~(0 if faces else gr.SHOW_FACES)
+    ctx = gr.Context(0)
+    try:
+        up = gr.UploadedScene(ctx, sc)
+        rgba, z, tpf = up.render()
+        ref = oracle.draw_scene(sc, items_override=up.matrices, nthreads=4)
+        assert ref[3] == 0 and tpf == ref[2] > 1000
+        assert np.array_equal(rgba, ref[0]) and np.array_equal(z.view(np.uint32), ref[1].view(np.uint32))
+    finally:
+        ctx.close()
