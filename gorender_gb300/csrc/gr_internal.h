@@ -18,10 +18,12 @@ constexpr int kKeysPerFace = 8;               // order key = face * 8 + fan + 1
 constexpr uint32_t kWholeFace = 0x80000000u;  // clip queue: a face beyond the narrow bound, set up without clipping
 constexpr uint32_t kClipFace = 0x80000000u;   // rec_of_face: a clipped face, the low bits its first fan record
 constexpr int kProjectThreads = 256;
-// k_cull (and k_vertex / k_light): faces (vertices, normals) a thread, 1, 2
-// or 4 by the frame's face count
+// k_cull (and k_vertex / k_light): faces (vertices, normals) a thread, 1, 2,
+// 4 or 8 by the frame's face count: a CTA finds its item and appends its kept
+// faces once, and at 4 M faces 8 still make more CTAs than run at a time (2.6 at
+// 5 an SM; 64-view step of 5.2 M faces 1205 us with 4, 1199 with 8)
 __host__ __device__ constexpr int project_faces_per_lane(unsigned long long faces) {
-  return faces >= 2000000ull ? 4 : faces >= 1000000ull ? 2 : 1;
+  return faces >= 4000000ull ? 8 : faces >= 2000000ull ? 4 : faces >= 1000000ull ? 2 : 1;
 }
 constexpr int kBinDirectMax = 4;              // triangles spanning <= 4 tiles bin directly
 // Triangles over more tiles than this are binned by k_plan, each tile's thread
@@ -295,7 +297,7 @@ struct FrameArgs {
   float* vlight;                    // per-normal Gouraud intensities (k_light)
   int light_blocks;                 // k_light grid (0: no Gouraud item)
   float4* vclip;                    // per item vertex: clip-space position (k_vertex)
-  float4* vscr;                     // per item vertex: screen x, y before int() and clip W (k_vertex)
+  float4* vscr;                     // per item vertex: screen x, y before int(), clip W, frustum planes it is inside of (k_vertex)
   int vert_blocks;                  // k_vertex grid
   unsigned long long* gkey;         // tiles x 1024 merged visibility keys of split tiles (zero when idle)
   uint32_t* tile_done;              // per tile: slices finished (zero when idle)

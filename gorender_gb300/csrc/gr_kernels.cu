@@ -771,6 +771,9 @@ __global__ void __launch_bounds__(256) k_vertex(const FrameArgs a) {
   if (threadIdx.x < 16) s_mvp[threadIdx.x] = it.mvp[threadIdx.x];
   if (threadIdx.x < 8) s_S[threadIdx.x] = a.views[it.view].S[threadIdx.x];
   __syncthreads();
+  const int vis = it.vis;
+  if (vis == 0) return;  // outside the frustum: nothing reads its vertices
+  const bool clips = (a.views[it.view].flags & 0x01u) && vis != 2;
   const int v0 = ((int)blockIdx.x - it.vert_block_base) * (256 * G) + (int)threadIdx.x;
 #pragma unroll
   for (int k = 0; k < G; ++k) {
@@ -779,7 +782,14 @@ __global__ void __launch_bounds__(256) k_vertex(const FrameArgs a) {
       const V4 c = mat_vec(s_mvp, ld4_stream(it.pos + 4 * (size_t)v));
       a.vclip[it.vert_base + v] = make_float4(c.x, c.y, c.z, c.w);
       const float2 sc = screen_of(c, s_S);
-      a.vscr[it.vert_base + v] = make_float4(sc.x, sc.y, c.w, 0.0f);  // W beside x, y: one gather in k_setup
+      uint32_t in = 0x3Fu;
+      if (clips) {
+#pragma unroll
+        for (int i = 0; i < 6; ++i) in &= plane_inside(i, c) ? ~0u : ~(1u << i);
+      }
+      // W beside x, y: one gather in k_setup; and the planes it is inside of
+      // (all of them where faces are not clipped), for k_cull
+      a.vscr[it.vert_base + v] = make_float4(sc.x, sc.y, c.w, __uint_as_float(in));
     }
   }
 }
@@ -824,9 +834,16 @@ __global__ void __launch_bounds__(256) k_light(const FrameArgs a) {
 // as soon as this pass ends.  With the coverage here the 5.0 M-face frame
 // takes 267 us instead of 329 (k_raster 72 -> 44, the rest k_setup), the
 // 256-view batch 1075 instead of 1139.
+//
+// Bound by the latency of the corner gathers and by issue (700 instructions for
+// 32 faces when each face tested its corners against the planes itself; those
+// tests are k_vertex's now, a vertex having six faces).  5 CTAs an SM: at 6 the
+// loop spills; 4 with the next face's corners gathered ahead was 1 % slower.
+// The plane masks and G = 8 from 4 M faces took the 64-view differentiable step
+// (5.2 M faces) from 1223 to 1199 us, the 5.0 M-face frame from 266 to 262.
 // ---------------------------------------------------------------------------
 template <int G>
-__global__ void __launch_bounds__(kProjectThreads, 6) k_cull(const FrameArgs a) {
+__global__ void __launch_bounds__(kProjectThreads, 5) k_cull(const FrameArgs a) {
   griddep_wait();
   __shared__ int s_item;
   constexpr int kWarps = kProjectThreads / 32;
@@ -844,8 +861,7 @@ __global__ void __launch_bounds__(kProjectThreads, 6) k_cull(const FrameArgs a) 
   const DevItem& it = a.items[item];
   // Frustum.BoxVisibility of the transformed bounding box (renderer.go:268-275),
   // computed once per item where the box is known (box_visibility)
-  const int vis = it.vis;
-  if (vis == 0) return;  // whole block: object outside the frustum
+  if (it.vis == 0) return;  // whole block: object outside the frustum
   const DevView& vw = a.views[it.view];
 
   const uint32_t fl = vw.flags;
@@ -884,21 +900,21 @@ __global__ void __launch_bounds__(kProjectThreads, 6) k_cull(const FrameArgs a) 
                    c2 = __ldg(a.vclip + it.vert_base + i2);
       const V4 v0{c0.x, c0.y, c0.z, c0.w}, v1{c1.x, c1.y, c1.z, c1.w}, v2{c2.x, c2.y, c2.z, c2.w};
       draw = !(fl & 0x04u) || facing_camera(v0, v1, v2);  // BackfaceCulling
+    }
+    float4 q0, q1, q2;
+    if (draw) {
+      const float4* scr = a.vscr + it.vert_base;
+      q0 = __ldg(scr + i0), q1 = __ldg(scr + i1), q2 = __ldg(scr + i2);
       // Frustum clipping (renderer.go:349-359).  At the first plane, in
       // clipping order, where not all three vertices are inside: all outside
       // means the polygon reaching that plane is still the face itself (every
       // earlier pass only rotated it), so ClipTriangle returns no triangle; a
       // mix needs the general clipper.  With no such plane the six passes
       // rotate the face back to itself and it passes through unchanged.
-      if (draw && (fl & 0x01u) && vis != 2) {
-        for (int i = 0; i < 6; ++i) {
-          const int m = (int)plane_inside(i, v0) + (int)plane_inside(i, v1) + (int)plane_inside(i, v2);
-          if (m == 3) continue;
-          if (m == 0) draw = false;
-          else general = true;
-          break;
-        }
-      }
+      const uint32_t m0 = __float_as_uint(q0.w), m1 = __float_as_uint(q1.w), m2 = __float_as_uint(q2.w);
+      const uint32_t cut = ~(m0 & m1 & m2) & 0x3Fu, first = cut & (0u - cut);
+      general = (first & (m0 | m1 | m2)) != 0;
+      draw = general || !first;
     }
     // The faces kept whole: the bin test (TPF), and out go those that cover no
     // pixel.  Views with overlays keep them for their marks, and frames of fixed
@@ -907,11 +923,9 @@ __global__ void __launch_bounds__(kProjectThreads, 6) k_cull(const FrameArgs a) 
     // which counts and sets it up without clipping it.
     bool keep = draw && !general, far = false;
     if (keep) {
-      const float4* scr = a.vscr + it.vert_base;
-      const float2 q0 = __ldg(reinterpret_cast<const float2*>(scr + i0)), q1 = __ldg(reinterpret_cast<const float2*>(scr + i1)),
-                   q2 = __ldg(reinterpret_cast<const float2*>(scr + i2));
+      const float2 p0 = make_float2(q0.x, q0.y), p1 = make_float2(q1.x, q1.y), p2 = make_float2(q2.x, q2.y);
       bool narrow;
-      const bool binned = bin_test_screen(q0, q1, q2, Wf, Hf, narrow);
+      const bool binned = bin_test_screen(p0, p1, p2, Wf, Hf, narrow);
       far = binned && !narrow;
       general = far;
       keep = binned && narrow;
@@ -919,7 +933,7 @@ __global__ void __launch_bounds__(kProjectThreads, 6) k_cull(const FrameArgs a) 
       if (keep && !(fl & 0xC0u) && !a.keep_uncovered) {
         keep = (fl & 0x02u) != 0;  // ShowFaces off: counted, not rasterised (renderer.go:180)
         if (keep) {
-          const Corners c = narrow_corners(q0, q1, q2);
+          const Corners c = narrow_corners(p0, p1, p2);
           keep = narrow_covers(c, narrow_box(c, vw.W, vw.H));
         }
       }
@@ -2451,17 +2465,20 @@ int launch_frame(const FrameArgs& a, int big_blocks, void* stream, int* launches
     const bool light = a.light_blocks > 0;
     if (light) {
       fork(0);
-      if (a.project_g == 4) k_light<4><<<a.light_blocks, 256, 0, s2>>>(a);
+      if (a.project_g == 8) k_light<8><<<a.light_blocks, 256, 0, s2>>>(a);
+      else if (a.project_g == 4) k_light<4><<<a.light_blocks, 256, 0, s2>>>(a);
       else if (a.project_g == 2) k_light<2><<<a.light_blocks, 256, 0, s2>>>(a);
       else k_light<1><<<a.light_blocks, 256, 0, s2>>>(a);
       ++n;
     }
-    if (a.project_g == 4) launch_after(k_vertex<4>, a.vert_blocks, 256, s, a);
+    if (a.project_g == 8) launch_after(k_vertex<8>, a.vert_blocks, 256, s, a);
+    else if (a.project_g == 4) launch_after(k_vertex<4>, a.vert_blocks, 256, s, a);
     else if (a.project_g == 2) launch_after(k_vertex<2>, a.vert_blocks, 256, s, a);
     else launch_after(k_vertex<1>, a.vert_blocks, 256, s, a);
     ++n;
     if (light) join(0);
-    if (a.project_g == 4) launch_after(k_cull<4>, a.total_blocks, kProjectThreads, s, a);
+    if (a.project_g == 8) launch_after(k_cull<8>, a.total_blocks, kProjectThreads, s, a);
+    else if (a.project_g == 4) launch_after(k_cull<4>, a.total_blocks, kProjectThreads, s, a);
     else if (a.project_g == 2) launch_after(k_cull<2>, a.total_blocks, kProjectThreads, s, a);
     else launch_after(k_cull<1>, a.total_blocks, kProjectThreads, s, a);
     ++n;

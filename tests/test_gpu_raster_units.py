@@ -148,3 +148,20 @@ def test_small_triangles_with_marks_and_without_faces(flags, faces):
         assert np.array_equal(rgba, ref[0]) and np.array_equal(z.view(np.uint32), ref[1].view(np.uint32))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("faces", [1000001, 2000003, 4000000, 4002055])
+def test_faces_a_thread(faces):
+    """2, 4 and 8 faces a thread in k_cull, with a last CTA that is not full."""
+    sc = _scene(2, 4001, seed=37)
+    m = sc.objects[0].mesh
+    m.vidx = np.ascontiguousarray(np.resize(m.vidx, (faces, 3)))
+    ctx = gr.Context(0)
+    try:
+        up = gr.UploadedScene(ctx, sc)
+        rgba, z, tpf = up.render()
+        ref = oracle.draw_scene(sc, items_override=up.matrices, nthreads=8)
+        assert ref[3] == 0 and tpf == ref[2] > faces // 2
+        assert np.array_equal(rgba, ref[0]) and np.array_equal(z.view(np.uint32), ref[1].view(np.uint32))
+    finally:
+        ctx.close()
