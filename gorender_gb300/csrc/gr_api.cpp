@@ -616,11 +616,11 @@ int32_t prepare(gr_context* c, const ViewIn* views, int nviews, const gr_draw_it
     c->h2d_bytes = (int64_t)bytes;
   } else if (!own_views && !own_items) {  // both tables with one k_stage, before the frame's graph
     const size_t bytes = live ? c->tables_off + sizeof(DevItem) * (size_t)live : sizeof(DevView) * (size_t)nviews;
-    CK((cudaError_t)launch_stage(c->d_tables, hslot, bytes, c->stream));
+    CK((cudaError_t)launch_stage({c->d_tables, hslot, bytes}, {}, c->stream));
     c->h2d_bytes = (int64_t)bytes;
-  } else {  // tables of their own (batches, the differentiable pass): one k_stage each
-    CK((cudaError_t)launch_stage(dviews, hviews, sizeof(DevView) * nviews, c->stream));
-    if (live) CK((cudaError_t)launch_stage(ditems, hitems, sizeof(DevItem) * live, c->stream));
+  } else {  // tables of their own (batches, the differentiable pass)
+    CK((cudaError_t)launch_stage({dviews, hviews, sizeof(DevView) * (size_t)nviews},
+                                 {ditems, hitems, sizeof(DevItem) * (size_t)live}, c->stream));
     c->h2d_bytes = (int64_t)sizeof(DevItem) * live + (int64_t)sizeof(DevView) * nviews;
   }
   if (!in_graph) {
@@ -740,7 +740,7 @@ int32_t launch(gr_context* c, const FrameArgs& a, void* const* events = nullptr,
     int n = 0;
     if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
       int err = 0;
-      if (copy_bytes) err = launch_stage(c->d_tables, copy_src, copy_bytes, c->stream);
+      if (copy_bytes) err = launch_stage({c->d_tables, copy_src, copy_bytes}, {}, c->stream);
       if (!err) err = launch_frame(a, big_blocks, c->stream, &n, nullptr, &c->aux);
       if (copy_bytes) ++n;  // k_stage
       const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
@@ -760,7 +760,7 @@ int32_t launch(gr_context* c, const FrameArgs& a, void* const* events = nullptr,
       cudaGetLastError();  // capture failed: fall back to plain launches
     }
   }
-  if (copy_bytes) CK((cudaError_t)launch_stage(c->d_tables, copy_src, copy_bytes, c->stream));
+  if (copy_bytes) CK((cudaError_t)launch_stage({c->d_tables, copy_src, copy_bytes}, {}, c->stream));
   int err = launch_frame(a, big_blocks, c->stream, &c->last_launches, events, &c->aux);
   if (err) return fail(GR_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString((cudaError_t)err));
   if (copy_bytes) ++c->last_launches;  // k_stage
@@ -1789,7 +1789,7 @@ struct gr_diff {
   uint32_t cols = 0, rows = 0;
   float* nhat = nullptr;
   float* d_world = nullptr;
-  float* bbox_partial = nullptr;        // kBBoxBlocks x 6
+  uint32_t* bbox_partial = nullptr;     // kBBoxBlocks x 6
   unsigned* bbox_done = nullptr;
   unsigned* sums_done = nullptr;        // k_diff_shade's and k_diff_scatter's finished CTAs, zero when idle
   double* d_partials = nullptr;         // per-warp sums (kDiffSlots x 4), zero when idle
@@ -2097,8 +2097,6 @@ int32_t gr_diff_backward(gr_diff* d, gr_diff_grads* g) {
   a.g_pos = g->positions;
   a.g_vcol = g->vertex_colors;
   a.g_tex = d->last.texture ? g->texture : nullptr;
-  CK(cudaMemsetAsync(g->positions, 0, sizeof(float) * 4 * (size_t)d->nv, c->stream));
-  CK(cudaMemsetAsync(g->vertex_colors, 0, sizeof(float) * 3 * (size_t)d->nv, c->stream));
   if (a.g_tex) CK(cudaMemsetAsync(a.g_tex, 0, sizeof(float) * 4 * (size_t)d->tw * (size_t)d->th, c->stream));
   int e = launch_diff_backward(a, c->stream);
   if (e) return fail(GR_ERR_CUDA, "diff backward: %s", cudaGetErrorString((cudaError_t)e));

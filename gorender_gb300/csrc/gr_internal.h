@@ -123,29 +123,36 @@ struct DevItem {
 // Plain float operations, one rounding each: device code is built with
 // --fmad=false and host code with -ffp-contract=off, so host and device give
 // the same bits.
-__host__ __device__ inline int box_visibility(const float* m, const float* bbox) {
+// The planes that a corner lies outside of, a bit each.
+__host__ __device__ inline unsigned box_corner_outside(const float* m, const float* b) {
   const float P[6][4] = {{-1, 0, 0, 1}, {1, 0, 0, 1}, {0, -1, 0, 1}, {0, 1, 0, 1}, {0, 0, 0, 1}, {0, 0, 50, 1}};
   const float N[6][4] = {{1, 0, 0, 1}, {-1, 0, 0, 1}, {0, 1, 0, 1}, {0, -1, 0, 1}, {0, 0, -1, 0}, {0, 0, 1, 0}};
-  unsigned out[8];
-  for (int c = 0; c < 8; ++c) {
-    const float* b = bbox + 4 * c;
-    float v[4];
-    for (int r = 0; r < 4; ++r) v[r] = ((m[4 * r] * b[0] + m[4 * r + 1] * b[1]) + m[4 * r + 2] * b[2]) + m[4 * r + 3] * b[3];
-    unsigned bits = 0;
-    for (int i = 0; i < 6; ++i) {
-      const float nv = ((N[i][0] * v[0] + N[i][1] * v[1]) + N[i][2] * v[2]) + N[i][3] * v[3];
-      const float np = ((N[i][0] * P[i][0] + N[i][1] * P[i][1]) + N[i][2] * P[i][2]) + N[i][3] * P[i][3];
-      if (nv - np > 0.0f) bits |= 1u << i;
-    }
-    out[c] = bits;
-  }
+  float v[4];
+  for (int r = 0; r < 4; ++r) v[r] = ((m[4 * r] * b[0] + m[4 * r + 1] * b[1]) + m[4 * r + 2] * b[2]) + m[4 * r + 3] * b[3];
+  unsigned bits = 0;
   for (int i = 0; i < 6; ++i) {
-    int outside = 0;
-    for (int c = 0; c < 8; ++c) outside += (out[c] >> i) & 1u;
-    if (outside == 8) return 0;
-    if (outside > 0) return 1;
+    const float nv = ((N[i][0] * v[0] + N[i][1] * v[1]) + N[i][2] * v[2]) + N[i][3] * v[3];
+    const float np = ((N[i][0] * P[i][0] + N[i][1] * P[i][1]) + N[i][2] * P[i][2]) + N[i][3] * P[i][3];
+    if (nv - np > 0.0f) bits |= 1u << i;
   }
-  return 2;
+  return bits;
+}
+
+// The visibility from the planes that some corners and all corners lie outside
+// of: the first plane with a corner outside decides.
+__host__ __device__ inline int box_visibility(unsigned some, unsigned all) {
+  if (!some) return 2;
+  return (all & some & (0u - some)) ? 0 : 1;
+}
+
+__host__ __device__ inline int box_visibility(const float* m, const float* bbox) {
+  unsigned some = 0, all = ~0u;
+  for (int c = 0; c < 8; ++c) {
+    const unsigned bits = box_corner_outside(m, bbox + 4 * c);
+    some |= bits;
+    all &= bits;
+  }
+  return box_visibility(some, all);
 }
 
 // Correctly rounded a / b from y = RN(1 / b), without a branch: one
@@ -415,9 +422,15 @@ struct AuxStream {
 int launch_frame(const FrameArgs& a, int big_blocks, void* stream, int* launches, void* const* events,
                  const AuxStream* aux = nullptr);
 
-// Copies bytes from a page-locked staging slot (its device address) to
+// Copies two ranges from a page-locked staging slot (its device address) to
 // device memory with one small kernel (16-byte aligned buffers).
-int launch_stage(void* dst, const void* src, size_t bytes, void* stream);
+struct StageCopy {
+  void* dst = nullptr;
+  const void* src = nullptr;
+  size_t bytes = 0;
+  __host__ __device__ uint32_t threads() const { return (uint32_t)(bytes / 16) + (uint32_t)(bytes % 16); }
+};
+int launch_stage(const StageCopy& c0, const StageCopy& c1, void* stream);
 
 // Persistent raster grid: SMs x resident CTAs of k_raster<TS> x waves.
 int raster_grid(int tile_shift, int waves);
@@ -426,7 +439,7 @@ int raster_grid(int tile_shift, int waves);
 // Writes the bounding box (Mesh.BoundingBox layout) of pos into each item's
 // bbox; partial holds 6 * kBBoxBlocks floats, *done is zero between calls.
 constexpr int kBBoxBlocks = 152;
-int launch_diff_bbox(const float* pos, int nv, DevItem* items, int num_items, float* partial, unsigned* done,
+int launch_diff_bbox(const float* pos, int nv, DevItem* items, int num_items, uint32_t* partial, unsigned* done,
                      void* stream);
 // nhat[n] = xyz of Vec4.Normalize(world * vnrm[n]) (renderer.go:328-331), w = 0.
 int launch_diff_normals(const float* world, const float* vnrm, int nn, float* nhat, void* stream);

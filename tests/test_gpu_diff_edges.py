@@ -27,6 +27,14 @@ def _records(diff):
     return torch.as_tensor(Dev(), device="cuda").cpu().numpy().copy()
 
 
+def _ids(diff):
+    ids, _, n = diff.buffers()
+
+    class Dev:
+        __cuda_array_interface__ = {"shape": (n,), "typestr": "<u4", "data": (ids, False), "version": 3}
+    return torch.as_tensor(Dev(), device="cuda").cpu().numpy().copy()
+
+
 def _dev(a):
     return torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
 
@@ -120,3 +128,33 @@ def test_losses_beyond_float32(value, count):
         assert np.isnan(loss)
     else:
         assert loss == np.inf
+
+
+@pytest.mark.parametrize("vertices", [1023, 1024, 1025, 2049])
+@pytest.mark.parametrize("last", [(0.0, 0.0, 0.0), (-0.0, 0.0, -0.0), (0.0, 9.0, 0.0), (np.nan, 0.0, 0.0), (np.inf, 0.0, 0.0)])
+def test_bounding_box_of_the_parameters(vertices, last):
+    """The box takes every vertex, faces or not, in CTAs of 1024, and decides
+    for each of 35 views (a warp takes a second one) what is clipped: views that
+    hold the mesh, cut it, look away from it, and a box with a NaN."""
+    sc = dc.small_case(views=35, size=40, level=3, tex_size=4, seed=8)
+    pos = np.tile(np.array(last + (1.0,), np.float32), (vertices, 1))
+    pos[:sc.mesh.nv] = sc.mesh.pos
+    sc.mesh = dataclasses.replace(sc.mesh, pos=pos)
+    for v, cam in enumerate(sc.cameras):
+        if v % 3 == 1:
+            cam.position = tuple(0.45 * x for x in cam.position)
+        elif v % 3 == 2:
+            cam.direction = tuple(-x for x in cam.direction)
+    views, world = dc.oracle_views(sc)
+    views = [(w, h, sc.flags, s, m) for w, h, s, m in views]
+    ctx = gr.Context(0)
+    try:
+        d = R.Diff(ctx, ctx.mesh(sc.mesh), world, views, tex_size=(0, 0))
+        p, vcol = _dev(pos), _dev(np.ones((vertices, 3)))
+        t = _dev(np.zeros((sum(w * h for w, h, *_ in views), 4)))
+        d.forward(p.data_ptr(), vcol.data_ptr(), None, sc.light, t.data_ptr())
+        ids, ref = _ids(d), dc.oracle_ids(sc)
+        assert (ref != dc.NO_FACE).any()
+        assert np.array_equal(ids, ref)
+    finally:
+        ctx.close()
