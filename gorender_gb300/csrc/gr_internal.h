@@ -193,15 +193,15 @@ struct alignas(16) TriWide {
 
 // The raster record of one binned triangle as stored (32 bytes): what the
 // raster needs of a narrow triangle follows from its integer screen corners
-// (|coordinate| < 2^14), its three W's and its order key -- the edge
-// functions, the top-left adjustment, the sum and the clamped pixel box are
+// (|coordinate| < 2^14), its three W's, the sum and its order key -- the edge
+// functions, the top-left adjustment and the clamped pixel box are
 // recomputed where the record is read (unpack_tri).  A wide triangle keeps
-// its sum here and its int64 edges and box in TriWide.
+// its int64 edges and box in TriWide.
 struct alignas(16) TriPacked {
   int16_t x0, y0, x1, y1, x2, y2;   // narrow triangles only
   uint32_t key;                     // bit 31: wide; bits 0..30: face*8 + fan + 1
   float w0, w1, w2;                 // clip-space W of the vertices (the rasteriser's z)
-  float sumf;                       // wide triangles only: float32(E01+E12+E20)
+  float sumf;                       // float32(E01+E12+E20)
 };
 static_assert(sizeof(TriPacked) == 32, "TriPacked layout");
 

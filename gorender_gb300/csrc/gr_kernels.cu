@@ -365,10 +365,10 @@ __device__ __forceinline__ TriRaster unpack_tri(const FrameArgs& a, uint32_t r, 
   TriRaster t;
   t.key = (uint32_t)c.w;
   t.w0 = w.x; t.w1 = w.y; t.w2 = w.z;
+  t.sumf = w.w;
   if (t.key & 0x80000000u) {
     const TriWide& wd = a.wide[r];
     t.a01 = t.b01 = t.c01 = t.a12 = t.b12 = t.c12 = t.a20 = t.b20 = t.c20 = 0;
-    t.sumf = w.w;
     t.bx0 = wd.bx0; t.bx1 = wd.bx1; t.by0 = wd.by0; t.by1 = wd.by1;
     return t;
   }
@@ -381,7 +381,6 @@ __device__ __forceinline__ TriRaster unpack_tri(const FrameArgs& a, uint32_t r, 
   if (!keeps_edge(t.a01, t.b01)) t.c01 -= 1;
   if (!keeps_edge(t.a12, t.b12)) t.c12 -= 1;
   if (!keeps_edge(t.a20, t.b20)) t.c20 -= 1;
-  t.sumf = __int2float_rn(t.c01 + t.c12 + t.c20);  // each within +-(2^29 + 1)
   t.bx0 = (int16_t)max(min(min(x0, x1), x2), 0);
   t.bx1 = (int16_t)min(max(max(x0, x1), x2), W - 1);
   t.by0 = (int16_t)max(min(min(y0, y1), y2), 0);
@@ -597,13 +596,13 @@ __device__ __forceinline__ bool narrow_covers(const Corners& c, const Box& box) 
   return cov < 0;
 }
 
-// Whether the adjusted edge functions of a narrow triangle add up to less than
-// zero: not those of the opposite winding.
-__device__ __forceinline__ bool narrow_faces(const Corners& c) {
+// The sum of a narrow triangle's adjusted edge functions: not below zero for
+// the opposite winding.
+__device__ __forceinline__ int narrow_sum(const Corners& c) {
   const int a01 = c.y0 - c.y1, b01 = c.x1 - c.x0, a12 = c.y1 - c.y2, b12 = c.x2 - c.x1, a20 = c.y2 - c.y0,
             b20 = c.x0 - c.x2;
   return c.x0 * c.y1 - c.x1 * c.y0 + c.x1 * c.y2 - c.x2 * c.y1 + c.x2 * c.y0 - c.x0 * c.y2 -
-             ((keeps_edge(a01, b01) ? 0 : 1) + (keeps_edge(a12, b12) ? 0 : 1) + (keeps_edge(a20, b20) ? 0 : 1)) < 0;
+         ((keeps_edge(a01, b01) ? 0 : 1) + (keeps_edge(a12, b12) ? 0 : 1) + (keeps_edge(a20, b20) ? 0 : 1));
 }
 
 // identifyTriangleTiles with the single screen tile on screen corners
@@ -1026,7 +1025,8 @@ __global__ void __maxnreg__(CTAS == 4 ? 64 : 104) k_setup(const FrameArgs a) {
         const Corners c = narrow_corners(make_float2(q0.x, q0.y), make_float2(q1.x, q1.y), make_float2(q2.x, q2.y));
         box = narrow_box(c, W, H);
         emit = box.x0 <= box.x1 && box.y0 <= box.y1;
-        if ((fl & 0xC0u) || a.keep_uncovered) emit = emit && narrow_faces(c);  // else k_cull has looked
+        const int sum = narrow_sum(c);
+        emit = emit && sum < 0;  // k_cull has looked, except in views with marks and fixed buffers
         if (emit && r >= a.rec_cap) {
           atomicMax(&a.work->rec_need, r + 1u);
           emit = false;
@@ -1036,7 +1036,7 @@ __global__ void __maxnreg__(CTAS == 4 ? 64 : 104) k_setup(const FrameArgs a) {
           dst[0] = make_int4((int)((uint32_t)(uint16_t)c.x0 | (uint32_t)c.y0 << 16),
                              (int)((uint32_t)(uint16_t)c.x1 | (uint32_t)c.y1 << 16),
                              (int)((uint32_t)(uint16_t)c.x2 | (uint32_t)c.y2 << 16), (int)okey);
-          reinterpret_cast<float4*>(dst)[1] = make_float4(q0.z, q1.z, q2.z, 0.0f);
+          reinterpret_cast<float4*>(dst)[1] = make_float4(q0.z, q1.z, q2.z, __int2float_rn(sum));
           if (!(fl & kViewFaceIds)) {  // face ids are drawn from the keys alone
             write_shade(a, r, p0.in, p1.in, p2.in, tex == -2 ? -3 : tex, p0.u, p0.v, q0.z, p1.u, p1.v, q1.z, p2.u, p2.v, q2.z);
             if (okey / (uint32_t)kKeysPerFace < a.face_cap) a.rec_of_face[okey / (uint32_t)kKeysPerFace] = r;
@@ -1319,12 +1319,17 @@ __device__ __forceinline__ uint32_t tex_sample(const DevTex* tex, float u, float
   return 0xFFFF00FFu;  // magenta (255, 0, 255, 255)
 }
 
+// colorIntensity (rasterizer.go:81-88).  Intensities in [0, 2^15) keep the
+// products below 2^23, where adding 2^23 rounded towards zero leaves their whole
+// part in the low bits: no range checks and no conversions.
 __device__ __forceinline__ uint32_t color_intensity(uint32_t c, float I) {
-  // colorIntensity (rasterizer.go:81-88)
-  uint32_t r = go_u8(fm((float)(c & 0xFFu), I));
-  uint32_t g = go_u8(fm((float)((c >> 8) & 0xFFu), I));
-  uint32_t b = go_u8(fm((float)((c >> 16) & 0xFFu), I));
-  return r | (g << 8) | (b << 16) | (c & 0xFF000000u);
+  const float fr = fm((float)(c & 0xFFu), I), fg = fm((float)((c >> 8) & 0xFFu), I), fb = fm((float)((c >> 16) & 0xFFu), I);
+  if (I >= 0.0f && I < 32768.0f) {
+    const uint32_t rg = __byte_perm(__float_as_uint(__fadd_rz(fr, 8388608.0f)), __float_as_uint(__fadd_rz(fg, 8388608.0f)), 0x0040);
+    const uint32_t ba = __byte_perm(__float_as_uint(__fadd_rz(fb, 8388608.0f)), c, 0x0070);
+    return __byte_perm(rg, ba, 0x5410);
+  }
+  return go_u8(fr) | (go_u8(fg) << 8) | (go_u8(fb) << 16) | (c & 0xFF000000u);
 }
 
 // FrameBuffer.CrossHair (rasterizer.go:209-217): four 3-pixel lines 3..5
@@ -1835,7 +1840,7 @@ __device__ __forceinline__ void resolve_pixel(const FrameArgs& a, const DevView&
 // fills 3840x2160 235 -> 87, 5.0 M-triangle icospheres 124 -> 79.
 template <int TS>
 __device__ __forceinline__ void raster_item(const FrameArgs& a, uint32_t tile, uint32_t slice, int view,
-                                            RasterSmem<TS>& sm) {
+                                            const uint4& ti, RasterSmem<TS>& sm) {
   constexpr int kThreads = RasterShape<TS>::kThreads;
   constexpr int kStride = RasterShape<TS>::kStride;
   constexpr int kWarps = RasterShape<TS>::kWarps;
@@ -1845,8 +1850,7 @@ __device__ __forceinline__ void raster_item(const FrameArgs& a, uint32_t tile, u
   const int warp = tid >> 5;
   const DevView& vw = a.views[view];
   // A tile's bin is split into up to kRasterMaxSlices slices, one work item each.
-  const uint4 ti = a.tile_info[tile];  // k_plan: entries, slices, key slot
-  const uint32_t n = ti.x;
+  const uint32_t n = ti.x;  // ti (k_plan): entries, slices, key slot, boxes
   const uint32_t nslices = ti.y;
   if (slice >= nslices) return;
   const uint32_t per = (((n + nslices - 1) / nslices) + 31u) & ~31u;
@@ -2207,26 +2211,34 @@ template <int TS, bool CLEAR>
 __global__ void __launch_bounds__(RasterShape<TS>::kThreads, RasterShape<TS>::kMinBlocks) k_raster(const FrameArgs a) {
   griddep_wait();
   __shared__ RasterSmem<TS> sm;
-  __shared__ uint32_t s_item, s_tile, s_slice, s_lastcta, s_clear;
-  __shared__ int s_view;
-  const uint32_t front = *(volatile uint32_t*)&a.work->plan_front;
-  const uint32_t total = front + *(volatile uint32_t*)&a.work->plan_back;
+  __shared__ uint32_t s_lastcta, s_clear;
+  // the queue and the item, here rather than in registers: the tile's info comes
+  // in the same chain as the item, and not again in every thread (960-triangle
+  // sphere at 640 x 360 50.3 -> 49.4 us, 8 views 65.1 -> 63.1; up to 8 items a
+  // grab while many are left: 256 views 2 % slower, 2 items 0.6 %)
+  __shared__ uint32_t s_front, s_total, s_item;
+  __shared__ uint2 s_work;
+  __shared__ uint4 s_info;
+  if (threadIdx.x == 0) {
+    s_front = *(volatile uint32_t*)&a.work->plan_front;
+    s_total = s_front + *(volatile uint32_t*)&a.work->plan_back;
+  }
   // The first item of every CTA is its block index; later ones come from the
   // counter, past the grid (no burst of atomics on one address at the start).
   for (bool first = true;; first = false) {
     if (threadIdx.x == 0) {
       const uint32_t i = first ? blockIdx.x : gridDim.x + atomicAdd(&a.work->raster_next, 1u);
       s_item = i;
-      if (i < total) {
-        const uint2 w = i < front ? a.plan[i] : a.plan[a.plan_cap - 1u - (i - front)];
-        s_tile = w.x;
-        s_slice = w.y & (uint32_t)(kRasterMaxSlices - 1);
-        s_view = (int)(w.y >> kSliceBits);  // found by k_plan
+      if (i < s_total) {
+        const uint2 w = i < s_front ? a.plan[i] : a.plan[a.plan_cap - 1u - (i - s_front)];
+        s_work = w;
+        s_info = a.tile_info[w.x];
       }
     }
     __syncthreads();
-    if (s_item >= total) break;
-    raster_item<TS>(a, s_tile, s_slice, s_view, sm);
+    if (s_item >= s_total) break;
+    const uint2 w = s_work;
+    raster_item<TS>(a, w.x, w.y & (uint32_t)(kRasterMaxSlices - 1), (int)(w.y >> kSliceBits), s_info, sm);
     __syncthreads();  // shared memory is reused by the next item
   }
   // Tiles without bin entries (batches shaded in place, k_plan's list): once
@@ -2273,7 +2285,7 @@ __global__ void __launch_bounds__(RasterShape<TS>::kThreads, RasterShape<TS>::kM
     r->nclip = w->nclip;
     r->clip_need = w->clip_need;
     r->max_bin = w->max_bin;
-    r->items = total;
+    r->items = s_total;
     r->novl = w->novl;
     r->ovl_need = w->ovl_need;
     w->novl = 0; w->ovl_need = 0;
@@ -2307,11 +2319,15 @@ __global__ void __launch_bounds__(RasterShape<TS>::kThreads, RasterShape<TS>::kM
 // k_resolve: one thread per pixel of a one-view frame, a warp 32 pixels of a
 // row; shades the winners whose keys k_raster stored (the shading of
 // resolve_pixel, at full occupancy so that its chain of dependent loads
-// overlaps across many warps).  Bound by issue (65-77 %, about 310 instructions a
+// overlaps across many warps).  Bound by issue (65-77 %, about 290 instructions a
 // textured pixel).  40 registers for six CTAs an SM: a box that fills 3840 x
 // 2160 96 -> 86 us (94 with the 44 registers and five CTAs that it takes by
 // itself), 1920 x 1080 20.9 -> 18.9, 1280 x 720 16.7 -> 15.7, against rows found by
 // a division, 64-bit texture coordinates and sums, and gathers one after the other.
+// Colours scaled without conversions and the edge sum read from the record: 87 ->
+// 82 us, the frame 211 -> 206 (1280 x 720 93.1 -> 90.4, with k_raster's 256 views
+// 1062 -> 1044).  Two or four rows a thread, the view's fields read once: 3-5 %
+// slower, the rows' loads one after the other.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256, 6) k_resolve(const FrameArgs a) {
   griddep_wait();

@@ -9,6 +9,7 @@ import pytest
 
 import gorender_gb300 as gr
 from gorender_gb300 import _native as N
+from gorender_gb300 import renderer as R
 from gorender_gb300 import scenes
 from oracle import oracle
 
@@ -77,7 +78,6 @@ def test_huge_triangles(tile):
     (the camera among them), more of them than its list holds (1024), alone and
     in a batch with a view of few tiles."""
     torch = pytest.importorskip("torch")
-    from gorender_gb300 import renderer as R
 
     ctx = gr.Context(0)
     try:
@@ -163,5 +163,35 @@ def test_faces_a_thread(faces):
         ref = oracle.draw_scene(sc, items_override=up.matrices, nthreads=8)
         assert ref[3] == 0 and tpf == ref[2] > faces // 2
         assert np.array_equal(rgba, ref[0]) and np.array_equal(z.view(np.uint32), ref[1].view(np.uint32))
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("strength", [1.0, -3.0, 300.0, 65534.9, 65535.1, 1e9, 1e38, np.inf, np.nan])
+def test_intensities(strength):
+    """Colours times intensities below zero, around 2^15 (products of 2^23 and
+    more are converted the general way), beyond whole numbers, infinite and NaN,
+    shaded by k_resolve and in place."""
+    torch = pytest.importorskip("torch")
+    sc = _scene(9, 900, seed=41)
+    light = np.array([0.3, 0.2, 1.0], np.float32) * np.float32(strength)
+    ctx = gr.Context(0)
+    try:
+        up = gr.UploadedScene(ctx, sc)
+        for k in range(3):
+            up.params.light[k] = float(light[k])
+        ref = oracle.draw_scene(sc, items_override=up.matrices, light=light, nthreads=4)
+        rgba, z, tpf = up.render()
+        assert ref[3] == 0 and tpf == ref[2] and len(np.unique(ref[0][..., 0])) > 1
+        assert np.array_equal(rgba, ref[0]) and np.array_equal(z.view(np.uint32), ref[1].view(np.uint32))
+        outs = [(torch.zeros((sc.height, sc.width, 4), dtype=torch.uint8, device="cuda"),
+                 torch.zeros((sc.height, sc.width), dtype=torch.float32, device="cuda")) for _ in range(2)]
+        torch.cuda.synchronize()
+        b = R.Batch(ctx, [(up.params, c.data_ptr(), d.data_ptr()) for c, d in outs],
+                    [(h, m[0], m[1], v) for v in range(2) for h, m in zip(up.mesh_handles, up.matrices)], autotune=False)
+        b.run()
+        b.sync()
+        for c, d in outs:
+            assert np.array_equal(c.cpu().numpy(), ref[0])
     finally:
         ctx.close()
