@@ -142,7 +142,7 @@ struct gr_context {
   unsigned long long* view_tpf_out = nullptr;
   unsigned long long* h_view_tpf = nullptr;
   int views_cap = 0;
-  uint2* plan = nullptr;            // raster work queue
+  RasterWork* plan = nullptr;       // raster work queue
   uint2* empty_tiles = nullptr;     // tiles without bin entries (cleared by k_raster<TS, true>)
   uint32_t empty_cap = 0;
   uint32_t plan_cap = 0;

@@ -227,6 +227,18 @@ struct TriColor {
   float c[9];
 };
 
+// One raster work item: a slice of a tile, with all that k_raster needs to know
+// of the tile (read with the item: one dependent load less than through the
+// tile's info).
+struct alignas(16) RasterWork {
+  uint32_t tile;
+  uint32_t slice_view;  // slice | view << kSliceBits
+  uint32_t entries;     // of the tile's bin
+  uint32_t slices;      // of the tile, and the two flags
+};
+constexpr uint32_t kWorkSmall = 0x40000000u;  // RasterWork::slices: no box of the tile beyond kSmallBox pixels
+constexpr uint32_t kWorkSlot = 0x80000000u;   // ... the slice's keys go to the slot numbered like the item
+
 // One binned fan triangle's overlay marks (ShowEdges / ShowVertices,
 // renderer.go:191-216): its screen corners and its draw-order key.
 struct Overlay {
@@ -317,7 +329,7 @@ struct FrameArgs {
                                     // host (every CTA fences at system scope before it retires)
   unsigned long long* view_tpf;     // per view: binned triangles (zeroed by k_plan)
   unsigned long long* view_tpf_out; // per view: published by k_plan
-  uint2* plan;                      // raster work items (tile, slice | view << kSliceBits), plan_cap entries
+  RasterWork* plan;                 // raster work items, plan_cap entries
   uint2* empty_tiles;               // (tile, view) of tiles without bin entries, cleared by k_raster
   uint32_t empty_cap;
   int clear_empty;                  // nonzero: tiles without bin entries go to that list (batches
@@ -329,7 +341,7 @@ struct FrameArgs {
   uint32_t* ovl_key;                // per pixel of every view: max (order key * 2 + vertex mark), 0 = none
   unsigned long long* pkey;         // per pixel of every view: final visibility keys, shaded by k_resolve
                                     // (null: k_raster shades each tile itself)
-  uint4* tile_info;                 // per tile, from k_plan: x bin entries, y raster slices, z first key
+  uint4* tile_info;                 // per tile of a one-view frame, from k_plan: x bin entries, y raster slices, z first key
                                     // slot of a split tile of a one-view frame (kNoSlot: merged in gkey),
                                     // w pixels of its large entries' boxes
   unsigned long long* slot_keys;    // one-view frames: slot_cap slots of TS x TS keys, one per slice of a

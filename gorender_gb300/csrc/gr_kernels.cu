@@ -1839,8 +1839,8 @@ __device__ __forceinline__ void resolve_pixel(const FrameArgs& a, const DevView&
 // at 1920x1080 40 -> 31, 960-triangle sphere at 640x360 28 -> 18, a box that
 // fills 3840x2160 235 -> 87, 5.0 M-triangle icospheres 124 -> 79.
 template <int TS>
-__device__ __forceinline__ void raster_item(const FrameArgs& a, uint32_t tile, uint32_t slice, int view,
-                                            const uint4& ti, RasterSmem<TS>& sm) {
+__device__ __forceinline__ void raster_item(const FrameArgs& a, const uint32_t& item, const RasterWork& work,
+                                            RasterSmem<TS>& sm) {
   constexpr int kThreads = RasterShape<TS>::kThreads;
   constexpr int kStride = RasterShape<TS>::kStride;
   constexpr int kWarps = RasterShape<TS>::kWarps;
@@ -1848,11 +1848,11 @@ __device__ __forceinline__ void raster_item(const FrameArgs& a, uint32_t tile, u
   uint32_t& s_last = sm.last;
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
-  const DevView& vw = a.views[view];
+  const uint32_t tile = work.tile, slice = work.slice_view & (uint32_t)(kRasterMaxSlices - 1);
+  const DevView& vw = a.views[work.slice_view >> kSliceBits];
   // A tile's bin is split into up to kRasterMaxSlices slices, one work item each.
-  const uint32_t n = ti.x;  // ti (k_plan): entries, slices, key slot, boxes
-  const uint32_t nslices = ti.y;
-  if (slice >= nslices) return;
+  const uint32_t n = work.entries;
+  const uint32_t nslices = work.slices & ~(kWorkSmall | kWorkSlot);
   const uint32_t per = (((n + nslices - 1) / nslices) + 31u) & ~31u;
   const uint32_t lo = min(n, slice * per), hi = min(n, lo + per);
   const uint32_t lt = tile - vw.tile_base;
@@ -1875,7 +1875,7 @@ __device__ __forceinline__ void raster_item(const FrameArgs& a, uint32_t tile, u
     *reinterpret_cast<ulonglong2*>(mine) = make_ulonglong2(BG_KEY, BG_KEY);
     *reinterpret_cast<ulonglong2*>(mine + 2) = make_ulonglong2(BG_KEY, BG_KEY);
     // no box of the tile beyond kSmallBox pixels: the tile may be one of tiny triangles
-    const bool tiny = ti.w == 0u && n >= 64u;
+    const bool tiny = (work.slices & kWorkSmall) && n >= 64u;
     if (tiny) __syncthreads();  // raster_stage tests pixels too
     for (uint32_t base = lo; base < hi; base += kThreads) {
       const uint32_t m = min((uint32_t)kThreads, hi - base);
@@ -1904,13 +1904,13 @@ __device__ __forceinline__ void raster_item(const FrameArgs& a, uint32_t tile, u
       __syncthreads();
     }
 
-    if (nslices > 1 && ti.z != kNoSlot) {
+    if (work.slices & kWorkSlot) {
       // One view: this slice's keys go to a slot of their own with plain
       // stores, and k_resolve takes the max over the tile's slots -- the
       // kernel boundary orders them, so no slice waits on a fence or hands
       // over (the merge below took a fifth of this kernel's warp time on
       // single frames).
-      ulonglong2* dst = reinterpret_cast<ulonglong2*>(a.slot_keys + (size_t)(ti.z + slice) * (TS * TS) + row * TS + col);
+      ulonglong2* dst = reinterpret_cast<ulonglong2*>(a.slot_keys + (size_t)item * (TS * TS) + row * TS + col);
       dst[0] = *reinterpret_cast<const ulonglong2*>(mine);
       dst[1] = *reinterpret_cast<const ulonglong2*>(mine + 2);
       return;
@@ -2188,14 +2188,16 @@ __global__ void __launch_bounds__(256) k_plan(const FrameArgs a) {
   // it the latter 1 % slower).
   const uint32_t slot =
       heavy && ns > 1 && ns <= 8u && a.slot_keys && s_bf + mf + ns <= a.slot_cap ? s_bf + mf : kNoSlot;
-  a.tile_info[tile] = make_uint4(min(count, a.bin_cap), ns, slot, boxes);
+  const uint32_t entries = min(count, a.bin_cap);
+  if (a.pkey) a.tile_info[tile] = make_uint4(entries, ns, slot, 0u);
+  const uint32_t slices = ns | (boxes ? 0u : kWorkSmall) | (slot != kNoSlot ? kWorkSlot : 0u);
   if (clear) {
     if (s_be + me < a.empty_cap) a.empty_tiles[s_be + me] = make_uint2(tile, (uint32_t)view);
   } else if (none) {
   } else if (heavy) {
-    for (uint32_t k = 0; k < ns; ++k) a.plan[s_bf + mf + k] = make_uint2(tile, k | vbits);
+    for (uint32_t k = 0; k < ns; ++k) a.plan[s_bf + mf + k] = RasterWork{tile, k | vbits, entries, slices};
   } else {
-    a.plan[a.plan_cap - 1u - (s_bb + mb)] = make_uint2(tile, vbits);
+    a.plan[a.plan_cap - 1u - (s_bb + mb)] = RasterWork{tile, vbits, entries, slices};
   }
 }
 
@@ -2262,13 +2264,13 @@ __global__ void __launch_bounds__(RasterShape<TS>::kThreads, RasterShape<TS>::kM
   griddep_wait();
   __shared__ RasterSmem<TS> sm;
   __shared__ uint32_t s_lastcta, s_clear;
-  // the queue and the item, here rather than in registers: the tile's info comes
-  // in the same chain as the item, and not again in every thread (960-triangle
-  // sphere at 640 x 360 50.3 -> 49.4 us, 8 views 65.1 -> 63.1; up to 8 items a
-  // grab while many are left: 256 views 2 % slower, 2 items 0.6 %)
+  // the queue and the item, here rather than in registers; what there is to know
+  // of the tile comes with the item, not through the tile's info in every thread
+  // (960-triangle sphere at 640 x 360 50.3 -> 49.4 us read by the thread that takes
+  // the item; a box that fills 3840 x 2160 203.5 -> 201.5 in the item itself).  Up to
+  // 8 items a grab while many are left: 256 views 2 % slower, 2 items 0.6 %.
   __shared__ uint32_t s_front, s_total, s_item;
-  __shared__ uint2 s_work;
-  __shared__ uint4 s_info;
+  __shared__ RasterWork s_work;
   if (threadIdx.x == 0) {
     s_front = *(volatile uint32_t*)&a.work->plan_front;
     s_total = s_front + *(volatile uint32_t*)&a.work->plan_back;
@@ -2279,16 +2281,11 @@ __global__ void __launch_bounds__(RasterShape<TS>::kThreads, RasterShape<TS>::kM
     if (threadIdx.x == 0) {
       const uint32_t i = first ? blockIdx.x : gridDim.x + atomicAdd(&a.work->raster_next, 1u);
       s_item = i;
-      if (i < s_total) {
-        const uint2 w = i < s_front ? a.plan[i] : a.plan[a.plan_cap - 1u - (i - s_front)];
-        s_work = w;
-        s_info = a.tile_info[w.x];
-      }
+      if (i < s_total) s_work = i < s_front ? a.plan[i] : a.plan[a.plan_cap - 1u - (i - s_front)];
     }
     __syncthreads();
     if (s_item >= s_total) break;
-    const uint2 w = s_work;
-    raster_item<TS>(a, w.x, w.y & (uint32_t)(kRasterMaxSlices - 1), (int)(w.y >> kSliceBits), s_info, sm);
+    raster_item<TS>(a, s_item, s_work, sm);
     __syncthreads();  // shared memory is reused by the next item
   }
   // Tiles without bin entries (batches shaded in place, k_plan's list): once

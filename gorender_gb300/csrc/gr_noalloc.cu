@@ -75,7 +75,7 @@ constexpr Layout make_layout() {
   l.views = o; o += up256(sizeof(DevView));
   l.view_tpf = o; o += up256(sizeof(unsigned long long));
   l.view_tpf_out = o; o += up256(sizeof(unsigned long long));
-  l.plan = o; o += up256(sizeof(uint2) * kTiles * kRasterMaxSlices);
+  l.plan = o; o += up256(sizeof(RasterWork) * kTiles * kRasterMaxSlices);
   l.empty = o; o += up256(sizeof(uint2) * kTiles);
   l.rast = o; o += up256(sizeof(TriPacked) * kRecCap);
   l.shade = o; o += up256(sizeof(TriShade) * kRecCap);
@@ -323,7 +323,7 @@ extern "C" int32_t gr_draw_noalloc(int32_t device, const gr_noalloc_object* obje
   a.result = (DevResult*)(base + kLayout.result);
   a.view_tpf = (unsigned long long*)(base + kLayout.view_tpf);
   a.view_tpf_out = (unsigned long long*)(base + kLayout.view_tpf_out);
-  a.plan = (uint2*)(base + kLayout.plan);
+  a.plan = (RasterWork*)(base + kLayout.plan);
   a.plan_cap = (uint32_t)(kTiles * kRasterMaxSlices);
   a.empty_tiles = (uint2*)(base + kLayout.empty);
   a.empty_cap = (uint32_t)kTiles;
