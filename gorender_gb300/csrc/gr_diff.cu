@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(kThreads) k_diff_shade(const DiffArgs a) {
     if (px >= vw.W || py >= vw.H) break;
     const size_t gp = (size_t)vw.pix_base + (size_t)py * (size_t)vw.W + (size_t)px;
     const uint32_t gf = a.ids[gp];
-    const float4 tg = reinterpret_cast<const float4*>(a.target)[gp];
+    const float4 tg = __ldcs(reinterpret_cast<const float4*>(a.target) + gp);
     DiffRecord rec{kNoFace, kNoFace, 0.0f, 0.0f};
     float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (gf != kNoFace) {
@@ -537,7 +537,8 @@ __global__ void __launch_bounds__(kThreads) k_diff_shade(const DiffArgs a) {
 // pixels were paired).  64 views of 512 x 512 pixels of an 81,920-face mesh: 400 ->
 // 254 us with the gathered data packed, the normals and the light's sums left
 // to k_diff_scatter (303 us), neighbouring pixels of a face paired (263; side
-// by side alone 272) and the face ids read a step ahead (254).
+// by side alone 272) and the face ids read a step ahead (254); records and targets, read once, evict-first here
+// and in k_diff_shade: the step 1184 -> 1179.
 __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
   const DiffView& vw = a.views[blockIdx.z];
   // the vertices' gradients, which only k_diff_scatter adds to, start at zero
@@ -559,7 +560,7 @@ __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
     if (!__any_sync(0xffffffffu, on)) continue;
     DiffRecord rec{kNoFace, kNoFace, 0.0f, 0.0f};
     if (on) {
-      const uint4 rw = reinterpret_cast<const uint4*>(a.rec)[gp];
+      const uint4 rw = __ldcs(reinterpret_cast<const uint4*>(a.rec) + gp);
       rec = DiffRecord{rw.x, rw.y, __uint_as_float(rw.z), __uint_as_float(rw.w)};
     }
     const int f = (int)(rec.face - vw.face_base);
@@ -571,7 +572,7 @@ __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
       Shade s;
       const int ni[3] = {(int)face.x[3], (int)face.x[4], (int)face.x[5]};
       shade(a, g, rec.l0, rec.l1, rec.texel, ni, s);
-      const float4 tg = reinterpret_cast<const float4*>(a.target)[gp];
+      const float4 tg = __ldcs(reinterpret_cast<const float4*>(a.target) + gp);  // read once, like the records
       const float go[4] = {2.0f * (s.out.x - tg.x), 2.0f * (s.out.y - tg.y), 2.0f * (s.out.z - tg.z),
                            2.0f * (s.out.w - tg.w)};
       const float t3[3] = {s.t.x, s.t.y, s.t.z};
