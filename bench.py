@@ -151,7 +151,7 @@ STAGES = {"project_stage": "k_light + k_vertex + k_cull + k_clip + k_setup",
 STAGE_KERNELS = {"project_stage": ["k_light", "k_vertex", "k_cull", "k_clip", "k_setup"],
                  "bin_stage": ["k_bin_big", "k_overlay"],
                  "raster_stage": ["k_plan", "k_raster", "k_resolve"],
-                 "forward": ["k_diff_vertices", "k_diff_tables", "k_diff_shade"],
+                 "forward": ["k_diff_prepare", "k_diff_shade"],
                  "backward": ["k_diff_grad", "k_diff_scatter"]}
 
 
@@ -553,8 +553,8 @@ def bench_diff(device):
         tb.append(ctx.elapsed_ms(7, 8))
     mf, mb = statistics.median(tf), statistics.median(tb)
     roof = roofline_of("diff64", {"forward": mf, "backward": mb}, diff_bytes(sc, views),
-                       {"forward": "visibility pass (the frame kernels in face-id mode) + k_diff_vertices + "
-                                   "k_diff_tables + k_diff_shade",
+                       {"forward": "visibility pass (the frame kernels in face-id mode) + k_diff_prepare + "
+                                   "k_diff_shade",
                         "backward": "k_diff_grad + k_diff_scatter"})
     d.close()
     for x in p + q + g + [target, zeros]:
