@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(kThreads) k_diff_shade(const DiffArgs a) {
 // 254 us with the gathered data packed, the normals and the light's sums left
 // to k_diff_scatter (303 us), neighbouring pixels of a face paired (263; side
 // by side alone 272) and the face ids read a step ahead (254); records and targets, read once, evict-first here
-// and in k_diff_shade: the step 1184 -> 1179.
+// and in k_diff_shade: the step 1184 -> 1179.  The light's weights in FP64: 288.
 __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
   const DiffView& vw = a.views[blockIdx.z];
   // the vertices' gradients, which only k_diff_scatter adds to, start at zero
@@ -620,13 +620,15 @@ __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
     // Colour and position gradients go to the face's corners first
     // (k_diff_scatter adds them to the vertices): a vertex is shared by about
     // six faces, so per-face sums meet far fewer atomics at one address
-    // (measured: the backward pass 20 % faster).  Each corner's seven sums are
-    // two float4 (padded to eight floats), and the texel's four one float4:
-    // seven vector reductions a pixel.  The seventh is the corner's weight in
-    // the light's gradient, dI/dL = sum_k l_k 0.5 nhat_k, which k_diff_scatter
-    // multiplies with its normal: no normal is read here.  The reductions'
-    // way out of the SM bounds this kernel, so pixels of one face side by side
-    // or one above the other are added up first.
+    // (measured: the backward pass 20 % faster).  Each corner's six sums are a
+    // float4 and a float2, the texel's four a float4.  Beside them stands, as a
+    // double, the corner's weight in the light's gradient, dI/dL = sum_k l_k 0.5
+    // nhat_k, which k_diff_scatter multiplies with its normal: no normal is read
+    // here, and the light is summed over all pixels in FP64, up to its end (in
+    // float32 it was 35 us faster at 64 views and its error, 1.3e-8 to 1.1e-7 over seven
+    // cases, up to three times as large in one).  The reductions' way out of
+    // the SM bounds this kernel, so pixels of one face side by side or one
+    // above the other are added up first.
     on = rec.face != kNoFace;
 #pragma unroll
     for (int o = 1; o <= 8; o <<= 3) {
@@ -649,7 +651,8 @@ __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         atomicAdd(gf + 2 * k, make_float4(gc[k][0], gc[k][1], gc[k][2], gc[k][3]));
-        atomicAdd(gf + 2 * k + 1, make_float4(gc[k][4], gc[k][5], gc[k][6], 0.0f));
+        atomicAdd(reinterpret_cast<float2*>(gf + 2 * k + 1), make_float2(gc[k][4], gc[k][5]));
+        atomicAdd(reinterpret_cast<double*>(gf + 2 * k + 1) + 1, (double)gc[k][6]);
       }
     }
   }
@@ -692,13 +695,14 @@ __global__ void __launch_bounds__(kThreads) k_diff_scatter(const DiffArgs a) {
           for (int j = 3; j < 6; ++j) atomicAdd(a.g_pos + 4 * (size_t)v + (j - 3), x[j]);
         }
       }
-      if (q.z != 0.0f) {
-        gl[0] += (double)q.z * (double)n.x;
-        gl[1] += (double)q.z * (double)n.y;
-        gl[2] += (double)q.z * (double)n.z;
+      const double w = __hiloint2double(__float_as_int(q.w), __float_as_int(q.z));
+      if (w != 0.0) {
+        gl[0] += w * (double)n.x;
+        gl[1] += w * (double)n.y;
+        gl[2] += w * (double)n.z;
       }
       if (p.x != 0.0f || p.y != 0.0f || p.z != 0.0f || p.w != 0.0f) gf[2 * k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (q.x != 0.0f || q.y != 0.0f || q.z != 0.0f) gf[2 * k + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (q.x != 0.0f || q.y != 0.0f || w != 0.0) gf[2 * k + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
   }
 #pragma unroll

@@ -410,7 +410,7 @@ struct DiffArgs {
   float* g_tex;                     // th x tw x 4
   double* g_light;                  // 3 (page-locked host memory, its device address)
   double* partials;                 // kDiffSlots x {loss, light x, y, z}: per-warp sums, zero when idle
-  float* g_face;                    // nf x 3 corners x {colour r, g, b, position x, y, z, light weight, 0}:
+  float* g_face;                    // nf x 3 corners x {colour r, g, b, position x, y, z, light weight (a double)}:
                                     // the backward's per-face sums before k_diff_scatter (zero when idle),
                                     // two float4 a corner
   unsigned* done;                   // CTAs that have added to the partials (zero when idle)
