@@ -1772,7 +1772,9 @@ struct gr_diff {
   std::vector<gr_draw_item> items;      // one item per view
   std::vector<DiffView> hviews;
   uint64_t pixels = 0;
-  int max_w = 0, max_h = 0;
+  int max_side = 0;
+  int blocks_down = 1;                  // blocks of pixels a CTA
+  uint32_t blocks = 0, view_blocks = 0; // CTAs of the per-pixel kernels, and of each view where all have as many
   DiffView* d_views = nullptr;
   DevView* d_frame_views = nullptr;     // the visibility pass's own tables
   DevItem* d_items = nullptr;
@@ -1809,11 +1811,10 @@ DiffArgs diff_args(const gr_diff* d, const gr_diff_params& p, const float* targe
   const MeshRec& mr = d->ctx->meshes[d->mesh];
   a.views = d->d_views;
   a.num_views = (int)d->hviews.size();
-  a.max_w = d->max_w;
-  a.max_h = d->max_h;
-  // four blocks of 8 rows a CTA where that leaves each SM several CTAs: one
-  // reduction of the loss and one look at the counter for 1024 pixels
-  a.rows8 = d->pixels >= (1ull << 21) ? 8 : 1;
+  a.max_side = d->max_side;
+  a.blocks_down = d->blocks_down;
+  a.blocks = d->blocks;
+  a.view_blocks = d->view_blocks;
   a.vert_blocks = (d->nv + 255) / 256;
   a.norm_blocks = (d->nn + 255) / 256;
   a.nv = d->nv; a.nf = d->nf; a.nn = d->nn;
@@ -1840,6 +1841,30 @@ DiffArgs diff_args(const gr_diff* d, const gr_diff_params& p, const float* targe
   a.g_face = d->d_gface;
   a.done = d->sums_done;
   return a;
+}
+
+// The CTAs of the per-pixel kernels: a list over all views, each with its own.
+int32_t diff_blocks(gr_diff* d) {
+  // eight blocks of 256 pixels a CTA where that leaves each SM several CTAs: one
+  // reduction of the loss and one look at the counter for 2048 pixels
+  d->blocks_down = d->pixels >= (1ull << 21) ? 8 : 1;
+  uint64_t total = 0;
+  d->view_blocks = 0;
+  bool even = true;
+  for (DiffView& v : d->hviews) {
+    const int wide = diff_block_wide(v.W), high = kDiffThreads / wide * d->blocks_down;
+    v.blocks_x = (v.W + wide - 1) / wide;
+    v.block_base = (uint32_t)total;
+    const uint32_t n = (uint32_t)v.blocks_x * (uint32_t)((v.H + high - 1) / high);
+    if (!total) d->view_blocks = n;
+    even = even && n == d->view_blocks;
+    total += n;
+    if (total > 0x7FFFFFFFull)  // out of reach: fewer than 2^32 pixels and 2^16 views make about 2^28 at most
+      return fail(GR_ERR_UNSUPPORTED, "too many blocks of pixels over all views");
+  }
+  d->blocks = (uint32_t)total;
+  if (!even) d->view_blocks = 0;
+  return GR_OK;
 }
 
 void diff_free(gr_diff* d) {
@@ -1961,11 +1986,11 @@ int32_t gr_diff_create(gr_context* c, int32_t mesh, const float* world, int32_t 
       hv.Qf[2 * j + 1] = (float)(hv.Q[j] - (double)hi);
     }
     pix += (uint64_t)dv.width * (uint64_t)dv.height;
-    d->max_w = std::max(d->max_w, dv.width);
-    d->max_h = std::max(d->max_h, dv.height);
+    d->max_side = std::max(d->max_side, std::max(dv.width, dv.height));
     if (pix >= (1ull << 32)) st = fail(GR_ERR_UNSUPPORTED, "more than 2^32 pixels over all views");
   }
   d->pixels = pix;
+  if (!st) st = diff_blocks(d);
   if (!st) st = dev_alloc(&d->d_views, (size_t)num_views);
   if (!st) st = dev_alloc(&d->d_frame_views, (size_t)num_views);
   if (!st) st = dev_alloc(&d->d_items, (size_t)num_views);

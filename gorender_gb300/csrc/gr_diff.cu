@@ -53,7 +53,7 @@ namespace gr {
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = kDiffThreads;
 static_assert(kDiffSlots == kThreads, "sum_slots takes a slot a thread");
 
 // Waits for the kernel ahead on the stream (launch_after); a no-op after a
@@ -394,33 +394,58 @@ __device__ __forceinline__ int wrap_index(float u, int n) {
   return i < 0 ? i + n : i;
 }
 
-// The pixels of a CTA: 32 wide, a.rows8 x 8 rows high, each warp an 8 x 4 block
-// of every 8 rows (blocks share more faces, and so more gathered lines, than
-// rows of 32 do).
-__device__ __forceinline__ int block_x() {
-  return (int)blockIdx.x * 32 + (int)((threadIdx.x >> 5) & 3u) * 8 + (int)(threadIdx.x & 7u);
-}
-__device__ __forceinline__ int block_y(const DiffArgs& a, int k) {
-  return ((int)blockIdx.y * a.rows8 + k) * 8 + (int)(threadIdx.x >> 7) * 4 + (int)((threadIdx.x >> 3) & 3u);
+// The pixels of a thread: column x of its view, rows y, y + rows, ..., a.blocks_down
+// of them.  A CTA's warps take an 8 x 4 block each (blocks share more faces, and so more
+// gathered lines, than rows of 32 do), side by side first (diff_block_wide).
+struct Pixels {
+  int view, x, y, rows;
+};
+
+// The CTAs of all views stand in one list, so that each view has those that its own
+// size asks for (a grid of the largest width by the largest height made 2048 x 64
+// views beside 64 x 2048 ones three times as slow, and numbers of CTAs beyond 32 bits).
+// Views of as many CTAs each, the usual case, need a division; others a search, 32
+// views a round and the same in every warp.
+__device__ __forceinline__ Pixels block_pixels(const DiffArgs& a) {
+  int view = 0;
+  if (a.view_blocks) {
+    view = (int)(blockIdx.x / a.view_blocks);
+  } else {
+    const int lane = (int)(threadIdx.x & 31u);
+    int hi = a.num_views - 1;  // the last view whose first CTA is at most this one lies in [view, hi]
+    while (view < hi) {
+      const int step = (hi - view + 31) >> 5, p = view + 1 + lane * step;
+      const unsigned got = __ballot_sync(0xffffffffu, p <= hi && a.views[p].block_base <= blockIdx.x);
+      if (!got) break;
+      view += 1 + (31 - __clz((int)got)) * step;
+      hi = min(hi, view + step - 1);
+    }
+  }
+  const DiffView& vw = a.views[view];
+  const int local = (int)(blockIdx.x - vw.block_base);
+  const int by = local / vw.blocks_x, bx = local - by * vw.blocks_x;
+  const int wide = diff_block_wide(vw.W), rows = kThreads / wide, warp = (int)(threadIdx.x >> 5);
+  const int across = wide >> 3, wy = warp / across, wx = warp - wy * across;
+  return Pixels{view, bx * wide + wx * 8 + (int)(threadIdx.x & 7u),
+                by * a.blocks_down * rows + wy * 4 + (int)((threadIdx.x >> 3) & 3u), rows};
 }
 
 // The calling warp's slot of DiffArgs::partials (warps spread over the slots
 // so that their atomics rarely meet).
-__device__ __forceinline__ int diff_slot(unsigned block) {
-  return (int)((block * (kThreads / 32) + (threadIdx.x >> 5)) & (kDiffSlots - 1));
+__device__ __forceinline__ int diff_slot() {
+  return (int)((blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) & (kDiffSlots - 1));
 }
 
-// The last of a grid's `blocks` CTAs to get here (an atomic counter, no
-// waiting) writes the sums of components [c0, c0 + N) of the slots to dst
+// The last of a grid's CTAs to get here (an atomic counter, no waiting) writes the sums of components [c0, c0 + N) of the slots to dst
 // (page-locked host memory, through its device address: no copy follows) and
 // returns the slots and the counter to zero.  Called by every thread.
 template <int N>
-__device__ __forceinline__ void sum_slots(const DiffArgs& a, unsigned blocks, int c0, double* dst) {
+__device__ __forceinline__ void sum_slots(const DiffArgs& a, int c0, double* dst) {
   __shared__ double s_w[N][kThreads / 32];
   __shared__ bool s_last;
   if ((threadIdx.x & 31) == 0) __threadfence();  // the warp's slot sums before the count
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(a.done, 1u) == blocks - 1u;
+  if (threadIdx.x == 0) s_last = atomicAdd(a.done, 1u) == gridDim.x - 1u;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
@@ -448,23 +473,23 @@ __device__ __forceinline__ void sum_slots(const DiffArgs& a, unsigned blocks, in
   if (threadIdx.x == 0) *a.done = 0u;
 }
 
-// Forward: per pixel record, shaded pixel and the loss.  Grid (columns / 32,
-// rows / (8 a.rows8), views).  Bound by the latency of its gathers (face, then
+// Forward: per pixel record, shaded pixel and the loss.  Bound by the latency of its gathers (face, then
 // corners, then texel: 40 % of the issue slots, 38 % of the memory rate).  64 views
 // of 512 x 512 pixels of an 81,920-face mesh: 394 -> 238 us with the gathered data
 // packed (36 loads a covered pixel before, 13 now), blocks instead of rows of
 // pixels a warp, and the loss out of the FP64 pipe.
-__global__ void __launch_bounds__(kThreads) k_diff_shade(const DiffArgs a) {
+__global__ void __launch_bounds__(kThreads, 4) k_diff_shade(const DiffArgs a) {
   griddep_wait();
-  const DiffView& vw = a.views[blockIdx.z];
-  const int px = block_x();
+  const Pixels at = block_pixels(a);
+  const DiffView& vw = a.views[at.view];
+  const int px = at.x;
   // the pixels' losses, summed as hi + lo (error-free sums; the warp's sum goes
   // to FP64), since FP64 additions, one a pixel or five for each warp's tree,
   // held this kernel at the FP64 pipe's rate.  Losses near float32's end, and
   // infinities and NaN, are summed apart, scaled by 2^-80.
   float hi = 0.0f, lo = 0.0f, bhi = 0.0f, blo = 0.0f;
-  for (int k = 0; k < a.rows8; ++k) {
-    const int py = block_y(a, k);
+  for (int k = 0; k < a.blocks_down; ++k) {
+    const int py = at.y + k * at.rows;
     if (px >= vw.W || py >= vw.H) break;
     const size_t gp = (size_t)vw.pix_base + (size_t)py * (size_t)vw.W + (size_t)px;
     const uint32_t gf = a.ids[gp];
@@ -475,7 +500,7 @@ __global__ void __launch_bounds__(kThreads) k_diff_shade(const DiffArgs a) {
       const int4* fr = a.faces + 4 * (size_t)(gf - vw.face_base);
       const Word8 face = ldg8(fr);
       FaceGeom g;
-      face_geom(a, blockIdx.z, face, px, py, g);
+      face_geom(a, at.view, face, px, py, g);
       if (g.ok) {
         // the visibility pass snaps corners to whole pixels, so a pixel may lie
         // just outside the unsnapped face: its barycentrics are clipped to it
@@ -527,9 +552,8 @@ __global__ void __launch_bounds__(kThreads) k_diff_shade(const DiffArgs a) {
     sum += (isfinite(bhi) ? (double)bhi + (double)blo : (double)bhi) * 0x1p80;
   }
   // one atomic into the warp's slot, so that warps never wait for each other
-  const unsigned block = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  if ((threadIdx.x & 31) == 0 && sum != 0.0) atomicAdd(a.partials + 4 * diff_slot(block), sum);
-  sum_slots<1>(a, gridDim.x * gridDim.y * gridDim.z, 0, a.loss);
+  if ((threadIdx.x & 31) == 0 && sum != 0.0) atomicAdd(a.partials + 4 * diff_slot(), sum);
+  sum_slots<1>(a, 0, a.loss);
 }
 
 // Backward: gradients of the loss of the last forward pass.  Bound by the
@@ -540,23 +564,23 @@ __global__ void __launch_bounds__(kThreads) k_diff_shade(const DiffArgs a) {
 // by side alone 272) and the face ids read a step ahead (254); records and targets, read once, evict-first here
 // and in k_diff_shade: the step 1184 -> 1179.  The light's weights in FP64: 288.
 __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
-  const DiffView& vw = a.views[blockIdx.z];
+  const Pixels at = block_pixels(a);
+  const DiffView& vw = a.views[at.view];
   // the vertices' gradients, which only k_diff_scatter adds to, start at zero
-  const unsigned block = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  for (size_t i = (size_t)block * kThreads + threadIdx.x; i < 4 * (size_t)a.nv;
-       i += (size_t)gridDim.x * gridDim.y * gridDim.z * kThreads) {
+  for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < 4 * (size_t)a.nv; i += (size_t)gridDim.x * kThreads) {
     a.g_pos[i] = 0.0f;
     if (i < 3 * (size_t)a.nv) a.g_vcol[i] = 0.0f;
   }
-  const int px = block_x();
-  size_t gp = (size_t)vw.pix_base + (size_t)block_y(a, 0) * (size_t)vw.W + (size_t)px;
+  const int px = at.x;
+  const size_t down = (size_t)at.rows * (size_t)vw.W;
+  size_t gp = (size_t)vw.pix_base + (size_t)at.y * (size_t)vw.W + (size_t)px;
   // the face ids first, a step ahead: most pixels of a view are background, and
   // their records (four times the bytes) are not read
-  uint32_t next = px < vw.W && block_y(a, 0) < vw.H ? a.ids[gp] : kNoFace;
-  for (int k8 = 0; k8 < a.rows8; ++k8, gp += 8 * (size_t)vw.W) {
-    const int py = block_y(a, k8);
+  uint32_t next = px < vw.W && at.y < vw.H ? a.ids[gp] : kNoFace;
+  for (int step = 0; step < a.blocks_down; ++step, gp += down) {
+    const int py = at.y + step * at.rows;
     bool on = next != kNoFace;
-    next = k8 + 1 < a.rows8 && px < vw.W && py + 8 < vw.H ? a.ids[gp + 8 * (size_t)vw.W] : kNoFace;
+    next = step + 1 < a.blocks_down && px < vw.W && py + at.rows < vw.H ? a.ids[gp + down] : kNoFace;
     if (!__any_sync(0xffffffffu, on)) continue;
     DiffRecord rec{kNoFace, kNoFace, 0.0f, 0.0f};
     if (on) {
@@ -568,7 +592,7 @@ __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
     if (rec.face != kNoFace) {
       const Word8 face = ldg8(a.faces + 4 * (size_t)f);
       FaceGeom g;
-      face_geom(a, blockIdx.z, face, px, py, g);
+      face_geom(a, at.view, face, px, py, g);
       Shade s;
       const int ni[3] = {(int)face.x[3], (int)face.x[4], (int)face.x[5]};
       shade(a, g, rec.l0, rec.l1, rec.texel, ni, s);
@@ -711,12 +735,12 @@ __global__ void __launch_bounds__(kThreads) k_diff_scatter(const DiffArgs a) {
     for (int j = 0; j < 3; ++j) gl[j] += __shfl_xor_sync(0xffffffffu, gl[j], o);
   }
   if ((threadIdx.x & 31) == 0) {
-    double* p = a.partials + 4 * diff_slot(blockIdx.x);
+    double* p = a.partials + 4 * diff_slot();
 #pragma unroll
     for (int j = 0; j < 3; ++j)
       if (gl[j] != 0.0) atomicAdd(p + 1 + j, gl[j]);
   }
-  sum_slots<3>(a, gridDim.x, 1, a.g_light);
+  sum_slots<3>(a, 1, a.g_light);
 }
 
 }  // namespace
@@ -758,22 +782,16 @@ int launch_diff_faces(const int* vidx, const int* nidx, const float* uv, int nf,
   return (int)cudaGetLastError();
 }
 
-// Grid of k_diff_shade and k_diff_grad.
-static dim3 pixel_grid(const DiffArgs& a) {
-  return dim3((unsigned)(a.max_w + 31) / 32u, (unsigned)(a.max_h + 8 * a.rows8 - 1) / (unsigned)(8 * a.rows8),
-              (unsigned)a.num_views);
-}
-
 int launch_diff_forward(const DiffArgs& a, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
-  const int sides = (std::max(a.max_w, a.max_h) + kThreads - 1) / kThreads;
+  const int sides = (a.max_side + kThreads - 1) / kThreads;
   k_diff_prepare<<<dim3((unsigned)(a.vert_blocks + a.norm_blocks + sides), (unsigned)a.num_views), kThreads, 0, s>>>(a);
-  launch_after(k_diff_shade, pixel_grid(a), kThreads, s, a);
+  launch_after(k_diff_shade, dim3(a.blocks), kThreads, s, a);
   return (int)cudaGetLastError();
 }
 
 int launch_diff_backward(const DiffArgs& a, void* stream) {
-  k_diff_grad<<<pixel_grid(a), kThreads, 0, (cudaStream_t)stream>>>(a);
+  k_diff_grad<<<a.blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
   launch_after(k_diff_scatter, dim3((unsigned)((a.nf + kThreads - 1) / kThreads)), kThreads, (cudaStream_t)stream, a);
   return (int)cudaGetLastError();
 }

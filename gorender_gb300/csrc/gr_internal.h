@@ -367,7 +367,15 @@ struct DiffView {
   uint32_t pix_base;                // first pixel of this view in the per-pixel buffers
   uint32_t face_base;               // first global face index of this view's item
   uint32_t col_base, row_base;      // first entry of this view in col_tab / row_tab
+  uint32_t block_base;              // first CTA of this view in k_diff_shade / k_diff_grad
+  int blocks_x;                     // ... and how many lie side by side
 };
+
+constexpr int kDiffThreads = 256;    // a CTA of the differentiable kernels
+// The pixels that a CTA of k_diff_shade / k_diff_grad (eight warps of 8 x 4) takes at
+// a time: 32 x 8, or in views of at most 16 and 8 columns 16 x 16 and 8 x 32, so that
+// narrow views leave no warp without pixels.
+__host__ __device__ inline int diff_block_wide(int W) { return W > 16 ? 32 : W > 8 ? 16 : 8; }
 
 // Per-pixel forward record: the visible face (or kNoFace), the texel it
 // sampled (or kNoFace without a texture) and two perspective-correct
@@ -381,8 +389,10 @@ struct DiffRecord {
 struct DiffArgs {
   const DiffView* views;
   int num_views;
-  int max_w, max_h;                 // the views' largest width and height
-  int rows8;                        // blocks of 8 rows a CTA of k_diff_shade / k_diff_grad takes (diff_rows8)
+  int max_side;                     // the views' largest width or height
+  int blocks_down;                  // blocks that a CTA of k_diff_shade / k_diff_grad takes, one below the other
+  uint32_t blocks;                  // CTAs over all views
+  uint32_t view_blocks;             // CTAs of every view where all have as many, otherwise 0
   int vert_blocks, norm_blocks;     // k_diff_prepare's blocks for vertices and normals
   int nv, nf, nn;
   const float* pos;                 // nv x 4 (parameter)
