@@ -207,6 +207,31 @@ __device__ __forceinline__ FF ff_mul(FF a, FF b) {  // the product of the his is
   e = __fadd_rn(e, __fadd_rn(__fmul_rn(a.hi, b.lo), __fmul_rn(a.lo, b.hi)));
   return fast_two_sum(p, e);
 }
+// A sum of floats as three: the additions' errors go to the next part, so it holds
+// some 70 bits (a double's sum rounds at each addition to 53), on the float32 pipes.
+struct Sum3 {
+  float hi = 0.0f, mid = 0.0f, lo = 0.0f;
+  __device__ __forceinline__ void add(float x) {
+    const FF t = two_sum(hi, x), u = two_sum(mid, t.lo);
+    hi = t.hi;
+    mid = u.hi;
+    lo = __fadd_rn(lo, u.lo);
+  }
+  __device__ __forceinline__ void add_lanes() {  // over the warp
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const FF t = two_sum(hi, __shfl_xor_sync(0xffffffffu, hi, o)), u = two_sum(mid, __shfl_xor_sync(0xffffffffu, mid, o)),
+               v = two_sum(u.hi, t.lo);
+      lo = __fadd_rn(__fadd_rn(lo, __shfl_xor_sync(0xffffffffu, lo, o)), __fadd_rn(u.lo, v.lo));
+      hi = t.hi;
+      mid = v.hi;
+    }
+  }
+  __device__ __forceinline__ double value() const {  // infinities and NaN stand in hi alone
+    return isfinite(hi) ? (double)hi + ((double)mid + (double)lo) : (double)hi;
+  }
+};
+
 __device__ __forceinline__ FF ff_mul_f(FF a, float b) {
   const float p = __fmul_rn(a.hi, b);
   float e = __fmaf_rn(a.hi, b, -p);
@@ -483,11 +508,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_diff_shade(const DiffArgs a) {
   const Pixels at = block_pixels(a);
   const DiffView& vw = a.views[at.view];
   const int px = at.x;
-  // the pixels' losses, summed as hi + lo (error-free sums; the warp's sum goes
-  // to FP64), since FP64 additions, one a pixel or five for each warp's tree,
-  // held this kernel at the FP64 pipe's rate.  Losses near float32's end, and
-  // infinities and NaN, are summed apart, scaled by 2^-80.
-  float hi = 0.0f, lo = 0.0f, bhi = 0.0f, blo = 0.0f;
+  // the pixels' losses, summed as three floats, no less exact than in FP64 (the warp's
+  // sum goes to FP64), since FP64 additions, one a pixel or five for each warp's
+  // tree, held this kernel at the FP64 pipe's rate.  (Two floats, which round to
+  // about 46 bits, are 1 % of the 64-view step faster.)  Losses near float32's
+  // end, and infinities and NaN, are summed apart, scaled by 2^-80.
+  Sum3 sum, big;
   for (int k = 0; k < a.blocks_down; ++k) {
     const int py = at.y + k * at.rows;
     if (px >= vw.W || py >= vw.H) break;
@@ -525,34 +551,17 @@ __global__ void __launch_bounds__(kThreads, 4) k_diff_shade(const DiffArgs a) {
     if (a.image) reinterpret_cast<float4*>(a.image)[gp] = out;
     const float dx = out.x - tg.x, dy = out.y - tg.y, dz = out.z - tg.z, dw = out.w - tg.w;
     const float lp = dx * dx + dy * dy + dz * dz + dw * dw;
-    if (lp < 1e36f) {
-      const FF t = two_sum(hi, lp);
-      hi = t.hi;
-      lo = __fadd_rn(lo, t.lo);
-    } else {
-      const FF t = two_sum(bhi, lp * 0x1p-80f);
-      bhi = t.hi;
-      blo = __fadd_rn(blo, t.lo);
-    }
+    if (lp < 1e36f) sum.add(lp);
+    else big.add(lp * 0x1p-80f);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const FF t = two_sum(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    lo = __fadd_rn(__fadd_rn(lo, __shfl_xor_sync(0xffffffffu, lo, o)), t.lo);
-    hi = t.hi;
-  }
-  double sum = (double)hi + (double)lo;
-  if (__any_sync(0xffffffffu, bhi != 0.0f)) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const FF t = two_sum(bhi, __shfl_xor_sync(0xffffffffu, bhi, o));
-      blo = __fadd_rn(__fadd_rn(blo, __shfl_xor_sync(0xffffffffu, blo, o)), t.lo);
-      bhi = t.hi;
-    }
-    sum += (isfinite(bhi) ? (double)bhi + (double)blo : (double)bhi) * 0x1p80;
+  sum.add_lanes();
+  double loss = sum.value();
+  if (__any_sync(0xffffffffu, big.hi != 0.0f)) {
+    big.add_lanes();
+    loss += big.value() * 0x1p80;
   }
   // one atomic into the warp's slot, so that warps never wait for each other
-  if ((threadIdx.x & 31) == 0 && sum != 0.0) atomicAdd(a.partials + 4 * diff_slot(), sum);
+  if ((threadIdx.x & 31) == 0 && loss != 0.0) atomicAdd(a.partials + 4 * diff_slot(), loss);
   sum_slots<1>(a, 0, a.loss);
 }
 

@@ -1,6 +1,8 @@
 """The per-pixel kernels of the differentiable step over views of uneven shapes:
 their CTAs stand in one list over all views, 32 x 8, 16 x 16 or 8 x 32 pixels a
 block by the view's width, one or eight blocks a CTA by the number of pixels."""
+import math
+
 import numpy as np
 import pytest
 
@@ -58,3 +60,34 @@ def test_uneven_shapes(large):
 def test_even_and_uneven_numbers_of_blocks(sizes):
     """Views of as many blocks each, in equal and in different shapes, and others."""
     edges._compare(*edges._case([(w * 3, h * 5) if w > 16 else (w, h * 9) for w, h in sizes], 4, 0, seed=11))
+
+
+@pytest.mark.parametrize("size", [(131, 97), (1531, 1429)])
+def test_loss_is_summed_in_64_bits(size):
+    """Losses in the pixels of one warp only (8 x 4, or eight such blocks one below
+    the other), one large among small ones, whose sum a pair of float32 rounds to
+    about 46 bits.  Nothing but zeros is added to the warp's own value, which rounds
+    three times."""
+    mesh, views, world, params, _ = edges._case([size], 3, 0, seed=13)
+    w, h = size
+    rows = [y for y in range(0, 64 if w * h >= 1 << 21 else 8) if y % 8 < 4]
+    at = np.array([y * w + x for y in rows for x in range(8)])
+    rng = np.random.default_rng(14)
+    ctx = gr.Context(0)
+    try:
+        d = R.Diff(ctx, ctx.mesh(mesh), world, views, tex_size=(0, 0))
+        pos, vcol = edges._dev(params["pos"]), edges._dev(params["vcol"])
+        zero = torch.zeros((w * h, 4), device="cuda")
+        image = torch.empty_like(zero)
+        forward = lambda t, i: d.forward(pos.data_ptr(), vcol.data_ptr(), None, params["light"], t.data_ptr(), i.data_ptr())
+        forward(zero, image)
+        for _ in range(40):
+            target = image.cpu().numpy().copy()
+            add = np.where(rng.random(len(at)) < 1 / 16, 1.0, 1.5e-4 * (0.5 + rng.random(len(at))))
+            target[at, 0] += add.astype(np.float32)
+            loss = forward(edges._dev(target), torch.empty_like(zero))
+            e = (image.cpu().numpy() - target)[at, 0]
+            want = math.fsum((e * e).astype(np.float64).tolist())
+            assert want > 0 and abs(loss - want) <= 3 * 2.0 ** -53 * want
+    finally:
+        ctx.close()
