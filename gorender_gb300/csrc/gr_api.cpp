@@ -52,6 +52,7 @@ struct MeshRec {
   int nv = 0, nn = 0, nf = 0;
   bool has_nidx = false, nidx_ok = false;
   float bbox[32];
+  bool plain_box = false;  // no NaN, nor numbers that overflow in a transform
   float *pos = nullptr, *vnrm = nullptr, *fnrm = nullptr, *uv = nullptr, *vcol = nullptr;
   int *vidx = nullptr, *nidx = nullptr, *tex = nullptr;
 };
@@ -268,10 +269,8 @@ int32_t ensure_tables(gr_context* c, int nviews, int nitems) {
   return GR_OK;
 }
 
-// Sizes the per-frame buffers for `faces` submitted faces and `tiles` tiles;
-// `unclipped`: some view does not clip, so that any face may lie beyond the
-// narrow bound and go to k_clip.
-int32_t ensure_frame_buffers(gr_context* c, uint64_t faces, uint32_t tiles, bool unclipped) {
+// Sizes the per-frame buffers for `faces` submitted faces and `tiles` tiles.
+int32_t ensure_frame_buffers(gr_context* c, uint64_t faces, uint32_t tiles) {
   bool synced = false;
   auto sync = [&]() -> int32_t {
     if (!synced) {
@@ -325,7 +324,7 @@ int32_t ensure_frame_buffers(gr_context* c, uint64_t faces, uint32_t tiles, bool
     c->tiles_cap = nt;
     c->bin_cap = nc;
   }
-  uint64_t want_clip = std::max<uint64_t>(c->want_clip_cap, (unclipped ? faces : faces / 16) + 1024);
+  uint64_t want_clip = std::max<uint64_t>(c->want_clip_cap, faces / 16 + 1024);
   if (want_clip > c->clip_cap) {
     if ((st = sync())) return st;
     dev_free(c->clip);
@@ -531,6 +530,9 @@ int32_t prepare(gr_context* c, const ViewIn* views, int nviews, const gr_draw_it
   uint64_t vert_total = 0;
   int vert_blocks = 0;
   int live = 0;
+  // Faces lie beyond the narrow bound in views that do not clip, and in boxes taken to be
+  // inside the frustum that are not (NaN, whose comparisons all fail).
+  bool far_setup = !(flags_all & GR_FRUSTUM_CLIPPING);
   uint64_t all_faces = 0;
   for (int i = 0; i < n; ++i) {
     const int m = items[i].mesh;
@@ -557,6 +559,7 @@ int32_t prepare(gr_context* c, const ViewIn* views, int nviews, const gr_draw_it
     std::memcpy(d.world, items[i].world, sizeof(d.world));
     std::memcpy(d.bbox, mr.bbox, sizeof(d.bbox));
     d.vis = box_visibility(d.mvp, d.bbox);
+    far_setup = far_setup || (d.vis == 2 && !mr.plain_box);
     d.pos = mr.pos; d.vnrm = mr.vnrm; d.fnrm = mr.fnrm; d.vidx = mr.vidx; d.nidx = mr.nidx;
     d.uv = mr.uv; d.tex = mr.tex; d.vcol = mr.vcol;
     d.nv = mr.nv; d.nn = mr.nn; d.nf = mr.nf;
@@ -578,7 +581,7 @@ int32_t prepare(gr_context* c, const ViewIn* views, int nviews, const gr_draw_it
     }
   }
   if (faces >= (1ull << 28)) return fail(GR_ERR_UNSUPPORTED, "more than 2^28 faces in one frame");
-  if ((st = ensure_frame_buffers(c, faces, total_tiles, !(flags_all & GR_FRUSTUM_CLIPPING)))) return st;
+  if ((st = ensure_frame_buffers(c, faces, total_tiles))) return st;
   if (flags_any & (GR_SHOW_EDGES | GR_SHOW_VERTICES)) {
     const uint64_t want_ovl = std::max<uint64_t>(c->want_ovl_cap, std::min<uint64_t>(faces + 1024, 1u << 30));
     if (want_ovl > c->ovl_cap) {
@@ -668,7 +671,8 @@ int32_t prepare(gr_context* c, const ViewIn* views, int nviews, const gr_draw_it
   a.clip_cap = c->clip_cap;
   a.kept = c->kept;
   a.kept_cap = c->kept_cap;
-  a.setup_blocks = (int)std::min<uint64_t>(setup_blocks_max(project_g), (faces + kProjectThreads - 1) / kProjectThreads);
+  a.far_setup = far_setup;
+  a.setup_blocks = (int)std::min<uint64_t>(setup_blocks_max(project_g, far_setup), (faces + kProjectThreads - 1) / kProjectThreads);
   a.vlight = c->vlight;
   a.light_blocks = light_blocks;
   a.vclip = c->vclip;
@@ -1022,6 +1026,7 @@ int32_t gr_mesh_create(gr_context* c, const gr_mesh_desc* d, int32_t* mesh_out) 
     for (long i = 0; i < 3L * nf && m.nidx_ok; ++i)
       if (d->normal_indices[i] < 0 || d->normal_indices[i] >= nn) m.nidx_ok = false;
   bounding_box(d->positions, nv, m.bbox);
+  m.plain_box = std::all_of(m.bbox, m.bbox + 32, [](float x) { return std::fabs(x) < 1e18f; });
   std::vector<float> fn;
   const float* fnp = d->face_normals;
   if (!fnp && nf > 0) {

@@ -56,10 +56,15 @@ constexpr int kSmallBox = 64;                 // larger tile-clipped boxes add h
 // them) below 1 M faces; 4 (at most 64 registers) from 1 M faces on, where more
 // warps hide more of the gathers (256-view batch 1101 us with 3 of 80 registers,
 // 1075 with 4; 5.0 M-face frame 275 and 270; a 200k-face frame 93.7 with 2, 97.1
-// with 3)
-__host__ __device__ constexpr int setup_ctas_per_sm(int project_g) { return project_g >= 2 ? 4 : 2; }
+// with 3).  Frames with faces beyond the narrow bound (FrameArgs::far_setup) need 80
+// registers for their set-up: 3 instead of 4.
+__host__ __device__ constexpr int setup_ctas_per_sm(int project_g, bool far) {
+  return project_g >= 2 ? (far ? 3 : 4) : 2;
+}
 // k_setup grid (grid-stride over the kept faces)
-__host__ __device__ constexpr int setup_blocks_max(int project_g) { return setup_ctas_per_sm(project_g) * 152; }
+__host__ __device__ constexpr int setup_blocks_max(int project_g, bool far) {
+  return setup_ctas_per_sm(project_g, far) * 152;
+}
 constexpr int kClipBlocks = 2 * 152;          // k_clip grid (grid-stride over the queue)
 constexpr int kBigBlocks = 3 * 152;           // k_bin_big / k_overlay grid (grid-stride over the queue)
 
@@ -311,6 +316,9 @@ struct FrameArgs {
   uint2* kept;                      // (item, face) of the faces k_cull kept whole; k_setup writes
                                     // the record of entry k as record k
   uint32_t kept_cap;                // >= the frame's faces: never overflows
+  int far_setup;                    // nonzero: k_setup takes faces beyond the narrow bound (frames with a view that
+                                    // does not clip, where any face may lie there); otherwise, where
+                                    // hardly any can, they go to k_clip
   int keep_uncovered;               // nonzero: faces that cover no pixel are kept and binned too (gr_draw_noalloc)
   int setup_blocks;                 // k_setup grid
   float* vlight;                    // per-normal Gouraud intensities (k_light)

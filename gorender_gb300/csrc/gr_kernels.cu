@@ -198,20 +198,12 @@ __device__ __forceinline__ float2 screen_of(V4 p, const float* S) {
                      fa(fa(fa(fm(S[4], dx), fm(S[5], dy)), fm(S[6], dz)), fm(S[7], dw)));
 }
 
-// Screen vertex from precomputed screen coordinates and the corner's attributes.
-__device__ __forceinline__ SV sv_of(float2 scr, float W, const PV& q) {
-  SV s;
-  s.sx = scr.x;
-  s.sy = scr.y;
-  s.X = go_int(s.sx);
-  s.Y = go_int(s.sy);
+// Screen vertex, as far as setup_tri needs it, from precomputed screen coordinates.
+__device__ __forceinline__ SV corner_of(float2 scr, float W) {
+  SV s{};
+  s.X = go_int(scr.x);
+  s.Y = go_int(scr.y);
   s.W = W;
-  s.u = q.u;
-  s.v = q.v;
-  s.in = q.in;
-  s.r = q.r;
-  s.g = q.g;
-  s.b = q.b;
   return s;
 }
 
@@ -605,13 +597,23 @@ __device__ __forceinline__ int narrow_sum(const Corners& c) {
          ((keeps_edge(a01, b01) ? 0 : 1) + (keeps_edge(a12, b12) ? 0 : 1) + (keeps_edge(a20, b20) ? 0 : 1));
 }
 
+// Whether all corners lie within the narrow bound, from their least and largest
+// coordinates (|int(x)| < 2^14 where |x| < 2^14) and, where none is a NaN, from themselves.
+__device__ __forceinline__ bool narrow_bound(float minX, float maxX, float minY, float maxY) {
+  const float lim = (float)kNarrowLimit;
+  return minX > -lim && maxX < lim && minY > -lim && maxY < lim;
+}
+__device__ __forceinline__ bool narrow_bound(float2 q0, float2 q1, float2 q2) {
+  return narrow_bound(fminf(fminf(q0.x, q1.x), q2.x), fmaxf(fmaxf(q0.x, q1.x), q2.x), fminf(fminf(q0.y, q1.y), q2.y),
+                      fmaxf(fmaxf(q0.y, q1.y), q2.y));
+}
+
 // identifyTriangleTiles with the single screen tile on screen corners
 // (bin_test), and whether all corners lie within the narrow bound.
 __device__ __forceinline__ bool bin_test_screen(float2 q0, float2 q1, float2 q2, float Wf, float Hf, bool& narrow) {
   const float minX = fminf(fminf(q0.x, q1.x), q2.x), maxX = fmaxf(fmaxf(q0.x, q1.x), q2.x);
   const float minY = fminf(fminf(q0.y, q1.y), q2.y), maxY = fmaxf(fmaxf(q0.y, q1.y), q2.y);
-  const float lim = (float)kNarrowLimit;  // |int(x)| < 2^14 where |x| < 2^14
-  narrow = minX > -lim && maxX < lim && minY > -lim && maxY < lim;
+  narrow = narrow_bound(minX, maxX, minY, maxY);
   if (isnan(q0.x) || isnan(q1.x) || isnan(q2.x) || isnan(q0.y) || isnan(q1.y) || isnan(q2.y)) return false;
   return maxX >= 0.0f && minX <= Wf && maxY >= 0.0f && minY <= Hf;
 }
@@ -917,21 +919,24 @@ __global__ void __launch_bounds__(kProjectThreads, 5) k_cull(const FrameArgs a) 
     }
     // The faces kept whole: the bin test (TPF), and out go those that cover no
     // pixel.  Views with overlays keep them for their marks, and frames of fixed
-    // buffers because their bins' limit is stated in them.  Corners beyond
-    // the narrow bound (hardly ever with clipping on) leave the face to k_clip,
-    // which counts and sets it up without clipping it.
+    // buffers because their bins' limit is stated in them.  Faces with corners
+    // beyond the narrow bound are k_setup's in frames that may hold many of them
+    // (a warp each in k_clip, a million took 950-1520 us where the lanes of
+    // k_setup take 30 to 45); with clipping on, where they hardly ever occur
+    // and k_setup goes without the code for them, k_clip counts them and sets them
+    // up without clipping them.
     bool keep = draw && !general, far = false;
     if (keep) {
       const float2 p0 = make_float2(q0.x, q0.y), p1 = make_float2(q1.x, q1.y), p2 = make_float2(q2.x, q2.y);
       bool narrow;
       const bool binned = bin_test_screen(p0, p1, p2, Wf, Hf, narrow);
-      far = binned && !narrow;
+      far = binned && !narrow && !a.far_setup;
       general = far;
-      keep = binned && narrow;
+      keep = binned && !far;
       ntpf += keep;
       if (keep && !(fl & 0xC0u) && !a.keep_uncovered) {
         keep = (fl & 0x02u) != 0;  // ShowFaces off: counted, not rasterised (renderer.go:180)
-        if (keep) {
+        if (keep && narrow) {
           const Corners c = narrow_corners(p0, p1, p2);
           keep = narrow_covers(c, narrow_box(c, vw.W, vw.H));
         }
@@ -989,11 +994,11 @@ __global__ void __launch_bounds__(kProjectThreads, 5) k_cull(const FrameArgs a) 
 // Bound by the latency of its gathers and atomics, so by resident warps.  CTAS
 // of them an SM (setup_ctas_per_sm): 2 with up to 104 registers (2 x 256 x 104 =
 // 53,248: a 96-register k_clip CTA still fits beside them, as k_clip runs beside
-// k_setup), 4 with up to 64.  All corners lie within the narrow bound here and
-// TPF is counted before, which leaves 32-bit arithmetic and 63 registers where
-// the general set-up took 80 and spilled.
-template <int CTAS>
-__global__ void __maxnreg__(CTAS == 4 ? 64 : 104) k_setup(const FrameArgs a) {
+// k_setup), 4 with up to 64.  Without FAR all corners lie within the narrow bound and
+// TPF is counted before, which leaves 32-bit arithmetic and 63 registers.  FAR: faces
+// beyond it are set up too, in 64 bits (at most 80 registers with 3 CTAs).
+template <int CTAS, bool FAR>
+__global__ void __maxnreg__(CTAS == 4 ? 64 : CTAS == 3 ? 80 : 104) k_setup(const FrameArgs a) {
   griddep_wait();
   const uint32_t nkept = min(*(volatile uint32_t*)&a.work->nkept, a.kept_cap);
   const unsigned lane = lane_id();
@@ -1021,8 +1026,21 @@ __global__ void __maxnreg__(CTAS == 4 ? 64 : 104) k_setup(const FrameArgs a) {
       PV p0, p1, p2;
       int tex = -1;
       if (!(fl & kViewFaceIds)) face_attributes(a, it, f, i0, i1, i2, it.world, p0, p1, p2, tex, true);
-      if (fl & 0x02u) {  // ShowFaces
-        const Corners c = narrow_corners(make_float2(q0.x, q0.y), make_float2(q1.x, q1.y), make_float2(q2.x, q2.y));
+      const float2 c0 = make_float2(q0.x, q0.y), c1 = make_float2(q1.x, q1.y), c2 = make_float2(q2.x, q2.y);
+      if (FAR && !narrow_bound(c0, c1, c2)) {
+        const SV s0 = corner_of(c0, q0.z), s1 = corner_of(c1, q1.z), s2 = corner_of(c2, q2.z);
+        Setup s;
+        emit = (fl & 0x02u) && setup_tri(s0, s1, s2, W, H, s);
+        if (emit && r >= a.rec_cap) {
+          atomicMax(&a.work->rec_need, r + 1u);
+          emit = false;
+        }
+        if (emit) {
+          box = Box{s.r.bx0, s.r.bx1, s.r.by0, s.r.by1};
+          write_raster(a, r, s, s0, s1, s2, okey);
+        }
+      } else if (fl & 0x02u) {  // ShowFaces
+        const Corners c = narrow_corners(c0, c1, c2);
         box = narrow_box(c, W, H);
         emit = box.x0 <= box.x1 && box.y0 <= box.y1;
         const int sum = narrow_sum(c);
@@ -1037,11 +1055,11 @@ __global__ void __maxnreg__(CTAS == 4 ? 64 : 104) k_setup(const FrameArgs a) {
                              (int)((uint32_t)(uint16_t)c.x1 | (uint32_t)c.y1 << 16),
                              (int)((uint32_t)(uint16_t)c.x2 | (uint32_t)c.y2 << 16), (int)okey);
           reinterpret_cast<float4*>(dst)[1] = make_float4(q0.z, q1.z, q2.z, __int2float_rn(sum));
-          if (!(fl & kViewFaceIds)) {  // face ids are drawn from the keys alone
-            write_shade(a, r, p0.in, p1.in, p2.in, tex == -2 ? -3 : tex, p0.u, p0.v, q0.z, p1.u, p1.v, q1.z, p2.u, p2.v, q2.z);
-            if (okey / (uint32_t)kKeysPerFace < a.face_cap) a.rec_of_face[okey / (uint32_t)kKeysPerFace] = r;
-          }
         }
+      }
+      if (emit && !(fl & kViewFaceIds)) {  // face ids are drawn from the keys alone
+        write_shade(a, r, p0.in, p1.in, p2.in, tex == -2 ? -3 : tex, p0.u, p0.v, q0.z, p1.u, p1.v, q1.z, p2.u, p2.v, q2.z);
+        if (okey / (uint32_t)kKeysPerFace < a.face_cap) a.rec_of_face[okey / (uint32_t)kKeysPerFace] = r;
       }
     }
 
@@ -2522,8 +2540,9 @@ int launch_frame(const FrameArgs& a, int big_blocks, void* stream, int* launches
     fork(1);  // k_clip needs only k_cull's queue: runs beside k_setup and k_bin_big
     k_clip<<<kClipBlocks, 128, 0, s2>>>(a);
     ++n;
-    if (setup_ctas_per_sm(a.project_g) == 4) launch_after(k_setup<4>, a.setup_blocks, kProjectThreads, s, a);
-    else launch_after(k_setup<2>, a.setup_blocks, kProjectThreads, s, a);
+    const bool wide = setup_ctas_per_sm(a.project_g, a.far_setup) > 2;
+    if (a.far_setup) launch_after(wide ? k_setup<3, true> : k_setup<2, true>, a.setup_blocks, kProjectThreads, s, a);
+    else launch_after(wide ? k_setup<4, false> : k_setup<2, false>, a.setup_blocks, kProjectThreads, s, a);
     ++n;
     if (events) cudaEventRecord((cudaEvent_t)events[1], s);
     if (events) k_bin_big<<<big_blocks, 256, 0, s>>>(a);  // timed stages: plain launches

@@ -311,7 +311,8 @@ extern "C" int32_t gr_draw_noalloc(int32_t device, const gr_noalloc_object* obje
   a.kept = (uint2*)(base + kLayout.kept);
   a.kept_cap = kMaxFaces;
   a.keep_uncovered = 1;  // the bins hold every binned triangle, as the limits say
-  a.setup_blocks = (int)std::min<long>(setup_blocks_max(a.project_g), (faces + kProjectThreads - 1) / kProjectThreads);
+  a.far_setup = !(p->flags & GR_FRUSTUM_CLIPPING);
+  a.setup_blocks = (int)std::min<long>(setup_blocks_max(a.project_g, a.far_setup), (faces + kProjectThreads - 1) / kProjectThreads);
   a.vlight = (float*)(base + kLayout.vlight);
   a.vclip = (float4*)(base + kLayout.vclip);
   a.vscr = (float4*)(base + kLayout.vscr);
