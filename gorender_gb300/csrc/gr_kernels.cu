@@ -1430,19 +1430,20 @@ struct RasterShape {
 // Exact depth test of one covered pixel: zRec in the reference's order,
 // then a 64-bit max of (ordered zRec, draw-order key) into the tile's keys.
 //
-// Early out: at a covered pixel the barycentrics are e/sum of adjusted edge
-// values that are all negative, so they lie in [0, 1] (to rounding) and
+// Early out (depth_beaten): at a covered pixel the barycentrics are e/sum of
+// adjusted edge values that are all negative, so they lie in [0, 1] (to rounding) and
 // zRec = -(al/w0 + be/w1 + ga/w2) <= (1 / min|w|) * (1 + ~1e-6) when every w
 // is negative (in front of the camera).  A candidate whose bound stays below
 // the depth the pixel already holds, with a 1e-5 margin for the roundings,
 // loses strictly (ties, where draw order decides, are never skipped), so its
 // five divisions are not needed.
 // The depth test proper at pixel p with edge values e12, e20 (as floats).
-__device__ __forceinline__ void depth_at(unsigned long long* p, const TriRaster& t, float e12f, float e20f) {
+__device__ __forceinline__ void depth_at(unsigned long long* p, float e12f, float e20f, float sumf, float w0, float w1,
+                                         float w2, uint32_t okey) {
   float al, be, ga;
-  const float z = zrec_of(e12f, e20f, t.sumf, t.w0, t.w1, t.w2, al, be, ga);
+  const float z = zrec_of(e12f, e20f, sumf, w0, w1, w2, al, be, ga);
   if (!(z >= -1.0f)) return;  // rasterizer.go:156 against the cleared Z of -1
-  const unsigned long long k = depth_key(z, t.key);
+  const unsigned long long k = depth_key(z, okey);
   if (k > *(volatile unsigned long long*)p) atomicMax(p, k);
 }
 
@@ -1454,27 +1455,14 @@ __device__ __forceinline__ bool depth_beaten(unsigned long long k, float wmin) {
   return __fmul_rn(__uint_as_float((uint32_t)(k >> 32) ^ 0x80000000u), wmin) > 1.00001f;
 }
 
-template <int TS>
-__device__ __forceinline__ void depth_candidate(unsigned long long* skey, const TriRaster& t, const TriWide* wide,
-                                                uint32_t r, int x, int y, int tx0, int ty0) {
-  unsigned long long* p = skey + (y - ty0) * RasterShape<TS>::kStride + (x - tx0);
-  const float wmin = fmaxf(fminf(fminf(-t.w0, -t.w1), -t.w2), 0.0f);
-  if (depth_beaten(*(volatile unsigned long long*)p, wmin)) return;
-  bool inside;
-  float e12f, e20f;
-  edges_at(t, wide, r, x, y, inside, e12f, e20f);
-  depth_at(p, t, e12f, e20f);
-}
-
-// Whether triangle t takes the raster's unit walk: a narrow triangle whose
-// W's magnitudes lie in [2^-60, 2^60], where div_by is exact.  Its sum and
-// edge values are whole numbers in [1, 2^32) by magnitude, so al and be lie in
-// [2^-32, 1] and ga is 0 or at least 2^-57 (a difference of values on a
-// 2^-57 grid): quotients by W stay above 2^-117 and residuals above 2^-104.
+// Whether narrow triangle t's W's have magnitudes in [2^-60, 2^61), where div_by is
+// exact.  Its sum and edge values are whole numbers in [1, 2^32) by magnitude, so
+// al and be lie in [2^-32, 1] and ga is 0 or at least 2^-57 (a difference of values
+// on a 2^-57 grid): quotients by W stay above 2^-118 and residuals above 2^-105.
 __device__ __forceinline__ bool narrow_fast(const TriRaster& t) {
   const uint32_t e0 = (__float_as_uint(t.w0) >> 23) & 0xFFu, e1 = (__float_as_uint(t.w1) >> 23) & 0xFFu,
                  e2 = (__float_as_uint(t.w2) >> 23) & 0xFFu;
-  return !(t.key & 0x80000000u) && e0 - 67u <= 120u && e1 - 67u <= 120u && e2 - 67u <= 120u;
+  return e0 - 67u <= 120u && e1 - 67u <= 120u && e2 - 67u <= 120u;
 }
 
 __device__ __forceinline__ int warp_incl_scan(int v) {
@@ -1485,18 +1473,6 @@ __device__ __forceinline__ int warp_incl_scan(int v) {
     if ((int)lane >= o) v += y;
   }
   return v;
-}
-
-// Coverage test of one pixel (rasterizer.go:147).
-__device__ __forceinline__ bool covers(const TriRaster& t, const TriWide* wide, uint32_t r, int x, int y) {
-  if (!(t.key & 0x80000000u)) {
-    return t.a01 * x + t.b01 * y + t.c01 < 0 && t.a12 * x + t.b12 * y + t.c12 < 0 &&
-           t.a20 * x + t.b20 * y + t.c20 < 0;
-  }
-  bool inside;
-  float e12f, e20f;
-  edges_at(t, wide, r, x, y, inside, e12f, e20f);
-  return inside;
 }
 
 // The raster cost per slice: the frame's own, less where it has fewer tiles
@@ -1534,9 +1510,11 @@ struct WarpTable {
   float4 d1[32];     // w1, 1 / w1, w2, 1 / w2
   int start[32];     // the slot's first unit (INT_MAX: no triangle)
   uint2 run[32];     // runs with covered pixels of the step: x | y << 8 | slot << 16, first pixel number
-  uint32_t wide[32]; // records of the other triangles
+  uint2 wide[32];    // the triangles with int64 edges: record, box in the tile (first x and y, last x and y, a byte
+                     // each)
   int units;         // the table's units
   int nwide;
+  bool general;      // some slot's W's are out of narrow_fast's range
 };
 
 template <int TS>
@@ -1547,15 +1525,20 @@ struct RasterSmem {
   uint32_t last;
 };
 
-// Depth test of a covered pixel: the exact zRec of the reference, then a max
-// of its key (depth_key, with a zRec of -0 made +0 by the subtraction; one
-// below -1 loses to the background key) into the tile's.  The first
-// compare-and-swap uses the key already read, so an uncontended pixel takes
-// one.
+// Depth test of a covered pixel: the exact zRec of the reference (GENERAL: for any
+// W's, by the general division), then a max of its key (depth_key, with a zRec
+// of -0 made +0 by the subtraction; one below -1 loses to the background key)
+// into the tile's.  The first compare-and-swap uses the key already read, so an
+// uncontended pixel takes one.
+template <bool GENERAL>
 __device__ __forceinline__ void depth_test(unsigned long long* p, const float4& d0, const float4& d1, float wmin,
                                            int e12, int e20, uint32_t okey) {
   unsigned long long c = *(volatile unsigned long long*)p;
   if (depth_beaten(c, wmin)) return;
+  if constexpr (GENERAL) {
+    depth_at(p, __int2float_rn(e12), __int2float_rn(e20), d0.x, d0.z, d1.x, d1.z, okey);
+    return;
+  }
   const float al = div_by(__int2float_rn(e12), d0.x, d0.y), be = div_by(__int2float_rn(e20), d0.x, d0.y);
   const float ga = fs(fs(1.0f, al), be);
   const float z = fs(0.0f, fa(fa(div_by(al, d0.z, d0.w), div_by(be, d1.x, d1.y)), div_by(ga, d1.z, d1.w)));
@@ -1589,9 +1572,14 @@ __device__ __forceinline__ void raster_stage(const FrameArgs& a, const DevView& 
     ly0 = max((int)t.by0, ty0); ly1 = min((int)t.by1, ty1);
   }
   const bool live = valid && lx1 >= lx0 && ly1 >= ly0;
-  bool fast = live && narrow_fast(t);
-  const unsigned wm = __ballot_sync(FULL_MASK, live && !fast);
-  if (live && !fast) tab.wide[__popc(wm & ((1u << lane) - 1u))] = r;
+  const bool wide = live && (t.key & 0x80000000u);
+  bool units_walk = live && !wide;
+  const bool fast = units_walk && narrow_fast(t);
+  const bool general = __any_sync(FULL_MASK, units_walk && !fast);
+  const unsigned wm = __ballot_sync(FULL_MASK, wide);
+  if (wide)
+    tab.wide[__popc(wm & ((1u << lane) - 1u))] =
+        make_uint2(r, (uint32_t)((lx0 - tx0) | (ly0 - ty0) << 8 | (lx1 - tx0) << 16 | (ly1 - ty0) << 24));
   const int bw = lx1 - lx0 + 1, bh = ly1 - ly0 + 1;
   if (tiny) {
     const bool here = fast && bw <= kTinyBox && bh <= kTinyBox;
@@ -1615,19 +1603,19 @@ __device__ __forceinline__ void raster_stage(const FrameArgs& a, const DevView& 
           while (cov) {
             const int k = __ffs((int)cov) - 1, x = k % kTinyBox, y = k / kTinyBox;
             cov &= cov - 1u;
-            depth_test(p + y * RasterShape<TS>::kStride + x, d0, d1, wmin, e12 + t.a12 * x + t.b12 * y,
-                       e20 + t.a20 * x + t.b20 * y, t.key);
+            depth_test<false>(p + y * RasterShape<TS>::kStride + x, d0, d1, wmin, e12 + t.a12 * x + t.b12 * y,
+                              e20 + t.a20 * x + t.b20 * y, t.key);
           }
         }
       }
-      fast = fast && !here;
+      units_walk = units_walk && !here;
     }
   }
-  const unsigned fm = __ballot_sync(FULL_MASK, fast);
-  const int units = fast ? bh * ((bw + kSeg - 1) >> kSegShift) : 0;
+  const unsigned fm = __ballot_sync(FULL_MASK, units_walk);
+  const int units = units_walk ? bh * ((bw + kSeg - 1) >> kSegShift) : 0;
   const int incl = warp_incl_scan(units);
   const unsigned slot = __popc(fm & ((1u << lane) - 1u));
-  if (fast) {
+  if (units_walk) {
     tab.e01[slot] = make_int4(t.a01, t.b01, t.c01 + t.a01 * tx0 + t.b01 * ty0,
                               (lx0 - tx0) | (ly0 - ty0) << 8 | bw << 16);
     tab.e12[slot] = make_int4(t.a12, t.b12, t.c12 + t.a12 * tx0 + t.b12 * ty0, (int)t.key);
@@ -1641,6 +1629,7 @@ __device__ __forceinline__ void raster_stage(const FrameArgs& a, const DevView& 
   if (lane == 31u) {
     tab.units = incl;
     tab.nwide = __popc(wm);
+    tab.general = general;
   }
 }
 
@@ -1651,7 +1640,7 @@ __device__ __forceinline__ void raster_stage(const FrameArgs& a, const DevView& 
 // scan) and depth-tested 32 at a time, so that the divisions run with every
 // lane busy; runs of nearly equal length are tested by their own lanes
 // instead, one pixel a turn.
-template <int TS>
+template <int TS, bool GENERAL>
 __device__ __forceinline__ void raster_units(const WarpTable& tab, uint2* runs, int total, int g0,
                                              unsigned long long* skey) {
   constexpr int kStride = RasterShape<TS>::kStride;
@@ -1688,7 +1677,7 @@ __device__ __forceinline__ void raster_units(const WarpTable& tab, uint2* runs, 
       int e12 = q1.x * x + q1.y * y + q1.z, e20 = q2.x * x + q2.y * y + q2.z;
       unsigned long long* p = skey + y * kStride + x;
       for (int k = 0; k < num; ++k, ++p) {
-        depth_test(p, d0, d1, __int_as_float(q2.w), e12, e20, (uint32_t)q1.w);
+        depth_test<GENERAL>(p, d0, d1, __int_as_float(q2.w), e12, e20, (uint32_t)q1.w);
         e12 += q1.x;
         e20 += q2.x;
       }
@@ -1708,27 +1697,85 @@ __device__ __forceinline__ void raster_units(const WarpTable& tab, uint2* runs, 
       const uint2 q = runs[before + __popc(starts & upto) - 1];
       const int px = (int)(q.x & 0xFFu) + h - (int)q.y, py = (int)((q.x >> 8) & 0xFFu), s = (int)(q.x >> 16);
       const int4 q1 = tab.e12[s], q2 = tab.e20[s];
-      depth_test(skey + py * kStride + px, tab.d0[s], tab.d1[s], __int_as_float(q2.w), q1.x * px + q1.y * py + q1.z,
-                 q2.x * px + q2.y * py + q2.z, (uint32_t)q1.w);
+      depth_test<GENERAL>(skey + py * kStride + px, tab.d0[s], tab.d1[s], __int_as_float(q2.w),
+                          q1.x * px + q1.y * py + q1.z, q2.x * px + q2.y * py + q2.z, (uint32_t)q1.w);
     }
   }
   __syncwarp();  // the runs are rewritten by the next step
 }
 
-// A triangle that the units do not take (int64 edges, or W's out of
-// narrow_fast's range): the CTA's warps share the 8 x 4 blocks of its box.
+// The batch's triangles with int64 edges: the CTA's warps take the 8 x 4 blocks of
+// all their boxes in turn, numbered from one triangle to the next, so that many
+// triangles of one block each keep all of them busy; a warp reads a triangle's
+// record only where it has a block of it.
 template <int TS>
-__device__ __forceinline__ void raster_wide(const FrameArgs& a, const DevView& vw, uint32_t r, int tx0, int ty0,
-                                            int tx1, int ty1, unsigned long long* skey) {
-  const unsigned lane = threadIdx.x & 31u;
-  const TriRaster t = unpack_tri(a, r, vw.W, vw.H);
-  const int bx0 = max((int)t.bx0, tx0), bx1 = min((int)t.bx1, tx1);
-  const int by0 = max((int)t.by0, ty0), by1 = min((int)t.by1, ty1);
-  const int nbx = (bx1 - bx0 + 8) >> 3, nblk = nbx * ((by1 - by0 + 4) >> 2);
-  for (int j = (int)(threadIdx.x >> 5); j < nblk; j += RasterShape<TS>::kWarps) {
-    const int x = bx0 + (j % nbx) * 8 + (int)(lane & 7u), y = by0 + (j / nbx) * 4 + (int)(lane >> 3);
-    if (x <= bx1 && y <= by1 && covers(t, a.wide, r, x, y)) depth_candidate<TS>(skey, t, a.wide, r, x, y, tx0, ty0);
+__device__ __forceinline__ void raster_wide(const TriPacked* rast, const TriWide* wide, RasterSmem<TS>& sm, int tx0,
+                                            int ty0) {
+  constexpr int kWarps = RasterShape<TS>::kWarps;
+  typedef unsigned long long u64;
+  const int lx = (int)(threadIdx.x & 7u), ly = (int)((threadIdx.x >> 3) & 3u), warp = (int)(threadIdx.x >> 5);
+  int base = 0;  // blocks of the triangles before this one
+  for (int w = 0; w < kWarps; ++w) {
+    const WarpTable& tab = sm.tab[w];
+    for (int k = 0; k < tab.nwide; ++k) {
+      const uint2 e = tab.wide[k];
+      const int x0 = (int)(e.y & 0xFFu), y0 = (int)((e.y >> 8) & 0xFFu), x1 = (int)((e.y >> 16) & 0xFFu),
+                y1 = (int)(e.y >> 24);
+      const int nbx = (x1 - x0 + 8) >> 3, nblk = nbx * ((y1 - y0 + 4) >> 2);
+      int j = (warp - base) & (kWarps - 1);
+      base += nblk;
+      if (j >= nblk) continue;
+      const TriPacked& t = rast[e.x];
+      const float4 ws = *reinterpret_cast<const float4*>(&t.w0);  // W's and the sum
+      const uint32_t okey = t.key & 0x7FFFFFFFu;
+      const float wmin = fmaxf(fminf(fminf(-ws.x, -ws.y), -ws.z), 0.0f);
+      const TriWide q = wide[e.x];
+      for (; j < nblk; j += kWarps) {
+        const int x = x0 + (j % nbx) * 8 + lx, y = y0 + (j / nbx) * 4 + ly;
+        if (x > x1 || y > y1) continue;
+        const u64 X = (u64)(tx0 + x), Y = (u64)(ty0 + y);
+        const long long e01 = (long long)((u64)q.a01 * X + (u64)q.b01 * Y + (u64)q.c01);
+        const long long e12 = (long long)((u64)q.a12 * X + (u64)q.b12 * Y + (u64)q.c12);
+        const long long e20 = (long long)((u64)q.a20 * X + (u64)q.b20 * Y + (u64)q.c20);
+        if ((e01 & e12 & e20) >= 0) continue;  // covered where all three are negative (rasterizer.go:147)
+        u64* p = sm.skey + y * RasterShape<TS>::kStride + x;
+        if (depth_beaten(*(volatile u64*)p, wmin)) continue;
+        depth_at(p, __ll2float_rn(e12), __ll2float_rn(e20), ws.w, ws.x, ws.y, ws.z, okey);
+      }
+    }
   }
+}
+
+// The batch's groups of 32 units, table by table, the CTA's warps in turn.
+template <int TS, bool GENERAL>
+__device__ __forceinline__ void raster_batch(RasterSmem<TS>& sm) {
+  constexpr int kWarps = RasterShape<TS>::kWarps;
+  const unsigned lane = lane_id();
+  const int warp = (int)(threadIdx.x >> 5);
+  // lane l < kWarps holds the number of groups up to table l
+  const int groups = warp_incl_scan(lane < (unsigned)kWarps ? (sm.tab[lane].units + 31) >> 5 : 0);
+  const int all = __shfl_sync(FULL_MASK, groups, kWarps - 1);
+  for (int g = warp; g < all; g += kWarps) {
+    const int seg = __popc(__ballot_sync(FULL_MASK, lane < (unsigned)kWarps && groups <= g));
+    const int prev = __shfl_sync(FULL_MASK, groups, (seg + 31) & 31);
+    raster_units<TS, GENERAL>(sm.tab[seg], sm.tab[warp].run, sm.tab[seg].units, (g - (seg ? prev : 0)) << 5, sm.skey);
+  }
+}
+
+// A batch with triangles beyond the usual: int64 edges, or W's out of narrow_fast's
+// range, which take the general divisions (and the batch's others with them).
+// 20,000 triangles of 9 pixels with W's of 2^-63 at 640 x 360: 79 us with those in
+// raster_wide, 35 here; an unclipped 199,712-triangle terrain with the camera
+// inside 2165 -> 2020.  Chosen once a batch: with a choice for each group of units
+// the 256-view batch took 1056 us instead of 1040, and with functions called
+// instead of inlined a 1280 x 720 terrain 95 instead of 89.
+template <int TS>
+__device__ __forceinline__ void raster_odd_batch(const TriPacked* rast, const TriWide* wide, RasterSmem<TS>& sm, int tx0,
+                                                 int ty0) {
+  const unsigned lane = lane_id();
+  if (__any_sync(FULL_MASK, lane < (unsigned)RasterShape<TS>::kWarps && sm.tab[lane].general)) raster_batch<TS, true>(sm);
+  else raster_batch<TS, false>(sm);
+  raster_wide<TS>(rast, wide, sm, tx0, ty0);
 }
 
 __device__ __forceinline__ TriShade load_shade(const FrameArgs& a, uint32_t r) {
@@ -1904,21 +1951,13 @@ __device__ __forceinline__ void raster_item(const FrameArgs& a, const uint32_t& 
       } else if (lane == 0) {
         sm.tab[warp].units = 0;
         sm.tab[warp].nwide = 0;
+        sm.tab[warp].general = false;
       }
       __syncthreads();
-      // the batch's groups of 32 units, table by table: lane l < kWarps holds
-      // the number of groups up to table l
-      const int groups = warp_incl_scan(lane < (unsigned)kWarps ? (sm.tab[lane].units + 31) >> 5 : 0);
-      const int all = __shfl_sync(FULL_MASK, groups, kWarps - 1);
-      for (int g = warp; g < all; g += kWarps) {
-        const int seg = __popc(__ballot_sync(FULL_MASK, lane < (unsigned)kWarps && groups <= g));
-        const int prev = __shfl_sync(FULL_MASK, groups, (seg + 31) & 31);
-        raster_units<TS>(sm.tab[seg], sm.tab[warp].run, sm.tab[seg].units, (g - (seg ? prev : 0)) << 5, skey);
-      }
-      if (__ballot_sync(FULL_MASK, lane < (unsigned)kWarps && sm.tab[lane].nwide != 0)) {
-        for (int w = 0; w < kWarps; ++w)
-          for (int k = 0; k < sm.tab[w].nwide; ++k) raster_wide<TS>(a, vw, sm.tab[w].wide[k], tx0, ty0, tx1, ty1, skey);
-      }
+      const unsigned odd =
+          __ballot_sync(FULL_MASK, lane < (unsigned)kWarps && (sm.tab[lane].nwide != 0 || sm.tab[lane].general));
+      if (!odd) raster_batch<TS, false>(sm);
+      else raster_odd_batch<TS>(a.rast, a.wide, sm, tx0, ty0);
       __syncthreads();
     }
 
