@@ -1045,6 +1045,7 @@ __global__ void __maxnreg__(CTAS == 4 ? 64 : CTAS == 3 ? 80 : 104) k_setup(const
         emit = box.x0 <= box.x1 && box.y0 <= box.y1;
         const int sum = narrow_sum(c);
         emit = emit && sum < 0;  // k_cull has looked, except in views with marks and fixed buffers
+        if (fl & 0xC0u) emit = emit && narrow_covers(c, box);
         if (emit && r >= a.rec_cap) {
           atomicMax(&a.work->rec_need, r + 1u);
           emit = false;
@@ -2101,8 +2102,14 @@ __global__ void __launch_bounds__(256) k_overlay(const FrameArgs a) {
   griddep_wait();
   const uint32_t nkept = min(*(volatile uint32_t*)&a.work->nkept, a.kept_cap);
   const uint32_t n = nkept + min(*(volatile uint32_t*)&a.work->novl, a.ovl_cap);
-  const int part = (int)(threadIdx.x >> 5);  // a warp's lanes do the same part of 32 triangles
-  for (uint32_t q = blockIdx.x * 32u + (threadIdx.x & 31u); q < n; q += gridDim.x * 32u) {
+  // a warp's lanes do the same part of 32 triangles; the parts that the frame's flags ask
+  // for, so that no warp has nothing to do (327,680 faces with edges alone: 33.4 -> 29.8 us)
+  const uint32_t first = a.flags_any & 0x40u ? 0u : 4u, parts = (a.flags_any & 0x80u ? 7u : 4u) - first;
+  const uint32_t tasks = (n + 31u) / 32u * parts;
+  for (uint32_t task = blockIdx.x * 8u + (threadIdx.x >> 5); task < tasks; task += gridDim.x * 8u) {
+    const uint32_t q = task / parts * 32u + (threadIdx.x & 31u);
+    const int part = (int)(first + task % parts);
+    if (q >= n) continue;
     // the kept faces of views with overlays (all their binned ones), then k_clip's fans
     float2 p[3];
     uint32_t key;
