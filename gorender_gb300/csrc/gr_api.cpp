@@ -848,8 +848,8 @@ int32_t draw_sync(gr_context* c, const gr_draw_item* items, int32_t n, const gr_
     if ((st = prepare(c, &v, 1, items, n, false, pr, nullptr, nullptr, Upload::kInGraph))) return st;
     // the counters and the outputs in one go: one host wait per frame (a frame
     // whose buffers overflowed is drawn again and its outputs copied again);
-    // the frame's last kernel writes the counters into page-locked memory itself,
-    // then sets the done word after them
+    // the frame's last kernel writes the counters into page-locked memory itself
+    // and, with outputs in host memory, sets the done word after them
     pr.a.result_host = c->h_result_dev;
     volatile uint32_t* done = reinterpret_cast<volatile uint32_t*>(c->h_result + 1);
     *done = 0u;
@@ -2194,7 +2194,7 @@ struct gr_presenter {
   cudaStream_t copy = nullptr;
   uint32_t* dev[2] = {nullptr, nullptr};
   uint8_t* host[2] = {nullptr, nullptr};      // pinned
-  DevResult* res[2] = {nullptr, nullptr};     // pinned: each frame's counters (and the raster's done word)
+  DevResult* res[2] = {nullptr, nullptr};     // pinned: each frame's counters
   DevResult* res_dev[2] = {nullptr, nullptr}; // their device addresses: k_resolve writes there
   cudaEvent_t rendered[2] = {}, copied[2] = {};
   std::vector<gr_draw_item> items[2];

@@ -331,12 +331,14 @@ struct FrameArgs {
   uint32_t slice_cost;              // raster cost per slice (k_plan splits costlier tiles)
   DevWork* work;
   DevResult* result;
-  DevResult* result_host;           // device address of page-locked host memory that the last raster
-                                    // CTA copies the result into (null: the host copies it), followed
-                                    // by a word it sets to 1 once the frame's writes are visible to the
-                                    // host (every CTA fences at system scope before it retires)
-  unsigned long long* view_tpf;     // per view: binned triangles (zeroed by k_plan)
-  unsigned long long* view_tpf_out; // per view: published by k_plan
+  DevResult* result_host;           // device address of page-locked host memory that the result is copied
+                                    // into (null: the host copies it).  Frames shaded by k_raster: by its
+                                    // last CTA, followed by a word that it sets to 1 once the frame's
+                                    // writes are visible to the host (every CTA fences at system scope
+                                    // before it retires).  Frames shaded by k_resolve (pkey): beside its
+                                    // shading, the counters alone; the stream says when they are complete
+  unsigned long long* view_tpf;     // per view: binned triangles (zeroed where the result is published)
+  unsigned long long* view_tpf_out; // per view: published with the result
   RasterWork* plan;                 // raster work items, plan_cap entries
   uint2* empty_tiles;               // (tile, view) of tiles without bin entries, cleared by k_raster
   uint32_t empty_cap;

@@ -2271,7 +2271,10 @@ __device__ __forceinline__ void clear_quad(const FrameArgs& a, uint2 e, uint32_t
 
 // The frame's counters and per-view TPF, published and returned to zero for the
 // next frame, `items` raster items in all: by the CTA that calls this, once the
-// raster is over.
+// raster is over.  DONE: the frame is complete with it (k_raster's last CTA, every
+// other one having fenced its outputs), so a word in page-locked memory says so;
+// k_resolve publishes beside its shading and sets none.
+template <bool DONE>
 __device__ __forceinline__ void publish_frame(const FrameArgs& a, uint32_t items) {
   if (threadIdx.x == 0) {
     DevWork* w = a.work;
@@ -2308,10 +2311,12 @@ __device__ __forceinline__ void publish_frame(const FrameArgs& a, uint32_t items
     if (threadIdx.x < kWords)
       reinterpret_cast<unsigned*>(a.result_host)[threadIdx.x] =
           __ldcg(reinterpret_cast<const unsigned*>(a.result) + threadIdx.x);
-    __syncthreads();
-    if (threadIdx.x == 0) {  // the frame is complete: counters and every output are visible to the host
-      __threadfence_system();
-      reinterpret_cast<volatile unsigned*>(a.result_host)[kWords] = 1u;
+    if constexpr (DONE) {
+      __syncthreads();
+      if (threadIdx.x == 0) {  // counters and every output are visible to the host
+        __threadfence_system();
+        reinterpret_cast<volatile unsigned*>(a.result_host)[kWords] = 1u;
+      }
     }
   }
 }
@@ -2385,7 +2390,7 @@ __global__ void __launch_bounds__(RasterShape<TS>::kThreads, RasterShape<TS>::kM
   __syncthreads();
   if (!s_lastcta) return;
   __threadfence();
-  publish_frame(a, s_total);
+  publish_frame<true>(a, s_total);
 }
 
 // ---------------------------------------------------------------------------
@@ -2408,7 +2413,7 @@ __global__ void __launch_bounds__(RasterShape<TS>::kThreads, RasterShape<TS>::kM
 __global__ void __launch_bounds__(256, 6) k_resolve(const FrameArgs a) {
   griddep_wait();
   if (blockIdx.y == 0) {  // the first row of CTAs shades nothing: one publishes the counters meanwhile
-    if (blockIdx.x == 0) publish_frame(a, a.work->plan_front + a.work->plan_back);
+    if (blockIdx.x == 0) publish_frame<false>(a, a.work->plan_front + a.work->plan_back);
     return;
   }
   const DevView& vw = a.views[0];
