@@ -256,7 +256,6 @@ constexpr long long kMaxLineSteps = 1ll << 22;  // longer overlay lines are refu
 // Counters the kernels append to.  Zeroed once at allocation; the raster
 // kernel copies them into DevResult and zeroes them again.
 struct DevWork {
-  unsigned long long tpf;           // binned triangles (Renderer.TPF, one tile)
   unsigned int nrec;                // raster records written
   unsigned int nbig;                // records in the multi-tile queue
   unsigned int bin_need;            // max (bin position + 1) seen when over capacity

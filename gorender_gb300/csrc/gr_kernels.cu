@@ -145,43 +145,6 @@ __device__ __forceinline__ PV intersect(int i, const PV& A, const PV& B) {
   return o;
 }
 
-// Frustum.ClipTriangle (clipping.go:167-236) in place on poly (count 3 on
-// entry).  Returns the polygon vertex count (0: clipped away) or -1 when the
-// polygon would exceed 9 vertices (the reference panics there).
-__device__ int clip_polygon(PV* poly, PV* tmp) {
-  int count = 3;
-  PV* a = poly;
-  PV* b = tmp;
-  for (int pi = 0; pi < 6; ++pi) {
-    int n2 = 0;
-    for (int bi = 0; bi < count; ++bi) {
-      int ai = (bi + 1 == count) ? 0 : bi + 1;
-      const PV A = a[ai];
-      const PV B = a[bi];
-      bool inA = plane_inside(pi, A.p);
-      if (inA) {
-        if (!plane_inside(pi, B.p)) {
-          if (n2 >= 9) return -1;
-          b[n2++] = intersect(pi, A, B);
-        }
-        if (n2 >= 9) return -1;
-        b[n2++] = A;
-      } else if (plane_inside(pi, B.p)) {
-        if (n2 >= 9) return -1;
-        b[n2++] = intersect(pi, A, B);
-      }
-    }
-    if (n2 == 0) return 0;
-    count = n2;
-    PV* t = a;
-    a = b;
-    b = t;
-  }
-  if (a != poly)
-    for (int k = 0; k < count; ++k) poly[k] = a[k];
-  return count;
-}
-
 // Screen-space vertex after divide + screen map (renderer.go:361-370) and
 // the int() truncations of drawProjection (renderer.go:182-184).
 struct SV {
@@ -2293,7 +2256,7 @@ __device__ __forceinline__ void publish_frame(const FrameArgs& a, uint32_t items
     r->novl = w->novl;
     r->ovl_need = w->ovl_need;
     w->novl = 0; w->ovl_need = 0;
-    w->tpf = 0; w->nrec = 0; w->nbig = 0; w->bin_need = 0; w->rec_need = 0; w->big_need = 0; w->error = 0;
+    w->nrec = 0; w->nbig = 0; w->bin_need = 0; w->rec_need = 0; w->big_need = 0; w->error = 0;
     w->nclip = 0; w->clip_need = 0; w->max_bin = 0; w->nkept = 0; w->nhuge = 0;
     w->plan_front = 0; w->plan_back = 0; w->raster_next = 0; w->raster_exit = 0;
     w->nempty = 0; w->clear_next = 0;
