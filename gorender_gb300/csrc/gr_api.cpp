@@ -695,8 +695,9 @@ int32_t prepare(gr_context* c, const ViewIn* views, int nviews, const gr_draw_it
   // Many views shaded in place: tiles without bin entries (most of a batch
   // of small meshes) are cleared by the raster CTAs once their queue is
   // empty, without keys (a 256-view batch 1.81 -> 1.62 ms with a kernel of
-  // their own, 1.335 -> 1.286 ms inside k_raster); one view keeps them in the
-  // raster queue (0.153 against 0.166 ms a frame with the separate kernel).
+  // their own, 1.335 -> 1.286 ms inside k_raster); one view shaded in place
+  // keeps them in the raster queue (0.153 against 0.166 ms a frame with the
+  // separate kernel), and one shaded by k_resolve makes no work item of them.
   a.clear_empty = (!separate && nviews > 1) ? 1 : 0;
   if (a.clear_empty && total_tiles > c->empty_cap) {  // allocated only for such frames
     CK(cudaStreamSynchronize(c->stream));

@@ -207,6 +207,7 @@ __device__ __forceinline__ FF ff_mul(FF a, FF b) {  // the product of the his is
   e = __fadd_rn(e, __fadd_rn(__fmul_rn(a.hi, b.lo), __fmul_rn(a.lo, b.hi)));
   return fast_two_sum(p, e);
 }
+
 // A sum of floats as three: the additions' errors go to the next part, so it holds
 // some 70 bits (a double's sum rounds at each addition to 53), on the float32 pipes.
 struct Sum3 {
@@ -227,9 +228,7 @@ struct Sum3 {
       mid = v.hi;
     }
   }
-  __device__ __forceinline__ double value() const {  // infinities and NaN stand in hi alone
-    return isfinite(hi) ? (double)hi + ((double)mid + (double)lo) : (double)hi;
-  }
+  __device__ __forceinline__ double value() const { return (double)hi + ((double)mid + (double)lo); }
 };
 
 __device__ __forceinline__ FF ff_mul_f(FF a, float b) {
@@ -498,11 +497,12 @@ __device__ __forceinline__ void sum_slots(const DiffArgs& a, int c0, double* dst
   if (threadIdx.x == 0) *a.done = 0u;
 }
 
-// Forward: per pixel record, shaded pixel and the loss.  Bound by the latency of its gathers (face, then
-// corners, then texel: 40 % of the issue slots, 38 % of the memory rate).  64 views
-// of 512 x 512 pixels of an 81,920-face mesh: 394 -> 238 us with the gathered data
-// packed (36 loads a covered pixel before, 13 now), blocks instead of rows of
-// pixels a warp, and the loss out of the FP64 pipe.
+// Forward: per pixel record, shaded pixel and the loss.  Bound by the latency of
+// its gathers (face, then corners, then texel: 46 % of the issue slots, 38 % of
+// the memory rate).  64 views of 512 x 512 pixels of an 81,920-face mesh: 394 -> 233
+// us with the gathered data packed (36 loads a covered pixel before, 13 now),
+// blocks instead of rows of pixels a warp, and the loss out of the FP64 pipe as
+// two floats; 245 with three, which hold all of its bits.
 __global__ void __launch_bounds__(kThreads, 4) k_diff_shade(const DiffArgs a) {
   griddep_wait();
   const Pixels at = block_pixels(a);
@@ -510,10 +510,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_diff_shade(const DiffArgs a) {
   const int px = at.x;
   // the pixels' losses, summed as three floats, no less exact than in FP64 (the warp's
   // sum goes to FP64), since FP64 additions, one a pixel or five for each warp's
-  // tree, held this kernel at the FP64 pipe's rate.  (Two floats, which round to
-  // about 46 bits, are 1 % of the 64-view step faster.)  Losses near float32's
-  // end, and infinities and NaN, are summed apart, scaled by 2^-80.
-  Sum3 sum, big;
+  // tree, held this kernel at the FP64 pipe's rate.  (Two floats round to about
+  // 46 bits.)  Losses near float32's end, and infinities and NaN, are summed
+  // apart, scaled by 2^-80, as two floats: multiples of 2^16 up to 2^48 then, 256 at
+  // most, so the low part is a multiple of 2^16 up to 2^39 and exact too.
+  Sum3 sum;
+  float bhi = 0.0f, blo = 0.0f;
   for (int k = 0; k < a.blocks_down; ++k) {
     const int py = at.y + k * at.rows;
     if (px >= vw.W || py >= vw.H) break;
@@ -551,14 +553,24 @@ __global__ void __launch_bounds__(kThreads, 4) k_diff_shade(const DiffArgs a) {
     if (a.image) reinterpret_cast<float4*>(a.image)[gp] = out;
     const float dx = out.x - tg.x, dy = out.y - tg.y, dz = out.z - tg.z, dw = out.w - tg.w;
     const float lp = dx * dx + dy * dy + dz * dz + dw * dw;
-    if (lp < 1e36f) sum.add(lp);
-    else big.add(lp * 0x1p-80f);
+    if (lp < 1e36f) {
+      sum.add(lp);
+    } else {
+      const FF t = two_sum(bhi, lp * 0x1p-80f);
+      bhi = t.hi;
+      blo = __fadd_rn(blo, t.lo);
+    }
   }
   sum.add_lanes();
   double loss = sum.value();
-  if (__any_sync(0xffffffffu, big.hi != 0.0f)) {
-    big.add_lanes();
-    loss += big.value() * 0x1p80;
+  if (__any_sync(0xffffffffu, bhi != 0.0f)) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const FF t = two_sum(bhi, __shfl_xor_sync(0xffffffffu, bhi, o));
+      blo = __fadd_rn(__fadd_rn(blo, __shfl_xor_sync(0xffffffffu, blo, o)), t.lo);
+      bhi = t.hi;
+    }
+    loss += (isfinite(bhi) ? (double)bhi + (double)blo : (double)bhi) * 0x1p80;
   }
   // one atomic into the warp's slot, so that warps never wait for each other
   if ((threadIdx.x & 31) == 0 && loss != 0.0) atomicAdd(a.partials + 4 * diff_slot(), loss);
@@ -570,8 +582,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_diff_shade(const DiffArgs a) {
 // pixels were paired).  64 views of 512 x 512 pixels of an 81,920-face mesh: 400 ->
 // 254 us with the gathered data packed, the normals and the light's sums left
 // to k_diff_scatter (303 us), neighbouring pixels of a face paired (263; side
-// by side alone 272) and the face ids read a step ahead (254); records and targets, read once, evict-first here
-// and in k_diff_shade: the step 1184 -> 1179.  The light's weights in FP64: 288.
+// by side alone 272) and the face ids read a step ahead (254); records and
+// targets, read once, evict-first here and in k_diff_shade: the step 1184 -> 1179.
+// The light's weights in FP64: 288.
 __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
   const Pixels at = block_pixels(a);
   const DiffView& vw = a.views[at.view];
@@ -657,11 +670,12 @@ __global__ void __launch_bounds__(kThreads) k_diff_grad(const DiffArgs a) {
     // float4 and a float2, the texel's four a float4.  Beside them stands, as a
     // double, the corner's weight in the light's gradient, dI/dL = sum_k l_k 0.5
     // nhat_k, which k_diff_scatter multiplies with its normal: no normal is read
-    // here, and the light is summed over all pixels in FP64, up to its end (in
+    // here, and from these doubles on the light is summed in FP64 up to its end (in
     // float32 it was 35 us faster at 64 views and its error, 1.3e-8 to 1.1e-7 over seven
     // cases, up to three times as large in one).  The reductions' way out of
     // the SM bounds this kernel, so pixels of one face side by side or one
-    // above the other are added up first.
+    // above the other, up to four, are added up first, in float32 like all that
+    // is a pixel's own.
     on = rec.face != kNoFace;
 #pragma unroll
     for (int o = 1; o <= 8; o <<= 3) {

@@ -253,8 +253,9 @@ struct Overlay {
 };
 constexpr long long kMaxLineSteps = 1ll << 22;  // longer overlay lines are refused (error bit 2)
 
-// Counters the kernels append to.  Zeroed once at allocation; the raster
-// kernel copies them into DevResult and zeroes them again.
+// Counters the kernels append to.  Zeroed once at allocation; the frame's last
+// kernel (k_resolve, or k_raster where that shades) copies them into DevResult and
+// zeroes them again.
 struct DevWork {
   unsigned int nrec;                // raster records written
   unsigned int nbig;                // records in the multi-tile queue
@@ -352,7 +353,7 @@ struct FrameArgs {
                                     // (null: k_raster shades each tile itself)
   uint4* tile_info;                 // per tile of a one-view frame, from k_plan: x bin entries, y raster slices, z first key
                                     // slot of a split tile of a one-view frame (kNoSlot: merged in gkey),
-                                    // w pixels of its large entries' boxes
+                                    // w unused (one 16-byte load)
   unsigned long long* slot_keys;    // one-view frames: slot_cap slots of TS x TS keys, one per slice of a
                                     // split tile; k_resolve takes the max over a tile's slots
   uint32_t slot_cap;
