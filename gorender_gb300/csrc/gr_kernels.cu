@@ -1465,7 +1465,9 @@ constexpr int kTinyBox = 3;                  // boxes of at most 3 x 3 pixels ma
 
 // A warp's share of a batch of bin entries: its narrow triangles, five
 // 16-byte words a slot with the slots side by side (lanes that read different
-// slots hit different banks), with coordinates relative to the tile.
+// slots hit different banks), with coordinates relative to the tile.  The slots
+// from the last one down hold its triangles with int64 edges: a01, b01, c01, a12,
+// ..., c20 in order, then min(-w) and the order key.
 struct WarpTable {
   int4 e01[32];      // a01, b01, c01; first pixel x | y << 8 | width << 16 of the box in the tile
   int4 e12[32];      // a12, b12, c12; order key
@@ -1541,9 +1543,18 @@ __device__ __forceinline__ void raster_stage(const FrameArgs& a, const DevView& 
   const bool fast = units_walk && narrow_fast(t);
   const bool general = __any_sync(FULL_MASK, units_walk && !fast);
   const unsigned wm = __ballot_sync(FULL_MASK, wide);
-  if (wide)
-    tab.wide[__popc(wm & ((1u << lane) - 1u))] =
-        make_uint2(r, (uint32_t)((lx0 - tx0) | (ly0 - ty0) << 8 | (lx1 - tx0) << 16 | (ly1 - ty0) << 24));
+  if (wide) {
+    const int k = __popc(wm & ((1u << lane) - 1u)), s = 31 - k;
+    tab.wide[k] = make_uint2(r, (uint32_t)((lx0 - tx0) | (ly0 - ty0) << 8 | (lx1 - tx0) << 16 | (ly1 - ty0) << 24));
+    const int4* q = reinterpret_cast<const int4*>(a.wide + r);  // TriWide: nine int64 first
+    tab.e01[s] = q[0];
+    tab.e12[s] = q[1];
+    tab.e20[s] = q[2];
+    tab.d0[s] = *reinterpret_cast<const float4*>(q + 3);
+    const int2 c20 = *reinterpret_cast<const int2*>(q + 4);
+    tab.d1[s] = make_float4(__int_as_float(c20.x), __int_as_float(c20.y),
+                            fmaxf(fminf(fminf(-t.w0, -t.w1), -t.w2), 0.0f), __uint_as_float(t.key & 0x7FFFFFFFu));
+  }
   const int bw = lx1 - lx0 + 1, bh = ly1 - ly0 + 1;
   if (tiny) {
     const bool here = fast && bw <= kTinyBox && bh <= kTinyBox;
@@ -1670,17 +1681,21 @@ __device__ __forceinline__ void raster_units(const WarpTable& tab, uint2* runs, 
 
 // The batch's triangles with int64 edges: the CTA's warps take the 8 x 4 blocks of
 // all their boxes in turn, numbered from one triangle to the next, so that many
-// triangles of one block each keep all of them busy; a warp reads a triangle's
-// record only where it has a block of it.
+// triangles of one block each keep all of them busy.  The edges come from the
+// tables for each block: held in registers they made every other frame spill and 1-2 %
+// slower, and read from the records the far ones took 12 % longer (unclipped
+// 199,712-triangle terrain with the camera inside: 2165 us a triangle after the
+// other, 2280 from the records, 2042 now).
 template <int TS>
-__device__ __forceinline__ void raster_wide(const TriPacked* rast, const TriWide* wide, RasterSmem<TS>& sm, int tx0,
-                                            int ty0) {
+__device__ __forceinline__ void raster_wide(const TriPacked* rast, RasterSmem<TS>& sm, int tx0, int ty0) {
   constexpr int kWarps = RasterShape<TS>::kWarps;
   typedef unsigned long long u64;
   const int lx = (int)(threadIdx.x & 7u), ly = (int)((threadIdx.x >> 3) & 3u), warp = (int)(threadIdx.x >> 5);
   int base = 0;  // blocks of the triangles before this one
+#pragma unroll 1
   for (int w = 0; w < kWarps; ++w) {
     const WarpTable& tab = sm.tab[w];
+#pragma unroll 1
     for (int k = 0; k < tab.nwide; ++k) {
       const uint2 e = tab.wide[k];
       const int x0 = (int)(e.y & 0xFFu), y0 = (int)((e.y >> 8) & 0xFFu), x1 = (int)((e.y >> 16) & 0xFFu),
@@ -1689,28 +1704,34 @@ __device__ __forceinline__ void raster_wide(const TriPacked* rast, const TriWide
       int j = (warp - base) & (kWarps - 1);
       base += nblk;
       if (j >= nblk) continue;
-      const TriPacked& t = rast[e.x];
-      const float4 ws = *reinterpret_cast<const float4*>(&t.w0);  // W's and the sum
-      const uint32_t okey = t.key & 0x7FFFFFFFu;
-      const float wmin = fmaxf(fminf(fminf(-ws.x, -ws.y), -ws.z), 0.0f);
-      const TriWide q = wide[e.x];
+      const int s = 31 - k;
+#pragma unroll 1
       for (; j < nblk; j += kWarps) {
         const int x = x0 + (j % nbx) * 8 + lx, y = y0 + (j / nbx) * 4 + ly;
         if (x > x1 || y > y1) continue;
         const u64 X = (u64)(tx0 + x), Y = (u64)(ty0 + y);
-        const long long e01 = (long long)((u64)q.a01 * X + (u64)q.b01 * Y + (u64)q.c01);
-        const long long e12 = (long long)((u64)q.a12 * X + (u64)q.b12 * Y + (u64)q.c12);
-        const long long e20 = (long long)((u64)q.a20 * X + (u64)q.b20 * Y + (u64)q.c20);
+        const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(tab.e01 + s),
+                         q1 = *reinterpret_cast<const ulonglong2*>(tab.e12 + s),
+                         q2 = *reinterpret_cast<const ulonglong2*>(tab.e20 + s),
+                         q3 = *reinterpret_cast<const ulonglong2*>(tab.d0 + s);
+        const float4 q4 = tab.d1[s];
+        const u64 c20 = (u64)__float_as_uint(q4.x) | (u64)__float_as_uint(q4.y) << 32;
+        const long long e01 = (long long)(q0.x * X + q0.y * Y + q1.x);
+        const long long e12 = (long long)(q1.y * X + q2.x * Y + q2.y);
+        const long long e20 = (long long)(q3.x * X + q3.y * Y + c20);
         if ((e01 & e12 & e20) >= 0) continue;  // covered where all three are negative (rasterizer.go:147)
         u64* p = sm.skey + y * RasterShape<TS>::kStride + x;
-        if (depth_beaten(*(volatile u64*)p, wmin)) continue;
-        depth_at(p, __ll2float_rn(e12), __ll2float_rn(e20), ws.w, ws.x, ws.y, ws.z, okey);
+        if (depth_beaten(*(volatile u64*)p, q4.z)) continue;
+        const float4 ws = __ldg(reinterpret_cast<const float4*>(&rast[e.x].w0));  // W's and the sum
+        depth_at(p, __ll2float_rn(e12), __ll2float_rn(e20), ws.w, ws.x, ws.y, ws.z, __float_as_uint(q4.w));
       }
     }
   }
 }
 
-// The batch's groups of 32 units, table by table, the CTA's warps in turn.
+// The batch's groups of 32 units, table by table, the CTA's warps in turn.  GENERAL
+// where some triangle's W's are out of narrow_fast's range (20,000 triangles of 9
+// pixels with W's of 2^-63 at 640 x 360: 79 us one after the other, 36 so).
 template <int TS, bool GENERAL>
 __device__ __forceinline__ void raster_batch(RasterSmem<TS>& sm) {
   constexpr int kWarps = RasterShape<TS>::kWarps;
@@ -1724,22 +1745,6 @@ __device__ __forceinline__ void raster_batch(RasterSmem<TS>& sm) {
     const int prev = __shfl_sync(FULL_MASK, groups, (seg + 31) & 31);
     raster_units<TS, GENERAL>(sm.tab[seg], sm.tab[warp].run, sm.tab[seg].units, (g - (seg ? prev : 0)) << 5, sm.skey);
   }
-}
-
-// A batch with triangles beyond the usual: int64 edges, or W's out of narrow_fast's
-// range, which take the general divisions (and the batch's others with them).
-// 20,000 triangles of 9 pixels with W's of 2^-63 at 640 x 360: 79 us with those in
-// raster_wide, 35 here; an unclipped 199,712-triangle terrain with the camera
-// inside 2165 -> 2020.  Chosen once a batch: with a choice for each group of units
-// the 256-view batch took 1056 us instead of 1040, and with functions called
-// instead of inlined a 1280 x 720 terrain 95 instead of 89.
-template <int TS>
-__device__ __forceinline__ void raster_odd_batch(const TriPacked* rast, const TriWide* wide, RasterSmem<TS>& sm, int tx0,
-                                                 int ty0) {
-  const unsigned lane = lane_id();
-  if (__any_sync(FULL_MASK, lane < (unsigned)RasterShape<TS>::kWarps && sm.tab[lane].general)) raster_batch<TS, true>(sm);
-  else raster_batch<TS, false>(sm);
-  raster_wide<TS>(rast, wide, sm, tx0, ty0);
 }
 
 __device__ __forceinline__ TriShade load_shade(const FrameArgs& a, uint32_t r) {
@@ -1918,10 +1923,11 @@ __device__ __forceinline__ void raster_item(const FrameArgs& a, const uint32_t& 
         sm.tab[warp].general = false;
       }
       __syncthreads();
-      const unsigned odd =
-          __ballot_sync(FULL_MASK, lane < (unsigned)kWarps && (sm.tab[lane].nwide != 0 || sm.tab[lane].general));
-      if (!odd) raster_batch<TS, false>(sm);
-      else raster_odd_batch<TS>(a.rast, a.wide, sm, tx0, ty0);
+      // (one choice a batch: one for each group of units took the 256-view batch from 1040 to 1056 us)
+      const bool wide = __any_sync(FULL_MASK, lane < (unsigned)kWarps && sm.tab[lane].nwide != 0);
+      if (__any_sync(FULL_MASK, lane < (unsigned)kWarps && sm.tab[lane].general)) raster_batch<TS, true>(sm);
+      else raster_batch<TS, false>(sm);
+      if (wide) raster_wide<TS>(a.rast, sm, tx0, ty0);
       __syncthreads();
     }
 
