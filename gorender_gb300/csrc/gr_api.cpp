@@ -1858,7 +1858,7 @@ int32_t diff_blocks(gr_diff* d) {
   d->view_blocks = 0;
   bool even = true;
   for (DiffView& v : d->hviews) {
-    const int wide = diff_block_wide(v.W), high = kDiffThreads / wide * d->blocks_down;
+    const int wide = 1 << diff_block_shift(v.W), high = kDiffThreads / wide * d->blocks_down;
     v.blocks_x = (v.W + wide - 1) / wide;
     v.block_base = (uint32_t)total;
     const uint32_t n = (uint32_t)v.blocks_x * (uint32_t)((v.H + high - 1) / high);

@@ -420,7 +420,7 @@ __device__ __forceinline__ int wrap_index(float u, int n) {
 
 // The pixels of a thread: column x of its view, rows y, y + rows, ..., a.blocks_down
 // of them.  A CTA's warps take an 8 x 4 block each (blocks share more faces, and so more
-// gathered lines, than rows of 32 do), side by side first (diff_block_wide).
+// gathered lines, than rows of 32 do), side by side first (diff_block_shift).
 struct Pixels {
   int view, x, y, rows;
 };
@@ -448,9 +448,9 @@ __device__ __forceinline__ Pixels block_pixels(const DiffArgs& a) {
   const DiffView& vw = a.views[view];
   const int local = (int)(blockIdx.x - vw.block_base);
   const int by = local / vw.blocks_x, bx = local - by * vw.blocks_x;
-  const int wide = diff_block_wide(vw.W), rows = kThreads / wide, warp = (int)(threadIdx.x >> 5);
-  const int across = wide >> 3, wy = warp / across, wx = warp - wy * across;
-  return Pixels{view, bx * wide + wx * 8 + (int)(threadIdx.x & 7u),
+  const int sh = diff_block_shift(vw.W), rows = kThreads >> sh, warp = (int)(threadIdx.x >> 5);
+  const int wy = warp >> (sh - 3), wx = warp & ((1 << (sh - 3)) - 1);
+  return Pixels{view, (bx << sh) + wx * 8 + (int)(threadIdx.x & 7u),
                 by * a.blocks_down * rows + wy * 4 + (int)((threadIdx.x >> 3) & 3u), rows};
 }
 
@@ -460,9 +460,10 @@ __device__ __forceinline__ int diff_slot() {
   return (int)((blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) & (kDiffSlots - 1));
 }
 
-// The last of a grid's CTAs to get here (an atomic counter, no waiting) writes the sums of components [c0, c0 + N) of the slots to dst
-// (page-locked host memory, through its device address: no copy follows) and
-// returns the slots and the counter to zero.  Called by every thread.
+// The last of a grid's CTAs to get here (an atomic counter, no waiting) writes
+// the sums of components [c0, c0 + N) of the slots to dst (page-locked host
+// memory, through its device address: no copy follows) and returns the slots and
+// the counter to zero.  Called by every thread.
 template <int N>
 __device__ __forceinline__ void sum_slots(const DiffArgs& a, int c0, double* dst) {
   __shared__ double s_w[N][kThreads / 32];

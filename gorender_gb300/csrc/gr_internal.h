@@ -385,7 +385,7 @@ constexpr int kDiffThreads = 256;    // a CTA of the differentiable kernels
 // The pixels that a CTA of k_diff_shade / k_diff_grad (eight warps of 8 x 4) takes at
 // a time: 32 x 8, or in views of at most 16 and 8 columns 16 x 16 and 8 x 32, so that
 // narrow views leave no warp without pixels.
-__host__ __device__ inline int diff_block_wide(int W) { return W > 16 ? 32 : W > 8 ? 16 : 8; }
+__host__ __device__ inline int diff_block_shift(int W) { return W > 16 ? 5 : W > 8 ? 4 : 3; }  // log2 of the width
 
 // Per-pixel forward record: the visible face (or kNoFace), the texel it
 // sampled (or kNoFace without a texture) and two perspective-correct
