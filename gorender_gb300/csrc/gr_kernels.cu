@@ -7,8 +7,8 @@
 //   k_cull     faces in groups of 32 x G per warp: backface and frustum
 //              tests on every face, the bin test (TPF) and the coverage of
 //              small faces; faces kept whole are compacted into one list,
-//              straddling faces and those beyond the narrow bound go to
-//              k_clip (the general clipper, one warp per face, beside k_setup).
+//              straddling faces go to k_clip (the general clipper, one warp
+//              per face, beside k_setup).
 //   k_setup    full warps of kept faces: attributes, screen vertices and
 //              their records, binned with warp-aggregated atomics
 //              (__match_any_sync) or, past four tiles, queued for k_bin_big.
